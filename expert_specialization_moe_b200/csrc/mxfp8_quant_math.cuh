@@ -28,6 +28,50 @@ __device__ __forceinline__ uint4 ld_stream_16B(const void* p) {
   return v;
 }
 
+// 32 bytes per lane in one instruction (sm_100); p must be 32-byte aligned
+__device__ __forceinline__ void ld_stream_32B(const void* p, uint32_t (&v)[8]) {
+  asm volatile("ld.global.nc.L1::no_allocate.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+               : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
+               : "l"(p));
+}
+
+__device__ __forceinline__ void st_stream_16B(void* p, const uint4& v) {
+  asm volatile("st.global.cs.v4.u32 [%0], {%1,%2,%3,%4};" ::"l"(p), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
+}
+
+__device__ __forceinline__ float ex2_approx_ftz(float a) {
+  float b;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(b) : "f"(a));
+  return b;
+}
+
+// two fp32 operations per instruction (sm_100), each rounded to nearest as the scalar form
+__device__ __forceinline__ unsigned long long pack_f32x2(float2 a) {
+  unsigned long long r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a.x), "f"(a.y));
+  return r;
+}
+__device__ __forceinline__ float2 unpack_f32x2(unsigned long long a) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(a));
+  return r;
+}
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
+  unsigned long long r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(pack_f32x2(a)), "l"(pack_f32x2(b)));
+  return unpack_f32x2(r);
+}
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+  unsigned long long r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(pack_f32x2(a)), "l"(pack_f32x2(b)));
+  return unpack_f32x2(r);
+}
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+  unsigned long long r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(pack_f32x2(a)), "l"(pack_f32x2(b)), "l"(pack_f32x2(c)));
+  return unpack_f32x2(r);
+}
+
 __device__ __forceinline__ void st_stream_8B(void* p, uint2 v) {
   asm volatile("st.global.cs.v2.u32 [%0], {%1,%2};" ::"l"(p), "r"(v.x), "r"(v.y) : "memory");
 }
@@ -87,6 +131,67 @@ __device__ __forceinline__ uint32_t quantize8(const uint4& raw, uint2& codes) {
   }
   codes.x = out[0];
   codes.y = out[1];
+  return sf.__x;
+}
+
+// max(|a|, |b|) per half, the sign of the result unspecified; NaN members dropped
+template <typename T>
+__device__ __forceinline__ uint32_t max_magnitude2(uint32_t a, uint32_t b);
+template <>
+__device__ __forceinline__ uint32_t max_magnitude2<__nv_bfloat16>(uint32_t a, uint32_t b) {
+  uint32_t r;
+  asm("max.xorsign.abs.bf16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+  return r;
+}
+template <>
+__device__ __forceinline__ uint32_t max_magnitude2<__half>(uint32_t a, uint32_t b) {
+  uint32_t r;
+  asm("max.xorsign.abs.f16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+  return r;
+}
+
+template <typename T>
+__device__ __forceinline__ uint32_t max_magnitude16(const uint32_t (&v)[8]) {
+  const uint32_t a = max_magnitude2<T>(max_magnitude2<T>(v[0], v[1]), max_magnitude2<T>(v[2], v[3]));
+  const uint32_t b = max_magnitude2<T>(max_magnitude2<T>(v[4], v[5]), max_magnitude2<T>(v[6], v[7]));
+  return max_magnitude2<T>(a, b);
+}
+
+// larger magnitude of the two halves as fp32 (NaN only if both are)
+template <typename T>
+__device__ __forceinline__ float magnitude_of_pair(uint32_t m) {
+  using V2 = typename Vec2<T>::type;
+  m &= 0x7fff7fffu;
+  const V2 mx = *reinterpret_cast<const V2*>(&m);
+  return Vec2<T>::to_float(__hmax(mx.x, mx.y));
+}
+
+// largest |v_i| of the lane's 16 elements, NaN members dropped
+template <typename T>
+__device__ __forceinline__ float max_abs16(const uint32_t (&v)[8]) {
+  return magnitude_of_pair<T>(max_magnitude16<T>(v));
+}
+
+// Quantise the 16 elements this lane holds; two neighbouring lanes share one 32-element block.  Same arithmetic as
+// quantize8; returns the block's UE8M0 byte in both lanes.
+template <typename T>
+__device__ __forceinline__ uint32_t quantize16(const uint32_t (&v)[8], uint4& codes) {
+  using V2 = typename Vec2<T>::type;
+  uint32_t mx = max_magnitude16<T>(v);
+  mx = max_magnitude2<T>(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
+  const float block_max = magnitude_of_pair<T>(mx);
+  __nv_fp8_e8m0 sf;
+  sf.__x = __nv_cvt_float_to_e8m0(block_max * rcp_approx_ftz(448.0f), __NV_SATFINITE, cudaRoundPosInf);
+  const float inv = block_max != 0.f ? rcp_approx_ftz(static_cast<float>(sf)) : 0.0f;
+  uint32_t out[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const float2 lo = mul2(Vec2<T>::to_float2(*reinterpret_cast<const V2*>(&v[2 * i])), make_float2(inv, inv));
+    const float2 hi = mul2(Vec2<T>::to_float2(*reinterpret_cast<const V2*>(&v[2 * i + 1])), make_float2(inv, inv));
+    out[i] = (uint32_t)__nv_cvt_float2_to_fp8x2(lo, __NV_SATFINITE, __NV_E4M3) |
+             ((uint32_t)__nv_cvt_float2_to_fp8x2(hi, __NV_SATFINITE, __NV_E4M3) << 16);
+  }
+  codes = make_uint4(out[0], out[1], out[2], out[3]);
   return sf.__x;
 }
 

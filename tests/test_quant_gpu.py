@@ -142,3 +142,54 @@ def test_fused_silu_mul_quant_matches_cpu_oracle():
     ocodes, osf = C.oracle_quant(act_bits, True, counts)
     assert (codes != ocodes).mean() < 1e-3
     assert (sf != osf).mean() < 1e-3
+
+
+@pytest.mark.parametrize("is_bf16", [True, False])
+def test_fused_silu_mul_quant_every_gate_value(is_bf16):
+    """Every finite 16-bit gate value (subnormals, zeros, the largest) times up values over the whole exponent range,
+    bit-exact against the unfused GPU sequence: the fast form of the activation and its hand-over to the exact one."""
+    import torch
+    bits = np.arange(65536, dtype=np.uint16)
+    exp_mask = 0x7F80 if is_bf16 else 0x7C00
+    bits[(bits & exp_mask) == exp_mask] = 0x3C00
+    rng = np.random.default_rng(3)
+    T, K = 640, 512                                    # five passes over the 65536 gate values
+    gate = np.stack([rng.permutation(bits) for _ in range(5)]).reshape(T, K)
+    up = rng.integers(0, 65536, size=(T, K)).astype(np.uint16)
+    up[(up & exp_mask) == exp_mask] = 0x0001
+    half = rng.random((T, K)) < 0.5                    # half of them ordinary values: |up| in [0.25, 8)
+    plain = C.activations_bits(T, K, seed=9, is_bf16=is_bf16, outliers=False)
+    gu_bits = np.concatenate([gate, np.where(half, plain, up)], axis=1)
+    counts = [600, 1, 39]
+    codes, sf, gu = _run_silu_mul_quant(gu_bits, is_bf16, counts)
+    act = (torch.nn.functional.silu(gu[:, :K].float()) * gu[:, K:].float()).to(gu.dtype)
+    ucodes, usf, *_ = C.run_quant_op(act.view(torch.int16).cpu().numpy().view(np.uint16), is_bf16, counts)
+    assert np.array_equal(codes, ucodes)
+    assert np.array_equal(sf, usf)
+
+
+@pytest.mark.parametrize("counts,K", [([1], 128), ([3, 0, 2], 128), ([37, 129, 1], 640), ([33] * 9, 768),
+                                      ([700, 1, 260], 2176)])
+def test_quant_unit_edges_and_alignment(counts, K):
+    """Units of one to sixteen steps with ragged last steps (K tiles per row that do not divide a step), an input that
+    starts 16 bytes past a 32-byte boundary, and scale offsets whose padding words are only 4-byte aligned."""
+    import torch
+    from expert_specialization_moe_b200 import es_sm100_mxfp8_blockscaled_grouped_quant as quant
+    T = sum(counts)
+    x_bits = C.activations_bits(T, K, seed=T + K)
+    ocodes, osf = C.oracle_quant(x_bits, True, counts)
+    ps, eo, bo, sf_rows = Q.offsets_from_counts(counts, 0, K)
+    flat = torch.empty(T * K + 8, dtype=torch.bfloat16, device="cuda")
+    x = flat[8:].view(T, K)
+    assert x.data_ptr() % 32 == 16
+    x.copy_(C.bits_to_tensor(x_bits, True, "cuda"))
+    codes = torch.zeros((T, K), dtype=torch.uint8, device="cuda").view(torch.float8_e4m3fn)
+    sf = torch.full((sf_rows + 8, K // 32), 0xCD, dtype=torch.uint8, device="cuda")
+    dev = [torch.from_numpy(a).to("cuda") for a in (ps, eo, bo + 1)]
+    quant(x, *dev, codes, sf)
+    torch.cuda.synchronize()
+    assert np.array_equal(codes.view(torch.uint8).cpu().numpy(), ocodes)
+    got = sf.cpu().numpy().reshape(-1)
+    lead = K // 32
+    assert np.array_equal(got[lead:lead + osf.size], osf)
+    assert (got[:lead] == 0xCD).all() and (got[lead + osf.size:] == 0xCD).all()
