@@ -155,6 +155,19 @@ __device__ __forceinline__ uint32_t pack_pair_from_f32<__half>(float lo, float h
   return *reinterpret_cast<const uint32_t*>(&p);
 }
 
+// 32 bytes per thread to global memory: one 256-bit store where the address allows it, two 128-bit stores otherwise
+// (out is at least 16-byte aligned)
+__device__ __forceinline__ void store_32B(void* out, const uint32_t (&w)[8], bool aligned32) {
+  if (aligned32) {
+    asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(out), "r"(w[0]), "r"(w[1]), "r"(w[2]),
+                 "r"(w[3]), "r"(w[4]), "r"(w[5]), "r"(w[6]), "r"(w[7])
+                 : "memory");
+  } else {
+    static_cast<uint4*>(out)[0] = make_uint4(w[0], w[1], w[2], w[3]);
+    static_cast<uint4*>(out)[1] = make_uint4(w[4], w[5], w[6], w[7]);
+  }
+}
+
 // ---- an epilogue that holds converted chunks in registers (the CTA-pair kernel) ---------------------------------
 // A held chunk is 32 accumulator columns (tokens) of the warp's 32 lanes (n): register i = tokens (2i, 2i+1) as two
 // 16-bit values.  The warp reads all its chunks of an accumulator into held registers, hands the accumulator back to

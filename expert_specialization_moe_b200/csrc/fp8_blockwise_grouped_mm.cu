@@ -3,33 +3,36 @@
 // Per expert e:  d[off_e + i, n] = sum_kb sa[off_e + i, kb] * sb[e, n/128, kb] * sum_{k in kb} a[off_e + i, k] * b[e, n, k]
 //
 // The reference runs this op on Hopper only (wgmma templates).  Here every 128-wide K block is one unscaled
-// tcgen05.mma.kind::f8f6f4 group (4 MMAs of K=32) into one of FOUR TMEM partial buffers; the epilogue warps pull
-// each partial out of TMEM (tcgen05.ld), multiply by the block's scale product and accumulate in fp32 registers
-// while the tensor core works up to three K blocks ahead (two-stage promotion, as the reference's Hopper kernel
-// does in registers).  Same mapping as the MXFP8 kernels: 128 weight rows on the MMA M axis, the expert's tokens on
-// the runtime-sized MMA N axis (multiple of 16), work list from a per-CTA prefix scan, persistent grid of one CTA
-// per SM, one launch per row-count bucket (<= 32, 33..64, >= 65 rows) chained with programmatic dependent launch.
-// The buckets differ in the token tile and therefore in how many stages of weights fit the ring: these shapes are
-// HBM-bound on the weights, and bytes in flight per SM are what saturates HBM.
+// tcgen05.mma.kind::f8f6f4 group (4 MMAs of K=32) into a TMEM partial buffer; the epilogue warps pull each partial out
+// of TMEM (tcgen05.ld), multiply by the block's scale product and accumulate in fp32 registers while the tensor core
+// works on the following K blocks (two-stage promotion, as the reference's Hopper kernel does in registers).  Work list
+// from a per-CTA prefix scan, persistent grids of one CTA per SM; two launches chained with programmatic dependent
+// launch, each taking the experts of its row counts:
+//   few_rows  (<= 32 rows) 128 WEIGHT rows on the MMA M axis, the expert's tokens on its N axis.  Bound by HBM on the
+//             weights: what counts is bytes in flight (10 stages of 20 KB) and little shared-memory traffic besides;
+//   many_rows (>= 33 rows) 128 TOKEN rows on the M axis, 128 weight rows on the N axis.  A TMEM lane is then one
+//             token, so the scale of a K block is ONE register per thread: the promotion is a packed FMA with a scalar,
+//             without the broadcast shared-memory read per four FMAs that the other mapping needs next to the MMAs'
+//             operand reads, and a thread ends up with consecutive columns of one output row, stored as 32-byte pieces
+//             without a transposition.
 //
+// This file: the few-rows kernel and the entry point.
 //   warp 0     producer: TMA loads of the weight tile and the token tile per K block
 //   warps 1, 2 MMA issue, one lane each: warp 1 (which also owns the TMEM allocation) takes the even K blocks, warp 2
 //              the odd ones — consecutive K blocks go to different partial buffers, and a tcgen05.mma costs its
 //              issuing thread ~90 cycles against 64 cycles of tensor time for a 128 x 128 x 32 MMA
-//   warps 3(,4) scale loaders (two of them alternate chunks where registers allow): sa[token, kb] * sb[tile, kb] for
-//              8 K blocks at a time, transposed to [kb][token] in a ring of chunks, so that the epilogue reads one broadcast float4 per 4 tokens and
-//              never waits on global memory, whatever K is
-//   then       promotion (partial * scale -> fp32 registers) and output through a per-warp shared-memory transpose:
-//              one set of four warps (the four TMEM lane quadrants) per 32 token columns, so that a warp holds
-//              32 accumulators, reads its share of a partial with ONE tcgen05.ld, and the sets hide each other's
-//              TMEM latency; for the narrow tiles two such groups take alternate tiles, which hides the per-tile
+//   warps 3, 4 scale loaders, alternating chunks: sa[token, kb] * sb[tile, kb] for 8 K blocks at a time, transposed to
+//              [kb][token] in a ring of chunks, so that the epilogue reads one broadcast float4 per 4 tokens and never
+//              waits on global memory, whatever K is
+//   warps 5-12 promotion (partial * scale -> fp32 registers) and output through a per-warp shared-memory transpose:
+//              two groups of four warps (the four TMEM lane quadrants) take alternate tiles, which hides the per-tile
 //              latencies (work-list decode, output) that dominate when K is only 2-4 blocks
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
-#include <cstdlib>
 #include "common.cuh"
 #include "epilogue.cuh"
+#include "fp8_blockwise_call.cuh"
 #include "sm100_ptx.cuh"
 #include "tensormap.cuh"
 
@@ -89,10 +92,7 @@ struct Shape {
   static_assert(STAGE_BYTES % 1024 == 0, "stages must keep the 1024-byte alignment of the swizzled tiles");
   static_assert(SMEM_BYTES <= 232448, "shared memory of one CTA per SM");
 };
-// 20 warps = 5 per scheduler leave 96 registers per thread; 21 would leave 80
-using ShapeTiny = Shape<32, 10, 4, 2, 2>;    // rows <= 32:   20 KB stages, 200 KB in flight; 13 warps
-using ShapeSmall = Shape<64, 8, 4, 1, 2>;    // rows 33..64:  24 KB stages; 20 warps
-using ShapeFull = Shape<128, 6, 2, 1, 1>;    // rows >= 65:   32 KB stages; 20 warps
+using FewRows = Shape<FEW_ROWS, 10, 4, 2, 2>;    // 20 KB stages, 200 KB in flight; 13 warps
 
 __device__ uint32_t g_status = 0;
 
@@ -136,21 +136,19 @@ struct TileWalk {
   }
 };
 
-// One CTA of shape S: `block` of the `blocks` CTAs that serve the experts with min_rows <= rows <= max_rows.  The tensor
-// maps are the kernel's __grid_constant__ parameters.
-template <typename OutT, class S>
-__device__ __forceinline__ void blockwise_cta(const CUtensorMap& map_w, const CUtensorMap& map_x16,
-                                              const CUtensorMap& map_x32, const CUtensorMap& map_x64,
-                                              const CUtensorMap& map_x128, const float* __restrict__ scales_a,
-                                              const float* __restrict__ scales_b, OutT* __restrict__ d,
-                                              const int* __restrict__ problem_sizes,
-                                              const int* __restrict__ expert_offsets, int num_experts, int n, int k,
-                                              int min_rows, int max_rows, int wait_at_start, int group, int block,
-                                              int blocks) {
+// One CTA per SM; serves the experts with 1 .. FEW_ROWS rows.  First kernel of its call.
+template <typename OutT>
+__global__ void __launch_bounds__(FewRows::THREADS, 1)
+fp8_blockwise_grouped_mm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x16,
+                                const __grid_constant__ CUtensorMap map_x32, const float* __restrict__ scales_a,
+                                const float* __restrict__ scales_b, OutT* __restrict__ d,
+                                const int* __restrict__ problem_sizes, const int* __restrict__ expert_offsets,
+                                int num_experts, int n, int k, int group) {
+  using S = FewRows;
+  const int block = (int)blockIdx.x, blocks = (int)gridDim.x;
   constexpr int TOK = S::TOK_TILE;
   constexpr int STAGES = S::STAGES;
   constexpr int NCH = S::NCH;
-  if (!wait_at_start) pdl_launch_dependents();   // not the first kernel of its call: the next one may launch at once
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   float* chunks = reinterpret_cast<float*>(smem + (size_t)STAGES * S::STAGE_BYTES);        // [NCH][CH_KT][TOK]
@@ -180,35 +178,32 @@ __device__ __forceinline__ void blockwise_cta(const CUtensorMap& map_w, const CU
     ptx::prefetch_tensormap(&map_w);
     ptx::prefetch_tensormap(&map_x16);
     ptx::prefetch_tensormap(&map_x32);
-    ptx::prefetch_tensormap(&map_x64);
-    ptx::prefetch_tensormap(&map_x128);
   }
   if (warp == 1) {
     ptx::tmem_alloc(&ctl->tmem_base, S::TMEM_COLS);
     ptx::tmem_relinquish();
   }
-  // The first kernel of a call waits for the stream's earlier work and then lets the other buckets' kernels start;
-  // those write disjoint rows of d and only wait for their predecessor before they exit (stream order).
-  if (wait_at_start) pdl_wait_prior_grid();
+  // This kernel waits for the stream's earlier work and then lets the many-rows kernel of the call start; that one writes
+  // other rows of d and only waits for this one before it exits (stream order).
+  pdl_wait_prior_grid();
   const int n_tiles = n / TILE_N;
   block_exclusive_scan(num_experts, ctl->tile_prefix, ctl->warp_sums, [&](int e) {
     const int m = problem_sizes[e * 3];
-    return (m > 0 && m >= min_rows && m <= max_rows) ? ((m + TOK - 1) / TOK) * ((n_tiles + group - 1) / group) : 0;
+    return (m > 0 && m <= FEW_ROWS) ? (n_tiles + group - 1) / group : 0;
   });
   // a launch without work (the host only knows an upper bound of the rows per expert) ends here
   if (ctl->tile_prefix[num_experts] == 0) {
-    if (wait_at_start) pdl_launch_dependents();
+    pdl_launch_dependents();
     ptx::tc_fence_before_sync();
     __syncthreads();
     if (warp == 1) ptx::tmem_dealloc(ctl->tmem_base, S::TMEM_COLS);
-    if (!wait_at_start) pdl_wait_prior_grid();
     return;
   }
   const ExpertTable tab = fill_expert_table(ctl->tile_prefix, num_experts, problem_sizes, expert_offsets, nullptr);
   ptx::tc_fence_before_sync();
   __syncthreads();
   ptx::tc_fence_after_sync();
-  if (wait_at_start) pdl_launch_dependents();
+  pdl_launch_dependents();
 
   const uint32_t tmem_base = ctl->tmem_base;
   const int total_items = ctl->tile_prefix[num_experts];
@@ -223,8 +218,8 @@ __device__ __forceinline__ void blockwise_cta(const CUtensorMap& map_w, const CU
       TileWalk<TOK> walk(block, blocks);
       while (ok && walk.next(tab, num_experts, total_items, n_tiles, group)) {
         const TileInfo& ti = walk.ti;
-        const CUtensorMap* xm = ti.n_mma <= 16 ? &map_x16 : ti.n_mma <= 32 ? &map_x32 : ti.n_mma <= 64 ? &map_x64 : &map_x128;
-        const uint32_t box_rows = ti.n_mma <= 16 ? 16u : ti.n_mma <= 32 ? 32u : ti.n_mma <= 64 ? 64u : 128u;
+        const CUtensorMap* xm = ti.n_mma <= 16 ? &map_x16 : &map_x32;
+        const uint32_t box_rows = ti.n_mma <= 16 ? 16u : 32u;
         const uint32_t tx = W_BYTES + box_rows * TILE_K;
         const int w_row = ti.e * n + ti.nt * TILE_N;
         for (int kt = 0; kt < kt_count; ++kt) {
@@ -445,57 +440,7 @@ __device__ __forceinline__ void blockwise_cta(const CUtensorMap& map_w, const CU
     __syncwarp();
     ptx::tmem_dealloc(tmem_base, S::TMEM_COLS);
   }
-  if (!wait_at_start) pdl_wait_prior_grid();   // do not complete before the preceding kernel of this call has
 }
-
-template <typename OutT, class S>
-__global__ void __launch_bounds__(S::THREADS, 1)
-fp8_blockwise_grouped_mm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x16,
-                                const __grid_constant__ CUtensorMap map_x32, const __grid_constant__ CUtensorMap map_x64,
-                                const __grid_constant__ CUtensorMap map_x128, const float* __restrict__ scales_a,
-                                const float* __restrict__ scales_b, OutT* __restrict__ d,
-                                const int* __restrict__ problem_sizes, const int* __restrict__ expert_offsets,
-                                int num_experts, int n, int k, int min_rows, int max_rows, int wait_at_start, int group) {
-  blockwise_cta<OutT, S>(map_w, map_x16, map_x32, map_x64, map_x128, scales_a, scales_b, d, problem_sizes, expert_offsets,
-                         num_experts, n, k, min_rows, max_rows, wait_at_start, group, (int)blockIdx.x, (int)gridDim.x);
-}
-
-// The 64-token and the 128-token shape in one launch (both run 20 warps): CTAs [0, small_ctas) serve the experts with
-// 33..64 rows, the others those with 65 rows and more.  The hardware starts CTAs in index order, so the second shape
-// takes the SMs as the first runs out of items — what two chained launches did, for one launch (and, when a bucket is
-// empty, one pass of empty CTAs over every SM) less per call.
-template <typename OutT>
-__global__ void __launch_bounds__(ShapeSmall::THREADS, 1)
-fp8_blockwise_two_shapes_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x16,
-                                const __grid_constant__ CUtensorMap map_x32, const __grid_constant__ CUtensorMap map_x64,
-                                const __grid_constant__ CUtensorMap map_x128, const float* __restrict__ scales_a,
-                                const float* __restrict__ scales_b, OutT* __restrict__ d,
-                                const int* __restrict__ problem_sizes, const int* __restrict__ expert_offsets,
-                                int num_experts, int n, int k, int small_ctas, int wait_at_start, int group) {
-  static_assert(ShapeSmall::THREADS == ShapeFull::THREADS, "the two shapes share one block size");
-  if ((int)blockIdx.x < small_ctas)
-    blockwise_cta<OutT, ShapeSmall>(map_w, map_x16, map_x32, map_x64, map_x128, scales_a, scales_b, d, problem_sizes,
-                                    expert_offsets, num_experts, n, k, 33, 64, wait_at_start, group, (int)blockIdx.x,
-                                    small_ctas);
-  else
-    blockwise_cta<OutT, ShapeFull>(map_w, map_x16, map_x32, map_x64, map_x128, scales_a, scales_b, d, problem_sizes,
-                                   expert_offsets, num_experts, n, k, 65, 0x7fffffff, wait_at_start, group,
-                                   (int)blockIdx.x - small_ctas, (int)gridDim.x - small_ctas);
-}
-
-struct LaunchArgs {
-  const void* a;
-  const void* b;
-  const float* sa;
-  const float* sb;
-  void* d;
-  const int32_t* ps;
-  const int32_t* eo;
-  int num_experts;
-  int64_t num_rows;
-  int n, k;
-  cudaStream_t stream;
-};
 
 // weight tiles per work item: the per-item work of every role (decode) is spread over ~8 K blocks
 static int tiles_per_item(int k) {
@@ -504,118 +449,54 @@ static int tiles_per_item(int k) {
   return group < 1 ? 1 : group;
 }
 
-static int make_maps(const LaunchArgs& c, CUtensorMap* map_w, CUtensorMap (&map_x)[4]) {
-  int rc = make_tensormap_u8_sw128(map_w, c.b, (uint64_t)c.num_experts * c.n, (uint64_t)c.k, TILE_N);
+template <typename OutT>
+int launch_few_rows(const CallArgs& c) {
+  using S = FewRows;
+  DeviceInfo info;
+  int rc = get_device_info(&info);
   if (rc != ES_B200_OK) return rc;
-  const uint32_t boxes[4] = {16, 32, 64, 128};
-  for (int i = 0; i < 4; ++i) {
-    rc = make_tensormap_u8_sw128(&map_x[i], c.a, (uint64_t)c.num_rows, (uint64_t)c.k, boxes[i]);
-    if (rc != ES_B200_OK) return rc;
-  }
-  return ES_B200_OK;
-}
-
-// CTAs for one shape: one per SM, fewer when the host-known upper bound of its item count is smaller
-template <class S>
-static int ctas_for(const LaunchArgs& c, int group, int sm_count) {
-  const int64_t max_items = ((c.num_rows + S::TOK_TILE - 1) / S::TOK_TILE + c.num_experts) *
-                            (int64_t)((c.n / TILE_N + group - 1) / group);
-  return (int)(max_items < sm_count ? max_items : sm_count);
-}
-
-template <typename Kernel>
-static int configure(Kernel kernel, size_t smem_bytes, bool (&configured)[64]) {
+  CUtensorMap map_w, map_x16, map_x32;
+  rc = make_tensormap_u8_sw128(&map_w, c.b, (uint64_t)c.num_experts * c.n, (uint64_t)c.k, TILE_N);
+  if (rc == ES_B200_OK) rc = make_tensormap_u8_sw128(&map_x16, c.a, (uint64_t)c.num_rows, (uint64_t)c.k, 16);
+  if (rc == ES_B200_OK) rc = make_tensormap_u8_sw128(&map_x32, c.a, (uint64_t)c.num_rows, (uint64_t)c.k, 32);
+  if (rc != ES_B200_OK) return rc;
+  auto kernel = fp8_blockwise_grouped_mm_kernel<OutT>;
+  static bool configured[64] = {false};
   int dev = 0;
   ES_CUDA_TRY(cudaGetDevice(&dev));
   if (!configured[dev & 63]) {
-    ES_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes));
+    ES_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::SMEM_BYTES));
     configured[dev & 63] = true;
   }
-  return ES_B200_OK;
-}
-
-static void pdl_config(cudaLaunchConfig_t* cfg, cudaLaunchAttribute* attr, int grid, int threads, size_t smem,
-                       cudaStream_t stream) {
-  *cfg = {};
-  cfg->gridDim = dim3(grid);
-  cfg->blockDim = dim3(threads);
-  cfg->dynamicSmemBytes = smem;
-  cfg->stream = stream;
+  const int group = tiles_per_item(c.k);
+  // one CTA per SM, fewer when the host-known upper bound of the item count is smaller
+  const int64_t experts = c.num_experts < c.num_rows ? c.num_experts : c.num_rows;
+  const int64_t max_items = experts * ((c.n / TILE_N + group - 1) / group);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(max_items < info.sm_count ? max_items : info.sm_count));
+  cfg.blockDim = dim3(S::THREADS);
+  cfg.dynamicSmemBytes = S::SMEM_BYTES;
+  cfg.stream = c.stream;
+  cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg->attrs = attr;
-  cfg->numAttrs = 1;
-}
-
-// the <= 32-row shape (13 warps), always the first kernel of a call
-template <typename OutT>
-int launch_tiny(const LaunchArgs& c) {
-  using S = ShapeTiny;
-  DeviceInfo info;
-  int rc = get_device_info(&info);
-  if (rc != ES_B200_OK) return rc;
-  CUtensorMap map_w, map_x[4];
-  rc = make_maps(c, &map_w, map_x);
-  if (rc != ES_B200_OK) return rc;
-  auto kernel = fp8_blockwise_grouped_mm_kernel<OutT, S>;
-  static bool configured[64] = {false};
-  rc = configure(kernel, S::SMEM_BYTES, configured);
-  if (rc != ES_B200_OK) return rc;
-  const int group = tiles_per_item(c.k);
-  cudaLaunchConfig_t cfg;
-  cudaLaunchAttribute attr[1];
-  pdl_config(&cfg, attr, ctas_for<S>(c, group, info.sm_count), S::THREADS, S::SMEM_BYTES, c.stream);
-  ES_CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, map_w, map_x[0], map_x[1], map_x[2], map_x[3], c.sa, c.sb,
-                                 static_cast<OutT*>(c.d), c.ps, c.eo, c.num_experts, c.n, c.k, 1, 32, 1, group));
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  ES_CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, map_w, map_x16, map_x32, c.sa, c.sb, static_cast<OutT*>(c.d), c.ps, c.eo,
+                                 c.num_experts, c.n, c.k, group));
   return ES_B200_OK;
-}
-
-// the 33..64-row and the >= 65-row shapes in one launch; want_full = false leaves the first alone
-template <typename OutT>
-int launch_small_and_full(const LaunchArgs& c, bool want_full) {
-  DeviceInfo info;
-  int rc = get_device_info(&info);
-  if (rc != ES_B200_OK) return rc;
-  CUtensorMap map_w, map_x[4];
-  rc = make_maps(c, &map_w, map_x);
-  if (rc != ES_B200_OK) return rc;
-  auto kernel = fp8_blockwise_two_shapes_kernel<OutT>;
-  constexpr size_t SMEM = ShapeSmall::SMEM_BYTES > ShapeFull::SMEM_BYTES ? ShapeSmall::SMEM_BYTES : ShapeFull::SMEM_BYTES;
-  static bool configured[64] = {false};
-  rc = configure(kernel, SMEM, configured);
-  if (rc != ES_B200_OK) return rc;
-  const int group = tiles_per_item(c.k);
-  const int small_ctas = ctas_for<ShapeSmall>(c, group, info.sm_count);
-  const int full_ctas = want_full ? ctas_for<ShapeFull>(c, group, info.sm_count) : 0;
-  cudaLaunchConfig_t cfg;
-  cudaLaunchAttribute attr[1];
-  pdl_config(&cfg, attr, small_ctas + full_ctas, ShapeSmall::THREADS, SMEM, c.stream);
-  ES_CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, map_w, map_x[0], map_x[1], map_x[2], map_x[3], c.sa, c.sb,
-                                 static_cast<OutT*>(c.d), c.ps, c.eo, c.num_experts, c.n, c.k, small_ctas, 0, group));
-  return ES_B200_OK;
-}
-
-template <typename OutT>
-int launch_buckets(const void* a, const void* b, const float* sa, const float* sb, void* d, const int32_t* ps,
-                   const int32_t* eo, int num_experts, int64_t num_rows, int n, int k, cudaStream_t stream) {
-  // The <= 32-row shape first, then the two larger shapes in one launch, chained with programmatic dependent launch;
-  // every CTA filters the experts in its own scan.  A bucket that even the host-known upper bound of rows per expert
-  // cannot reach gets no CTAs.
-  const LaunchArgs c = {a, b, sa, sb, d, ps, eo, num_experts, num_rows, n, k, stream};
-  int rc = launch_tiny<OutT>(c);
-  if (rc != ES_B200_OK || num_rows <= 32) return rc;
-  return launch_small_and_full<OutT>(c, num_rows > 64);
 }
 
 int read_and_clear_status(uint32_t* out) {
-  uint32_t v = 0;
+  uint32_t v = 0, many = 0;
   ES_CUDA_TRY(cudaMemcpyFromSymbol(&v, g_status, sizeof(v)));
   if (v != 0) {
     uint32_t zero = 0;
     ES_CUDA_TRY(cudaMemcpyToSymbol(g_status, &zero, sizeof(zero)));
   }
-  *out = v;
-  return ES_B200_OK;
+  const int rc = read_and_clear_status_many_rows(&many);
+  *out = v | many;
+  return rc;
 }
 
 }  // namespace bw
@@ -641,10 +522,12 @@ extern "C" int es_b200_fp8_blockwise_grouped_mm(const void* a, const void* b, co
   ES_REQUIRE(aligned16(a) && aligned16(b) && aligned16(d), "a, b and d must be 16-byte aligned");
   ES_REQUIRE((reinterpret_cast<uintptr_t>(scales_a) & 3u) == 0 && (reinterpret_cast<uintptr_t>(scales_b) & 3u) == 0,
              "scales must be 4-byte aligned");
-  cudaStream_t s = static_cast<cudaStream_t>(stream);
-  if (out_dtype == ES_B200_BF16)
-    return bw::launch_buckets<__nv_bfloat16>(a, b, scales_a, scales_b, d, problem_sizes, expert_offsets, num_experts,
-                                             num_rows, n, k, s);
-  return bw::launch_buckets<__half>(a, b, scales_a, scales_b, d, problem_sizes, expert_offsets, num_experts, num_rows,
-                                    n, k, s);
+  // The few-rows kernel first, then the many-rows kernel; every CTA filters the experts in its own scan.  A bucket that
+  // even the host-known upper bound of rows per expert cannot reach gets no launch.
+  const bw::CallArgs c = {a, b, scales_a, scales_b, d, problem_sizes, expert_offsets, num_experts, num_rows, n, k,
+                          static_cast<cudaStream_t>(stream)};
+  const bool bf16 = out_dtype == ES_B200_BF16;
+  const int rc = bf16 ? bw::launch_few_rows<__nv_bfloat16>(c) : bw::launch_few_rows<__half>(c);
+  if (rc != ES_B200_OK || num_rows <= bw::FEW_ROWS) return rc;
+  return bf16 ? bw::launch_many_rows_bf16(c) : bw::launch_many_rows_fp16(c);
 }

@@ -93,3 +93,27 @@ def test_blockwise_rejects_bad_arguments():
         op(torch.zeros((4, 128), dtype=torch.float32, device=dev), a, b, sa, sb, st, st, st, ps, eo, ws)
     with pytest.raises(RuntimeError, match="problem_sizes must be int32"):
         op(torch.zeros((4, 128), dtype=torch.bfloat16, device=dev), a, b, sa, sb, st, st, st, ps.long(), eo, ws)
+
+
+@pytest.mark.parametrize("counts,N,K", [
+    ([33], 128, 128),                                    # one K block, one tile
+    ([32, 33, 64, 65, 128, 129, 256, 257], 384, 640),    # edges of the split, of the token boxes and of the 128-row tiles
+    ([96] * 40, 1024, 1280),                             # ten K blocks: scales read four at a time with a rest of two
+    ([40] * 160, 640, 256),                              # short tiles: more than 32 tiles per CTA in the work list
+])
+def test_blockwise_many_rows_edges(counts, N, K):
+    """Experts of more than 32 rows; an output and scales whose base is only 16- and 4-byte aligned gives the same bits."""
+    from expert_specialization_moe_b200 import es_fp8_blockwise_scaled_grouped_mm as op
+    inp = C.fp8_blockwise_inputs(counts, N, K, seed=17)
+    d = C.run_fp8_blockwise_op(inp)
+    _check(inp, d, torch.bfloat16)
+    T, dev = sum(counts), "cuda"
+    out = torch.zeros(T * N + 8, dtype=torch.bfloat16, device=dev)[8:].view(T, N)
+    sa = torch.zeros(T * (K // 128) + 1, device=dev)[1:].view(T, K // 128)
+    sa.copy_(inp["sa"])
+    ld = torch.full((len(counts),), K, dtype=torch.int64, device=dev)
+    op(out, inp["a_q"].to(dev), inp["w_q"].to(dev).transpose(1, 2), sa, inp["sb"].to(dev).transpose(1, 2), ld, ld, ld,
+       torch.from_numpy(inp["ps"]).to(dev), torch.from_numpy(inp["eo"]).to(dev),
+       torch.empty(16, dtype=torch.uint8, device=dev))
+    torch.cuda.synchronize()
+    assert torch.equal(out.cpu(), d)
