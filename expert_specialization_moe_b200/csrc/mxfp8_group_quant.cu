@@ -9,11 +9,11 @@
 //   code  = cvt.rn.satfinite.e4m3x2.f32(fp32(x_i) * inv)
 //
 // Schedule: an expert's rows are one contiguous stream of 128-element K tiles (rows are densely packed), whatever k is.
-// Eight lanes take a tile, sixteen elements each; a warp takes four consecutive tiles per step and `steps` steps per
-// work unit.  Units of all experts form one flat list found with a per-CTA prefix scan over the row counts, so neither
-// the split of the rows between experts nor k leaves lanes idle, and a call of a few rows is spread over as many warps
-// as it has tiles (the host picks `steps` from the row count).  Zeroing the scale bytes of the padding rows is work
-// units of its own, in 16-byte pieces: in a decode call they are as many bytes as the codes.
+// Eight lanes take a tile, sixteen elements each, a CTA 32 consecutive tiles per step.  The steps of all experts form one
+// flat list (a per-CTA prefix scan over the row counts) that the resident CTAs share evenly: neither the split of the rows
+// between experts nor k leaves lanes or CTAs idle.  (Work units of 16 steps of a warp dealt round-robin came to 6.05 units
+// per warp, so 7, at 32768 x 7168.)  Zeroing the scale bytes of the padding rows is steps of its own, in 16-byte pieces: in
+// a decode call they are as many bytes as the codes.
 //
 // What bounds it: HBM (3 + 1/32 bytes per element; with silu 5 + 1/32).  One lane per 8 elements and a warp per row
 // cost 10.5 instructions per element, enough to keep the issue slots 62 % busy; 16 elements per lane halve the scale
@@ -31,62 +31,83 @@ namespace es_b200 {
 
 constexpr int QUANT_THREADS = 256;
 constexpr int QUANT_WARPS = QUANT_THREADS / 32;
-constexpr int QUANT_TILES_PER_STEP = 4;       // a warp's four groups of eight lanes, one 128-element K tile each
-constexpr int QUANT_PAD_ATOMS = 16;           // scale atoms per unit of padding work
-constexpr int QUANT_MAX_STEPS_LOG2 = 4;
+constexpr int QUANT_WARP_TILES = 4;           // a warp's four groups of eight lanes, one 128-element K tile each
+constexpr int QUANT_STEP_TILES = QUANT_WARPS * QUANT_WARP_TILES;
+constexpr int QUANT_PAD_ATOMS = 16;           // scale atoms per warp and step of padding work
+// Consecutive steps that a CTA takes before it moves on by a grid's worth: an equal share of the list in one stretch, but
+// eight steps where the share is long and the kernel is bound by memory — 592 streams 0.8 MB apart cost it 10 % of the
+// bandwidth (32768 x 7168: 134 us in one stretch, 121 in chunks of 8, 125 of 4, 140 of 2; with silu, bound by its
+// arithmetic, 106 us either way, and the last round of chunks is not paid for).
+constexpr int QUANT_CHUNK = 8, QUANT_LONG_SHARE = 48;
 // registers: two steps of input in flight per warp; the fused variant holds gate and up of both
 constexpr int QUANT_MIN_BLOCKS = 4, QUANT_MIN_BLOCKS_SILU = 3;
 
 // exact arithmetic of an unfused silu(gate.float()) * up.float() -> T: accurate expf, IEEE division and multiply
 __device__ __forceinline__ float silu_mul_exact(float g, float u) { return (g / (1.0f + expf(-g))) * u; }
 
-// act = round_to_T( silu(gate) * up ) on two elements, bit for bit what silu_mul_exact gives, for a quarter of its
+// act = round_to_T( silu(gate) * up ) on 16 elements, bit for bit what silu_mul_exact gives, for a third of its
 // instructions: p = g * rcp(1 + 2^(-g log2 e)) * u with the hardware approximations is within `eps` (relative) of the
 // exact sequence's fp32 value, so wherever p (1 - eps) and p (1 + eps) round to the same 16-bit value, that value is the
-// answer (rounding is monotonic); the few pairs where they do not (bf16: 0.04 % of the elements) take the exact
-// sequence.  `wild` sends a pair there too: |g| > 64, where 1 + 2^x can leave the range of the approximate reciprocal.
+// answer (rounding is monotonic); the few pairs where they do not (bf16: 0.04 % of the elements) take the exact sequence.
 // Error of p against the exact sequence, in units of 2^-24: 2^x 4 (2 ulp), its argument |g| (one rounding of g log2 e
 // and of the constant), reciprocal 2 (1 ulp), sum and two products 3 x 1; exact sequence: expf 2 (1 ulp), sum, quotient
-// and product 3 x 1; rounding of the two bounds 2.  16 + |g| in all; eps = (24 + 1.5 |g|) 2^-24.
-// bf16 gates and results below 2^-100 (zeros among them) also go the exact way: the bounds are relative, and next to
-// the fp32 subnormals a relative bound says nothing.  fp16 values are at least 2^-24, so q and p cannot get there.
+// and product 3 x 1; rounding of the two bounds 2.  16 + |g| in all; eps = (24 + 1.5 |g|) 2^-24 with the lane's largest g.
+// Lanes with an element outside the range in which these relative bounds hold go the exact way altogether: |g| > 64
+// (1 + 2^x can leave the range of the approximate reciprocal), and in bf16 |g| or |u| < 2^-36 (zeros among them: with
+// g = -64 the product is then 2^-122, next to the fp32 subnormals).  fp16 values are zero, which is exact, or at least
+// 2^-24.
 template <typename T>
-__device__ __forceinline__ uint32_t silu_mul2(uint32_t gw, uint32_t uw, float eps, bool wild) {
+__device__ __forceinline__ void silu_mul16(const uint32_t (&g)[8], const uint32_t (&u)[8], uint32_t (&out)[8]) {
   using V2 = typename Vec2<T>::type;
-  const float2 g = Vec2<T>::to_float2(*reinterpret_cast<const V2*>(&gw));
-  const float2 u = Vec2<T>::to_float2(*reinterpret_cast<const V2*>(&uw));
-  const float2 t = mul2(g, make_float2(-1.4426950408889634f, -1.4426950408889634f));
-  const float2 d = add2(make_float2(ex2_approx_ftz(t.x), ex2_approx_ftz(t.y)), make_float2(1.0f, 1.0f));
-  const float2 q = mul2(g, make_float2(rcp_approx_ftz(d.x), rcp_approx_ftz(d.y)));
-  const float2 p = mul2(q, u);
-  const float2 hi = fma2(p, make_float2(eps, eps), p);
-  const float2 lo = fma2(p, make_float2(-eps, -eps), p);
-  V2 r = Vec2<T>::from_floats(hi.x, hi.y);
-  const V2 r2 = Vec2<T>::from_floats(lo.x, lo.y);
-  uint32_t out = *reinterpret_cast<const uint32_t*>(&r);
-  uint32_t differ = out ^ *reinterpret_cast<const uint32_t*>(&r2);
+  const float g_max = max_abs16<T>(g);
+  bool irregular = !(g_max <= 64.0f);
   if constexpr (std::is_same<T, __nv_bfloat16>::value) {
-    const uint32_t limit = 0x0d800d80u;      // 2^-100 twice
-    differ |= __hlt2_mask(__habs2(r), *reinterpret_cast<const V2*>(&limit)) |
-              __hlt2_mask(__habs2(*reinterpret_cast<const V2*>(&gw)), *reinterpret_cast<const V2*>(&limit));
+    const uint32_t least = min_magnitude2(min_magnitude16(g), min_magnitude16(u)) & 0x7fff7fffu;
+    irregular |= (least & 0xffffu) < 0x2d80u || least < 0x2d800000u;      // 2^-36
   }
-  if (differ != 0 || wild) {
-    r = Vec2<T>::from_floats(silu_mul_exact(g.x, u.x), silu_mul_exact(g.y, u.y));
-    out = *reinterpret_cast<const uint32_t*>(&r);
+  const float eps = fmaf(g_max, 8.940696716e-8f, 1.430511475e-6f);      // (24 + 1.5 |g|) 2^-24
+  uint32_t undecided = irregular ? 0xffu : 0u;      // one bit per pair
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const float2 gf = Vec2<T>::to_float2(*reinterpret_cast<const V2*>(&g[i]));
+    const float2 uf = Vec2<T>::to_float2(*reinterpret_cast<const V2*>(&u[i]));
+    const float2 t = mul2(gf, make_float2(-1.4426950408889634f, -1.4426950408889634f));
+    const float2 d = add2(make_float2(ex2_approx_ftz(t.x), ex2_approx_ftz(t.y)), make_float2(1.0f, 1.0f));
+    const float2 p = mul2(mul2(gf, make_float2(rcp_approx_ftz(d.x), rcp_approx_ftz(d.y))), uf);
+    const float2 hi = fma2(p, make_float2(eps, eps), p);
+    const float2 lo = fma2(p, make_float2(-eps, -eps), p);
+    const V2 r_hi = Vec2<T>::from_floats(hi.x, hi.y), r_lo = Vec2<T>::from_floats(lo.x, lo.y);
+    out[i] = *reinterpret_cast<const uint32_t*>(&r_hi);
+    if (out[i] != *reinterpret_cast<const uint32_t*>(&r_lo)) undecided |= 1u << i;
   }
-  return out;
+  // no branch above: the sixteen chains overlap.  One undecided pair per turn here (a warp's step has one in 18 %).
+  while (undecided != 0) {
+    const int i = __ffs((int)undecided) - 1;
+    undecided &= undecided - 1;
+    uint32_t gw = g[0], uw = u[0];
+#pragma unroll
+    for (int j = 1; j < 8; ++j) {
+      if (i == j) { gw = g[j]; uw = u[j]; }
+    }
+    const float2 gf = Vec2<T>::to_float2(*reinterpret_cast<const V2*>(&gw));
+    const float2 uf = Vec2<T>::to_float2(*reinterpret_cast<const V2*>(&uw));
+    const V2 r = Vec2<T>::from_floats(silu_mul_exact(gf.x, uf.x), silu_mul_exact(gf.y, uf.y));
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      if (i == j) out[j] = *reinterpret_cast<const uint32_t*>(&r);
+    }
+  }
 }
 
-// 32 bytes of input per lane: one 256-bit load where the tensor starts on a 32-byte boundary (tiles are multiples of
-// 256 bytes), two 128-bit loads otherwise
+// 32 bytes of input per lane (v is left alone where `on` is false): one 256-bit load where the tensor starts on a 32-byte
+// boundary (tiles are multiples of 256 bytes), two 128-bit loads otherwise
 template <bool kWide>
-__device__ __forceinline__ void load_16_elements(const void* p, uint32_t (&v)[8]) {
+__device__ __forceinline__ void load_16_elements(const void* p, bool on, uint32_t (&v)[8]) {
   if constexpr (kWide) {
-    ld_stream_32B(p, v);
+    ld_stream_32B_if(p, on, v);
   } else {
-    const uint4 a = ld_stream_16B(p), b = ld_stream_16B(static_cast<const uint8_t*>(p) + 16);
-    v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
-    v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+    ld_stream_16B_if(p, on, v[0], v[1], v[2], v[3]);
+    ld_stream_16B_if(static_cast<const uint8_t*>(p) + 16, on, v[4], v[5], v[6], v[7]);
   }
 }
 
@@ -96,43 +117,48 @@ __global__ void __launch_bounds__(QUANT_THREADS, kSiluMul ? QUANT_MIN_BLOCKS_SIL
 mxfp8_group_quant_kernel(const T* __restrict__ input, const int* __restrict__ problem_sizes,
                          const int* __restrict__ expert_offsets, const int* __restrict__ blockscale_offsets,
                          uint8_t* __restrict__ quant_output, uint8_t* __restrict__ scale_factor, int num_experts,
-                         int k, int steps_log2) {
+                         int k) {
   __shared__ int table[ES_B200_MAX_EXPERTS + 1];
   __shared__ int warp_sums[32];
 
   const int kt = k >> 7;                          // K tiles (= 32-bit scale words) per row
-  const int unit_log2 = 2 + steps_log2;           // tiles per unit, as a power of two
-  const int pad_units = (kt + QUANT_PAD_ATOMS - 1) / QUANT_PAD_ATOMS;
+  const int step_rows = QUANT_STEP_TILES / kt, step_q = QUANT_STEP_TILES - step_rows * kt;
+  const int pad_steps = (kt + QUANT_WARPS * QUANT_PAD_ATOMS - 1) / (QUANT_WARPS * QUANT_PAD_ATOMS);
   // (a tile is at least 256 bytes of input: 32 bits count the tiles of any tensor that fits the GPU)
-  auto data_units = [&](int m) { return (int)(((uint32_t)m * (uint32_t)kt + (1u << unit_log2) - 1u) >> unit_log2); };
+  auto data_steps = [&](int m) { return (int)(((uint32_t)m * (uint32_t)kt + QUANT_STEP_TILES - 1u) / QUANT_STEP_TILES); };
   pdl_wait_prior_grid();
   block_exclusive_scan(num_experts, table, warp_sums, [&](int e) {
     const int m = problem_sizes[e * 3];
-    return m > 0 ? data_units(m) + ((m & 127) ? pad_units : 0) : 0;
+    return m > 0 ? data_steps(m) + ((m & 127) ? pad_steps : 0) : 0;
   });
   const ExpertTable tab = fill_expert_table(table, num_experts, problem_sizes, expert_offsets, blockscale_offsets);
   __syncthreads();
   pdl_launch_dependents();
-  const int total_units = table[num_experts];
+  const int total = tab.prefix[num_experts];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int first_tile = warp * QUANT_WARP_TILES;                // of a step's 32 tiles
+  const int group = lane >> 3, l8 = lane & 7;     // this lane's tile of the warp's four, and its 16 elements of the tile
 
-  const int lane = threadIdx.x & 31;
-  const int group = lane >> 3, l8 = lane & 7;     // this lane's tile of the step, and its 16 elements of the tile
-
-  // neighbouring units on neighbouring SMs first: a call of few units is spread over the whole GPU
-  for (int u = (threadIdx.x >> 5) * gridDim.x + blockIdx.x; u < total_units; u += gridDim.x * QUANT_WARPS) {
-    const int e = upper_bound_expert(tab.prefix, num_experts, u);
+  const int share = (total + (int)gridDim.x - 1) / (int)gridDim.x;
+  const int chunk = (kSiluMul || share <= QUANT_LONG_SHARE) ? share : QUANT_CHUNK;
+  int u = (int)blockIdx.x * chunk, end = min(u + chunk, total);
+  if (u >= total) return;
+  int e = upper_bound_expert(tab.prefix, num_experts, u);
+  for (int run; u < end; ) {
+    while (tab.prefix[e + 1] <= u) ++e;             // empty experts share their prefix with the next one
     const int i = u - tab.prefix[e];
     const int m = tab.m(e);
     uint8_t* sf_expert = scale_factor + (int64_t)tab.scale0(e) * (k >> 5);
-    const int n_data = data_units(m);
+    const int n_data = data_steps(m);
     if (i >= n_data) {
+      run = 1;
       // scale bytes of the padding rows m .. align128(m) - 1: lane j clears, in each atom, the words of its line (rows
       // j, j + 32, j + 64, j + 96 of the last 128) that belong to rows past the end
       const int last = m & 127;
       const int first_word = last <= lane ? 0 : (last - lane + 31) >> 5;      // 0 .. 4
       uint8_t* line = sf_expert + (int64_t)(m >> 7) * kt * 512 + lane * 16;
-      const int q_end = min(kt, (i - n_data + 1) * QUANT_PAD_ATOMS);
-      for (int q = (i - n_data) * QUANT_PAD_ATOMS; q < q_end; ++q) {
+      const int q0 = ((i - n_data) * QUANT_WARPS + warp) * QUANT_PAD_ATOMS;
+      for (int q = q0; q < min(kt, q0 + QUANT_PAD_ATOMS); ++q) {
         uint32_t* words = reinterpret_cast<uint32_t*>(line + (int64_t)q * 512);
         if (first_word == 0 && (reinterpret_cast<uintptr_t>(words) & 15u) == 0) {
           *reinterpret_cast<uint4*>(words) = make_uint4(0, 0, 0, 0);
@@ -140,72 +166,91 @@ mxfp8_group_quant_kernel(const T* __restrict__ input, const int* __restrict__ pr
           for (int w = first_word; w < 4; ++w) words[w] = 0u;
         }
       }
-      continue;
-    }
-    const uint32_t t0 = ((uint32_t)i << unit_log2) + (uint32_t)group;               // this lane group's first tile
-    const int tiles_left = (int)((uint32_t)m * (uint32_t)kt - ((uint32_t)i << unit_log2));   // from the unit's first on
-    const int n_steps = min(1 << steps_log2, (tiles_left + QUANT_TILES_PER_STEP - 1) / QUANT_TILES_PER_STEP);
-    int row = (int)(t0 / (uint32_t)kt);
-    int q = (int)(t0 - (uint32_t)row * (uint32_t)kt);
-    int load_row = row, load_q = q;
-    const int64_t row0 = tab.row0(e);
-    const T* src = input + row0 * (kSiluMul ? 2 * (int64_t)k : (int64_t)k) + l8 * 16;
-    uint8_t* dst = quant_output + (row0 * kt + t0) * 128 + l8 * 16;
+    } else {
+      run = min(end - u, n_data - i);
+      const uint32_t t0 = (uint32_t)i * QUANT_STEP_TILES + (uint32_t)(first_tile + group);    // this lane group's first tile
+      // tiles from the warp's first on; the same number of steps for all its lanes: the shuffles need them
+      const int warp_left = (int)((uint32_t)m * (uint32_t)kt - (uint32_t)i * QUANT_STEP_TILES) - first_tile;
+      const int n_steps = min(run, (warp_left + QUANT_STEP_TILES - 1) / QUANT_STEP_TILES);
+      int row = (int)(t0 / (uint32_t)kt);
+      int q = (int)(t0 - (uint32_t)row * (uint32_t)kt);
+      int load_q = q;
+      const int64_t row0 = tab.row0(e);
+      // gate tiles of one row and the next are kt tiles further apart than those inside a row
+      const T* src = input + (kSiluMul ? row0 * 2 * kt + t0 + (int64_t)row * kt : row0 * kt + t0) * 128 + l8 * 16;
+      uint8_t* dst = quant_output + (row0 * kt + t0) * 128 + l8 * 16;
+      int left = warp_left - group, load_left = left;       // tiles from this lane group's next one on: to do / to load
 
-    uint32_t raw[2][8], raw_up[kSiluMul ? 2 : 1][8];
-    auto load = [&](int s, uint32_t (&g)[8], uint32_t (&up)[8]) {
-      if (s < n_steps && s * QUANT_TILES_PER_STEP + group < tiles_left) {
+      auto load = [&](uint32_t (&g)[8], uint32_t (&up)[8]) {
+        const bool on = load_left > 0;
+        load_left -= QUANT_STEP_TILES;
+        load_16_elements<kWide>(src, on, g);
         if constexpr (kSiluMul) {
-          const T* p = src + ((int64_t)load_row * 2 * kt + load_q) * 128;
-          load_16_elements<kWide>(p, g);
-          load_16_elements<kWide>(p + k, up);
-          load_q += QUANT_TILES_PER_STEP;
-          while (load_q >= kt) { load_q -= kt; ++load_row; }
+          load_16_elements<kWide>(src + k, on, up);
+          load_q += step_q;
+          int skip = step_rows;
+          if (load_q >= kt) { load_q -= kt; ++skip; }
+          src += (QUANT_STEP_TILES + skip * kt) * 128;
         } else {
-          load_16_elements<kWide>(src + ((int64_t)t0 + s * QUANT_TILES_PER_STEP) * 128, g);
+          src += QUANT_STEP_TILES * 128;
+        }
+      };
+      // quantises the step in (g, up); the loads of the step after next go out in front of the quantisation, into `next`
+      // (silu: into the registers that the activation has just freed)
+      auto step = [&](uint32_t (&g)[8], uint32_t (&up)[8], uint32_t (&next)[8]) {
+        uint4 codes;
+        uint32_t sf;
+        if constexpr (kSiluMul) {
+          uint32_t v[8];
+          silu_mul16<T>(g, up, v);
+          load(g, up);
+          sf = quantize16<T>(v, codes);
+        } else {
+          load(next, up);
+          sf = quantize16<T>(g, codes);
+        }
+        // the four scale bytes of the tile as one aligned 32-bit word (two lanes hold the byte of a 32-element block)
+        uint32_t w = sf << ((l8 >> 1) * 8);
+        w |= __shfl_xor_sync(0xffffffffu, w, 2);
+        w |= __shfl_xor_sync(0xffffffffu, w, 4);
+        const bool on = left > 0;
+        left -= QUANT_STEP_TILES;
+        st_stream_16B_if(dst, on, codes);
+        dst += QUANT_STEP_TILES * 128;
+        // (an expert's scale bytes are 1/64 of its input: 32 bits address them)
+        const uint32_t at = ((uint32_t)(row >> 7) * (uint32_t)kt + (uint32_t)q) * 512u + (row & 31) * 16 + ((row & 127) >> 5) * 4;
+        st_4B_if(sf_expert + at, on && l8 == 0, w);
+        row += step_rows;
+        q += step_q;
+        if (q >= kt) { q -= kt; ++row; }
+      };
+      // two steps in flight besides the one at work; tiles past the end quantise zeros and store nothing
+      constexpr int BUFFERS = kSiluMul ? 2 : 3;
+      uint32_t raw[BUFFERS][8], raw_up[2][8];
+#pragma unroll
+      for (int b = 0; b < BUFFERS; ++b) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          raw[b][j] = 0u;
+          if (b < 2) raw_up[b][j] = 0u;
         }
       }
-    };
-    auto step = [&](int s, uint32_t (&g)[8], uint32_t (&up)[8]) {
-      uint32_t v[8];
-      if constexpr (kSiluMul) {
-        const float g_max = max_abs16<T>(g);
-        const bool wild = !(g_max <= 64.0f);
-        const float eps = fmaf(g_max, 8.940696716e-8f, 1.430511475e-6f);      // (24 + 1.5 |g|) 2^-24
-#pragma unroll
-        for (int j = 0; j < 8; ++j) v[j] = silu_mul2<T>(g[j], up[j], eps, wild);
-      } else {
-#pragma unroll
-        for (int j = 0; j < 8; ++j) v[j] = g[j];
-      }
-      load(s + 2, g, up);
-      uint4 codes;
-      const uint32_t sf = quantize16<T>(v, codes);
-      // the four scale bytes of the tile as one aligned 32-bit word (two lanes hold the byte of a 32-element block)
-      uint32_t w = sf << ((l8 >> 1) * 8);
-      w |= __shfl_xor_sync(0xffffffffu, w, 2);
-      w |= __shfl_xor_sync(0xffffffffu, w, 4);
-      if (s * QUANT_TILES_PER_STEP + group < tiles_left) {
-        st_stream_16B(dst + (int64_t)s * (QUANT_TILES_PER_STEP * 128), codes);
-        if (l8 == 0) *reinterpret_cast<uint32_t*>(sf_expert + scale_word_offset(row, kt) + (int64_t)q * 512) = w;
-      }
-      q += QUANT_TILES_PER_STEP;
-      while (q >= kt) { q -= kt; ++row; }
-    };
-#pragma unroll
-    for (int b = 0; b < 2; ++b) {
-#pragma unroll
-      for (int j = 0; j < 8; ++j) raw[b][j] = 0u;      // tiles past the end quantise zeros and store nothing
-      if constexpr (kSiluMul) {
-#pragma unroll
-        for (int j = 0; j < 8; ++j) raw_up[b][j] = 0u;
+      load(raw[0], raw_up[0]);
+      load(raw[1], raw_up[1]);
+      for (int s = 0; s < n_steps; ++s) {
+        step(raw[0], raw_up[0], raw[BUFFERS - 1]);
+        if (++s == n_steps) break;
+        step(raw[1], raw_up[1], raw[0]);
+        if constexpr (BUFFERS == 3) {
+          if (++s == n_steps) break;
+          step(raw[2], raw_up[0], raw[1]);
+        }
       }
     }
-    load(0, raw[0], raw_up[0]);
-    load(1, raw[1], raw_up[kSiluMul ? 1 : 0]);
-    for (int s = 0; s < n_steps; s += 2) {
-      step(s, raw[0], raw_up[0]);
-      if (s + 1 < n_steps) step(s + 1, raw[1], raw_up[kSiluMul ? 1 : 0]);
+    u += run;
+    if (u >= end) {                                 // on to the CTA's next chunk
+      u += ((int)gridDim.x - 1) * chunk;
+      end = min(u + chunk, total);
     }
   }
 }
@@ -225,15 +270,10 @@ static int launch_quant(const void* input, const int32_t* problem_sizes, const i
     blocks_per_sm = v > 0 ? v : 1;
   }
   const int64_t resident = (int64_t)info.sm_count * blocks_per_sm;
-  // steps per unit: as many as leave every resident warp about four units (a short tail), 16 at most
+  // at most one partial step and the padding steps per expert on top of the full steps of num_rows rows
   const int kt = k >> 7;
-  const int64_t steps_total = (num_rows * kt + QUANT_TILES_PER_STEP - 1) / QUANT_TILES_PER_STEP;
-  int steps_log2 = 0;
-  while (steps_log2 < QUANT_MAX_STEPS_LOG2 && (steps_total >> (steps_log2 + 1)) >= 4 * resident * QUANT_WARPS) ++steps_log2;
-  // at most one partial unit and the padding units per expert on top of the full units of num_rows rows
-  const int64_t max_units = (steps_total >> steps_log2) + 1 +
-                            (int64_t)num_experts * (1 + (kt + QUANT_PAD_ATOMS - 1) / QUANT_PAD_ATOMS);
-  const int64_t max_ctas = (max_units + QUANT_WARPS - 1) / QUANT_WARPS;
+  const int64_t max_ctas = (num_rows * kt + QUANT_STEP_TILES - 1) / QUANT_STEP_TILES +
+                           (int64_t)num_experts * (1 + (kt + QUANT_WARPS * QUANT_PAD_ATOMS - 1) / (QUANT_WARPS * QUANT_PAD_ATOMS));
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)(max_ctas < resident ? max_ctas : resident));
   cfg.blockDim = dim3(QUANT_THREADS);
@@ -244,8 +284,7 @@ static int launch_quant(const void* input, const int32_t* problem_sizes, const i
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   ES_CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, static_cast<const T*>(input), problem_sizes, expert_offsets,
-                                 blockscale_offsets, static_cast<uint8_t*>(quant_output), scale_factor, num_experts, k,
-                                 steps_log2));
+                                 blockscale_offsets, static_cast<uint8_t*>(quant_output), scale_factor, num_experts, k));
   return ES_B200_OK;
 }
 

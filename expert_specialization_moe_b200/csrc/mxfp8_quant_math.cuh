@@ -28,15 +28,45 @@ __device__ __forceinline__ uint4 ld_stream_16B(const void* p) {
   return v;
 }
 
+// Predicated streaming accesses: no branch around them, and the registers of a load that is off keep their value.
 // 32 bytes per lane in one instruction (sm_100); p must be 32-byte aligned
-__device__ __forceinline__ void ld_stream_32B(const void* p, uint32_t (&v)[8]) {
-  asm volatile("ld.global.nc.L1::no_allocate.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-               : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
-               : "l"(p));
+__device__ __forceinline__ void ld_stream_32B_if(const void* p, bool on, uint32_t (&v)[8]) {
+  asm volatile(
+      "{\n\t"
+      ".reg .pred P;\n\t"
+      "setp.ne.b32 P, %9, 0;\n\t"
+      "@P ld.global.nc.L1::no_allocate.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];\n\t"
+      "}"
+      : "+r"(v[0]), "+r"(v[1]), "+r"(v[2]), "+r"(v[3]), "+r"(v[4]), "+r"(v[5]), "+r"(v[6]), "+r"(v[7])
+      : "l"(p), "r"((int)on));
 }
-
-__device__ __forceinline__ void st_stream_16B(void* p, const uint4& v) {
-  asm volatile("st.global.cs.v4.u32 [%0], {%1,%2,%3,%4};" ::"l"(p), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
+__device__ __forceinline__ void ld_stream_16B_if(const void* p, bool on, uint32_t& a, uint32_t& b, uint32_t& c, uint32_t& d) {
+  asm volatile(
+      "{\n\t"
+      ".reg .pred P;\n\t"
+      "setp.ne.b32 P, %5, 0;\n\t"
+      "@P ld.global.nc.L1::no_allocate.v4.b32 {%0,%1,%2,%3}, [%4];\n\t"
+      "}"
+      : "+r"(a), "+r"(b), "+r"(c), "+r"(d)
+      : "l"(p), "r"((int)on));
+}
+__device__ __forceinline__ void st_stream_16B_if(void* p, bool on, const uint4& v) {
+  asm volatile(
+      "{\n\t"
+      ".reg .pred P;\n\t"
+      "setp.ne.b32 P, %5, 0;\n\t"
+      "@P st.global.cs.v4.b32 [%0], {%1,%2,%3,%4};\n\t"
+      "}" ::"l"(p), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w), "r"((int)on)
+      : "memory");
+}
+__device__ __forceinline__ void st_4B_if(void* p, bool on, uint32_t v) {
+  asm volatile(
+      "{\n\t"
+      ".reg .pred P;\n\t"
+      "setp.ne.b32 P, %2, 0;\n\t"
+      "@P st.global.b32 [%0], %1;\n\t"
+      "}" ::"l"(p), "r"(v), "r"((int)on)
+      : "memory");
 }
 
 __device__ __forceinline__ float ex2_approx_ftz(float a) {
@@ -157,6 +187,18 @@ __device__ __forceinline__ uint32_t max_magnitude16(const uint32_t (&v)[8]) {
   return max_magnitude2<T>(a, b);
 }
 
+// min(|a|, |b|) per half, the sign of the result unspecified; NaN members dropped
+__device__ __forceinline__ uint32_t min_magnitude2(uint32_t a, uint32_t b) {
+  uint32_t r;
+  asm("min.xorsign.abs.bf16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+  return r;
+}
+__device__ __forceinline__ uint32_t min_magnitude16(const uint32_t (&v)[8]) {
+  const uint32_t a = min_magnitude2(min_magnitude2(v[0], v[1]), min_magnitude2(v[2], v[3]));
+  const uint32_t b = min_magnitude2(min_magnitude2(v[4], v[5]), min_magnitude2(v[6], v[7]));
+  return min_magnitude2(a, b);
+}
+
 // larger magnitude of the two halves as fp32 (NaN only if both are)
 template <typename T>
 __device__ __forceinline__ float magnitude_of_pair(uint32_t m) {
@@ -172,6 +214,20 @@ __device__ __forceinline__ float max_abs16(const uint32_t (&v)[8]) {
   return magnitude_of_pair<T>(max_magnitude16<T>(v));
 }
 
+// four fp32 values -> four e4m3 codes, the first in the lowest byte
+__device__ __forceinline__ uint32_t e4m3x4(float2 lo, float2 hi) {
+  uint32_t r;
+  asm("{\n\t"
+      ".reg .b16 a, b;\n\t"
+      "cvt.rn.satfinite.e4m3x2.f32 a, %2, %1;\n\t"
+      "cvt.rn.satfinite.e4m3x2.f32 b, %4, %3;\n\t"
+      "mov.b32 %0, {a, b};\n\t"
+      "}"
+      : "=r"(r)
+      : "f"(lo.x), "f"(lo.y), "f"(hi.x), "f"(hi.y));
+  return r;
+}
+
 // Quantise the 16 elements this lane holds; two neighbouring lanes share one 32-element block.  Same arithmetic as
 // quantize8; returns the block's UE8M0 byte in both lanes.
 template <typename T>
@@ -180,19 +236,18 @@ __device__ __forceinline__ uint32_t quantize16(const uint32_t (&v)[8], uint4& co
   uint32_t mx = max_magnitude16<T>(v);
   mx = max_magnitude2<T>(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
   const float block_max = magnitude_of_pair<T>(mx);
-  __nv_fp8_e8m0 sf;
-  sf.__x = __nv_cvt_float_to_e8m0(block_max * rcp_approx_ftz(448.0f), __NV_SATFINITE, cudaRoundPosInf);
-  const float inv = block_max != 0.f ? rcp_approx_ftz(static_cast<float>(sf)) : 0.0f;
+  const uint32_t sf = __nv_cvt_float_to_e8m0(block_max * rcp_approx_ftz(448.0f), __NV_SATFINITE, cudaRoundPosInf);
+  // rcp.approx.ftz(2^(sf - 127)): 2^(127 - sf); the subnormal 2^-127 (sf = 0) counts as zero, 1 / 2^127 (254) flushes to
+  // zero; a block whose 32 members are all NaN has the scale NaN (255)
+  const uint32_t inv_bits = sf == 0 ? 0x7f800000u : sf == 255u ? 0x7fffffffu : (254u - sf) << 23;
+  const float inv = block_max != 0.f ? __uint_as_float(inv_bits) : 0.0f;
   uint32_t out[4];
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const float2 lo = mul2(Vec2<T>::to_float2(*reinterpret_cast<const V2*>(&v[2 * i])), make_float2(inv, inv));
-    const float2 hi = mul2(Vec2<T>::to_float2(*reinterpret_cast<const V2*>(&v[2 * i + 1])), make_float2(inv, inv));
-    out[i] = (uint32_t)__nv_cvt_float2_to_fp8x2(lo, __NV_SATFINITE, __NV_E4M3) |
-             ((uint32_t)__nv_cvt_float2_to_fp8x2(hi, __NV_SATFINITE, __NV_E4M3) << 16);
-  }
+  for (int i = 0; i < 4; ++i)
+    out[i] = e4m3x4(mul2(Vec2<T>::to_float2(*reinterpret_cast<const V2*>(&v[2 * i])), make_float2(inv, inv)),
+                    mul2(Vec2<T>::to_float2(*reinterpret_cast<const V2*>(&v[2 * i + 1])), make_float2(inv, inv)));
   codes = make_uint4(out[0], out[1], out[2], out[3]);
-  return sf.__x;
+  return sf;
 }
 
 // Byte offset, inside one operand's swizzled scale buffer, of the 32-bit scale word of (row r, K tile 0): 512-byte
