@@ -150,7 +150,7 @@ fp8_blockwise_grouped_mm_kernel(const __grid_constant__ CUtensorMap map_w, const
   constexpr int STAGES = S::STAGES;
   constexpr int NCH = S::NCH;
   extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint8_t* smem = ptx::align1024(smem_raw);
   float* chunks = reinterpret_cast<float*>(smem + (size_t)STAGES * S::STAGE_BYTES);        // [NCH][CH_KT][TOK]
   uint8_t* epi_stage = reinterpret_cast<uint8_t*>(chunks + NCH * S::CHUNK_FLOATS);        // 1 KB per epilogue warp
   SharedCtl* ctl = reinterpret_cast<SharedCtl*>(epi_stage + (size_t)S::EPI_WARPS * EPI_TILE_BYTES);

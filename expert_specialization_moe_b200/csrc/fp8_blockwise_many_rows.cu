@@ -129,7 +129,7 @@ fp8_blockwise_many_rows_kernel(const __grid_constant__ CUtensorMap map_w, const 
                                const int* __restrict__ problem_sizes, const int* __restrict__ expert_offsets,
                                int num_experts, int n, int k, int wide_stores, int scales_vec4) {
   extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint8_t* smem = ptx::align1024(smem_raw);
   SharedCtl* ctl = reinterpret_cast<SharedCtl*>(smem + (size_t)STAGES * STAGE_BYTES);
   const int kt_count = k / TILE_K;
   const int warp = threadIdx.x >> 5;

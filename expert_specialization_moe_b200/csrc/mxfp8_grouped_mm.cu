@@ -236,7 +236,7 @@ __device__ __forceinline__ void grouped_mm_cta(const CUtensorMap& map_w, const C
   constexpr int TOK_TILE = S::TOK_TILE, STAGES = S::STAGES, X_BYTES = S::X_BYTES, STAGE_BYTES = S::STAGE_BYTES;
   constexpr int LANES = S::LANES;
   extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint8_t* smem = ptx::align1024(smem_raw);
   uint8_t* epi_stage = smem + (size_t)STAGES * STAGE_BYTES;      // 2 KB per epilogue warp
   SharedCtl* ctl = reinterpret_cast<SharedCtl*>(epi_stage + S::EPILOGUE_TILES * EPI_STAGE_BYTES_PER_WARP);
   const int warp = threadIdx.x >> 5;

@@ -13,6 +13,13 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
 
+// The first 1024-byte boundary in the kernel's dynamic shared memory, as an offset from it: rounding the address as an
+// integer makes every access through the result a generic one (LD / ST instead of LDS / STS), staging stores and table
+// look-ups included.
+__device__ __forceinline__ uint8_t* align1024(uint8_t* smem_raw) {
+  return smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
+}
+
 __device__ __forceinline__ uint64_t globaltimer_ns() {
   uint64_t t;
   asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
