@@ -2,9 +2,9 @@
 //
 // In TMEM the accumulator's lane is the output COLUMN n and its column is the token ROW, so a thread that reads its
 // lane with tcgen05.ld holds one n for many tokens — the transpose of what coalesced stores of d[token, n] want.
-// Each epilogue warp therefore passes 32 tokens x 32 n at a time through a private 2 KB shared-memory tile: written
-// as [token][n] with 2-byte stores (32 lanes = 64 contiguous bytes, conflict free), read back as 16-byte pieces of a
-// token row, and stored to global memory as 128-bit stores, four lanes per 64-byte row segment.
+// Each epilogue warp therefore passes TOK (16 or 32) tokens x 32 n at a time through a private shared-memory tile:
+// written as [token][n] with 2-byte stores (32 lanes = 64 contiguous bytes, conflict free), read back as 16-byte pieces
+// of a token row, and stored to global memory as 128-bit stores, four lanes per 64-byte row segment.
 #pragma once
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
@@ -13,7 +13,6 @@
 
 namespace es_b200 {
 
-constexpr int EPI_STAGE_BYTES_PER_WARP = 32 * 32 * 2;
 
 // Optional destination map of the output rows (expert-parallel combine fused into the GEMM): output row r goes to row
 // meta[r].y of the [slots, n] array base[meta[r].x] — another GPU's buffer mapped into this process, or a local one —
@@ -55,6 +54,7 @@ __device__ __forceinline__ void store_chunk(const uint32_t (&v)[32], int c, int 
   const int part = lane & 3;
 #pragma unroll
   for (int p = 0; p < 32 / TOK; ++p) {
+    if (c + p * TOK >= valid) break;       // warp-uniform: no rows left
 #pragma unroll
     for (int j = 0; j < TOK; ++j) stage_warp[j * 32 + lane] = out_from_f32<OutT>(__uint_as_float(v[p * TOK + j]));
     __syncwarp();
@@ -83,19 +83,12 @@ __device__ __forceinline__ void store_chunk(const uint32_t (&v)[32], int c, int 
 // a scatter map, to the mapped row of output row `first_row + j` at column offset `col_off` (`dst` is then unused).
 // `release` is called once, after the last TMEM read (the accumulator may then be overwritten); `status` is the
 // kernel's error word.
-template <typename OutT, int PARTS, class Release>
+template <typename OutT, int PARTS, int TOK, class Release>
 __device__ __forceinline__ void drain_partial_sums(uint32_t taddr, uint32_t part_stride, int parts_written, int n_cols,
                                                    int valid, OutT* stage_warp, OutT* dst, int64_t ld, int lane,
                                                    Release release, const RowScatter& scatter, int64_t first_row,
-                                                   int col_off, uint32_t* status, bool direct_stores,
-                                                   int first_col = 0, int col_stride = 32) {
-  // (a warp that shares its lane quadrant with another takes the 32-column chunks first_col, first_col + col_stride,
-  // ...; one without a chunk in this tile only hands the accumulator back)
-  if (first_col >= n_cols) {
-    release();
-    return;
-  }
-  for (int c = first_col; c < n_cols; c += col_stride) {
+                                                   int col_off, uint32_t* status, bool direct_stores) {
+  for (int c = 0; c < n_cols; c += 32) {
     OutT* dest = nullptr;
     if (scatter.meta != nullptr)
       dest = scatter_row_ptr<OutT>(scatter, first_row + c + lane, c + lane < valid, ld, col_off, status);
@@ -122,7 +115,7 @@ __device__ __forceinline__ void drain_partial_sums(uint32_t taddr, uint32_t part
         for (int i = 0; i < 16; ++i) acc[h * 16 + i] = 0u;
       }
     }
-    if (c + col_stride >= n_cols) release();
+    if (c + 32 >= n_cols) release();
     if (direct_stores && scatter.meta == nullptr) {
       // dense output without shared memory: a warp-wide 2-byte store writes the 64 contiguous bytes of one token row.
       // The caller asks for it when K is long (the output is a small part of the call's bytes): no store -> sync ->
@@ -137,7 +130,7 @@ __device__ __forceinline__ void drain_partial_sums(uint32_t taddr, uint32_t part
         out += ld;
       }
     } else {
-      store_chunk<OutT, 32>(acc, c, valid, stage_warp, dst, ld, lane, scatter, dest);
+      store_chunk<OutT, TOK>(acc, c, valid, stage_warp, dst, ld, lane, scatter, dest);
     }
   }
 }

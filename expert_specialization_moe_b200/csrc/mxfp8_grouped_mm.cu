@@ -36,9 +36,8 @@
 //               double-buffered against the MMAs of the next tile
 //   warps 6, 14 scale copies, one lane each: the slot's weight / token scale atom smem -> the slot's TMEM columns
 //               (tcgen05.cp), tcgen05.commit to the slot's sf_ready barrier
-//   warps 7-10  second load path: the odd ring slots by cp.async — or, for the 112-token shape when K is short, a
-//               second epilogue group (every slot is then filled by TMA and the two groups take alternate 32-token
-//               chunks of a tile)
+//   warps 7-10  second load path: the odd ring slots by cp.async — or, when K is short, a second epilogue group (every
+//               slot is then filled by TMA and the two groups take alternate tiles)
 //
 // Work list: items (expert, 1..8 consecutive weight tiles of 128 — one tile when K is long, several when it is short, so
 // that an item spans ~16 K steps) found with a per-CTA prefix scan over the problem sizes (device resident: no host
@@ -65,18 +64,20 @@ constexpr int COPY_WARP0 = 6, COPY_WARP1 = 14;
 constexpr int LOADER_WARP0 = 7;        // warps 7..10: cp.async loaders
 constexpr int LOADER_THREADS = 128;
 constexpr int MMA_WARP1 = 11;          // MMA lanes 1..3 sit in warps 11..13 (lane 0 in warp 1)
+constexpr int PRODUCER2_WARP = 13;     // second producer when K is short (two MMA lanes)
 constexpr int MAX_LANES = 4;
 constexpr int TILE_N = 128;     // weight rows per tile  (tcgen05.mma M)
 constexpr int TILE_K = 128;     // bytes of K per ring slot (one 128-byte swizzle atom)
 constexpr int W_BYTES = TILE_N * TILE_K;
 constexpr int SF_BYTES = 512;
 constexpr int MAX_STAGES = 10;
+constexpr int SHORT_K_STEPS = 8;      // tiles of fewer K steps: two epilogue groups, staged stores
 constexpr uint32_t TMEM_COLS = 512;
 constexpr uint32_t SF_SLOT_COLS = 8;    // per ring slot: 4 columns of weight scales + 4 of token scales
 
 // A streaming shape: experts with at most TOK_TILE rows (ONE token tile per expert: the tile's token scales are then
 // exactly one 128-row atom), STAGES ring slots, LANES MMA-issuing threads = partial accumulators.
-template <int TOK_TILE_, int STAGES_, int LANES_, bool SECOND_LOAD_PATH_, bool SECOND_EPILOGUE_>
+template <int TOK_TILE_, int STAGES_, int LANES_, bool SECOND_LOAD_PATH_, int STORE_TOK_>
 struct Shape {
   static constexpr int TOK_TILE = TOK_TILE_;     // token rows per tile (tcgen05.mma N, runtime multiple of 16)
   static constexpr int STAGES = STAGES_;
@@ -85,12 +86,15 @@ struct Shape {
   // loader threads copy as many token bytes, L2 hits, as weight bytes: 48 vs 52 GB/s per SM) but inside a call, next to
   // the other kernels, the call is faster with it (reference-distribution workload at 32 experts: 0.1938 vs 0.1967 ms)
   static constexpr bool SECOND_LOAD_PATH = SECOND_LOAD_PATH_;
-  // With few K steps per tile the four epilogue warps set the pace of a tile of many tokens (partial sums and the store
-  // of four 32-token chunks take ~10000 cycles, the loads of three K steps ~1500).  The shape can then run the four
-  // loader warps as a second epilogue group instead (every ring slot by TMA; the two groups take alternate chunks).
-  // Needs four more 2 KB store tiles, which the 32-token shape has no room for and, with its single chunk, no use for.
-  static constexpr bool SECOND_EPILOGUE = SECOND_EPILOGUE_;
-  static constexpr int EPILOGUE_TILES = SECOND_EPILOGUE ? 8 : 4;
+  // With few K steps per tile four epilogue warps set the pace (k = 256: 2050 cycles for a tile of up to 32 tokens, 1430
+  // is what its bytes take at HBM speed; a 112-token tile ~10000, its loads ~1500).  The four loader warps are then a
+  // second epilogue group (every ring slot by TMA, from two producer warps): the groups take alternate tiles, one
+  // accumulator buffer each.  Reference benchmark's row distribution at n = 7168, k = 256: the 187 experts of <= 32 rows
+  // alone 98.8 -> 80.8 us, the whole call 187 -> 168.  The 32-token shape runs that way up to two K steps (with 3 to 5 its
+  // second load path is worth more: E = 264, n = 3968, k = 384 54.5 us against 59.9), the 112-token shape below eight.
+  static constexpr int STORE_TOK = STORE_TOK_;             // tokens per pass through a warp's store tile
+  static constexpr int STORE_TILE_BYTES = STORE_TOK * 32 * 2;
+  static constexpr int EPILOGUE_BYTES = 8 * STORE_TILE_BYTES;
   static constexpr int X_BYTES = TOK_TILE * TILE_K;
   static constexpr int STAGE_BYTES = W_BYTES + X_BYTES + 2 * SF_BYTES;   // W | X | weight scales | token scales
   static constexpr uint32_t ACC_COLS = LANES * TOK_TILE;                 // one accumulator buffer: LANES partials
@@ -99,8 +103,8 @@ struct Shape {
   static_assert(TOK_TILE % 16 == 0 && TOK_TILE <= 128 && (LANES == 1 || LANES == 2 || LANES == 4), "tile shape");
   static_assert(SF_COL0 + STAGES * SF_SLOT_COLS <= TMEM_COLS, "TMEM budget");
 };
-using ShapeTiny = Shape<32, 10, 4, true, false>;   // 21 KB slots; TMEM: 2 x 4 x 32 accumulator columns + 80 scale columns
-using ShapeMid = Shape<112, 6, 2, true, true>;   // 31 KB slots; TMEM: 2 x 2 x 112 accumulator columns + 48 scale columns
+using ShapeTiny = Shape<32, 10, 4, true, 16>;   // 21 KB slots; TMEM: 2 x 4 x 32 accumulator columns + 80 scale columns
+using ShapeMid = Shape<112, 6, 2, true, 32>;   // 31 KB slots; TMEM: 2 x 2 x 112 accumulator columns + 48 scale columns
 
 // CTAs of the 112-token shape in front of the 32-token shape's (tunable mm_stream_mid_lead_ctas < 0).  Measured in one
 // process, bursts of 20 calls, on the reference benchmark's row distribution: n = 512, E = 256: 0.1980 ms with 0,
@@ -116,7 +120,7 @@ struct SharedCtl {
   uint64_t empty[MAX_STAGES];           // 1 arrival: the commit of the MMA lane that owns the K step
   uint64_t sf_ready[MAX_STAGES];        // 2 arrivals: both scale atoms of the slot are in its TMEM columns
   uint64_t tmem_full[2];                // LANES arrivals: every MMA lane's share of the tile is complete
-  uint64_t tmem_empty[2];               // 4 (8 with the second group) arrivals: the epilogue warps have read the buffer
+  uint64_t tmem_empty[2];               // 4 arrivals: the warps of the epilogue group that owns the tile have read the buffer
   uint64_t q_full[QUEUE_DEPTH];         // 1 arrival: the producer lane has written q_tile[slot]
   uint64_t q_empty[QUEUE_DEPTH];        // every consuming role has read it
   int q_tile[QUEUE_DEPTH];              // tile index, or -1: no more work
@@ -128,7 +132,7 @@ struct SharedCtl {
 
 template <class S>
 constexpr size_t smem_bytes() {
-  return 1024 /*alignment slack*/ + (size_t)S::STAGES * S::STAGE_BYTES + S::EPILOGUE_TILES * EPI_STAGE_BYTES_PER_WARP +
+  return 1024 /*alignment slack*/ + (size_t)S::STAGES * S::STAGE_BYTES + S::EPILOGUE_BYTES +
          sizeof(SharedCtl);
 }
 
@@ -212,9 +216,9 @@ __device__ __forceinline__ void grouped_mm_cta(const CUtensorMap& map_w, const C
                                                const RowScatter& scatter, int min_rows, int max_rows, int bucket,
                                                int load_mode, int block, int blocks) {
   // load_mode 0: every ring slot by TMA; 1: odd slots by cp.async from warps 7..10; 2: every slot by TMA and warps 7..10
-  // are a second epilogue group (shapes with SECOND_EPILOGUE only)
+  // are a second epilogue group
   const bool use_lsu = load_mode == 1;
-  const bool epi2 = S::SECOND_EPILOGUE && load_mode == 2;
+  const bool epi2 = load_mode == 2;
   const uint8_t* __restrict__ a_codes = args.a_codes;
   const uint8_t* __restrict__ w_codes = args.w_codes;
   const uint8_t* __restrict__ sf_tokens = args.sf_tokens;
@@ -234,11 +238,12 @@ __device__ __forceinline__ void grouped_mm_cta(const CUtensorMap& map_w, const C
   uint32_t* counters = args.counters;
   const uint32_t earlier_ctas = args.earlier_ctas;
   constexpr int TOK_TILE = S::TOK_TILE, STAGES = S::STAGES, X_BYTES = S::X_BYTES, STAGE_BYTES = S::STAGE_BYTES;
-  constexpr int LANES = S::LANES;
+  // short K: two MMA lanes (a tile has no use for more); the warp of another then fills the odd ring slots
+  const int lanes = epi2 ? 2 : S::LANES;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = ptx::align1024(smem_raw);
-  uint8_t* epi_stage = smem + (size_t)STAGES * STAGE_BYTES;      // 2 KB per epilogue warp
-  SharedCtl* ctl = reinterpret_cast<SharedCtl*>(epi_stage + S::EPILOGUE_TILES * EPI_STAGE_BYTES_PER_WARP);
+  uint8_t* epi_stage = smem + (size_t)STAGES * STAGE_BYTES;      // one store tile per epilogue warp
+  SharedCtl* ctl = reinterpret_cast<SharedCtl*>(epi_stage + S::EPILOGUE_BYTES);
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
 
@@ -249,14 +254,14 @@ __device__ __forceinline__ void grouped_mm_cta(const CUtensorMap& map_w, const C
       ptx::mbar_init(&ctl->sf_ready[s], 2);
     }
     for (int a = 0; a < 2; ++a) {
-      ptx::mbar_init(&ctl->tmem_full[a], LANES);
-      ptx::mbar_init(&ctl->tmem_empty[a], epi2 ? 8 : 4);
+      ptx::mbar_init(&ctl->tmem_full[a], lanes);
+      ptx::mbar_init(&ctl->tmem_empty[a], 4);
     }
     for (int q = 0; q < QUEUE_DEPTH; ++q) {
       ptx::mbar_init(&ctl->q_full[q], 1);
-      // readers: LANES MMA lanes, 2 copy lanes, 4 epilogue warps, and warps 7..10 when they run (as loaders or as the
-      // second epilogue group)
-      ptx::mbar_init(&ctl->q_empty[q], LANES + 2 + 4 + ((use_lsu || epi2) ? LOADER_THREADS / 32 : 0));
+      // readers: the MMA lanes, 2 copy lanes, 4 epilogue warps, warps 7..10 when they run (as loaders or as the second
+      // epilogue group), and the second producer of a short-K launch
+      ptx::mbar_init(&ctl->q_empty[q], lanes + 2 + 4 + ((use_lsu || epi2) ? LOADER_THREADS / 32 : 0) + (epi2 ? 1 : 0));
     }
     ctl->abort_flag = 0;
     ptx::fence_mbar_init();
@@ -312,9 +317,10 @@ __device__ __forceinline__ void grouped_mm_cta(const CUtensorMap& map_w, const C
   volatile int* abort_flag = &ctl->abort_flag;
   const int mma_lane = warp == 1 ? 0 : (warp >= MMA_WARP1 && warp < MMA_WARP1 + MAX_LANES - 1) ? warp - MMA_WARP1 + 1 : -1;
 
-  // ------------------------------------------------------------------ epilogue: warps 2..5, and warps 7..10 as a second
-  // group when the shape runs that way; a group's warp takes the 32-token chunks first_col, first_col + col_stride, ...
-  auto run_epilogue = [&](OutT* stage_warp, int first_col, int col_stride) {
+  // ------------------------------------------------------------------ epilogue: warps 2..5 (group 0), and warps 7..10 as
+  // group 1 when the launch runs that way: buffer b, every second tile, then belongs to group b
+  auto run_epilogue = [&](int group_id, int warp_in_group) {
+    OutT* stage_warp = reinterpret_cast<OutT*>(epi_stage + (group_id * 4 + warp_in_group) * S::STORE_TILE_BYTES);
     const int quad = warp & 3;   // TMEM lane quadrant this warp may access
     QueueReader q;
     int acc = 0;
@@ -327,13 +333,14 @@ __device__ __forceinline__ void grouped_mm_cta(const CUtensorMap& map_w, const C
       const TileInfo ti = decode_tile(t, tab, num_experts, n_tiles, group);
       for (int sub = 0; ok && sub < ti.n_sub; ++sub) {
       const int nt = ti.nt + sub;
+      if (!epi2 || acc == group_id) {
       const bool got = ptx::mbar_wait(&ctl->tmem_full[acc], acc_ph, abort_flag);
       if (!__all_sync(0xffffffffu, got)) { ok = false; break; }
       ptx::tc_fence_after_sync();
       const uint32_t taddr = tmem_base + acc * S::ACC_COLS + ((uint32_t)(quad * 32) << 16);
       OutT* dst = d + (int64_t)ti.row0 * n + (nt * TILE_N + quad * 32);
-      drain_partial_sums<OutT, LANES>(
-          taddr, TOK_TILE, kt_count < LANES ? kt_count : LANES, ti.n_mma, ti.valid,
+      drain_partial_sums<OutT, S::LANES, S::STORE_TOK>(
+          taddr, TOK_TILE, kt_count < lanes ? kt_count : lanes, ti.n_mma, ti.valid,
           stage_warp, dst, n, lane,
           [&] {
             // all of this warp's accumulator reads are done: hand the buffer back to the MMA lanes
@@ -341,7 +348,8 @@ __device__ __forceinline__ void grouped_mm_cta(const CUtensorMap& map_w, const C
             __syncwarp();
             if (lane == 0) ptx::mbar_arrive(&ctl->tmem_empty[acc]);
           },
-          scatter, ti.row0, nt * TILE_N + quad * 32, &g_status, kt_count >= 8, first_col, col_stride);
+          scatter, ti.row0, nt * TILE_N + quad * 32, &g_status, kt_count >= SHORT_K_STEPS);
+      }   // this group's tile
       acc ^= 1;
       if (acc == 0) acc_ph ^= 1u;
       }   // weight tiles of the item
@@ -350,6 +358,45 @@ __device__ __forceinline__ void grouped_mm_cta(const CUtensorMap& map_w, const C
       *abort_flag = 1;
       atomicOr(&g_status, ERR_EPILOGUE);
     }
+  };
+
+  // ------------------------------------------------------------------ TMA loads of one work item by a whole warp.  The
+  // slots are all this warp's, or only those of its parity: odd slots belong to the cp.async loaders when they run, and
+  // with short K to a second producer warp — the ~650 cycles that a slot costs its producer are then half a tile's time.
+  const bool split_slots = use_lsu || epi2;
+  const int parity = warp == 0 ? 0 : 1;
+  auto load_item = [&](const TileInfo& ti, int& s, uint32_t& ph) {
+    const CUtensorMap* xm = ti.n_mma <= 16 ? &map_x16 : ti.n_mma <= 32 ? &map_x32 : ti.n_mma <= 64 ? &map_x64 : &map_xt;
+    const uint32_t box_rows = ti.n_mma <= 16 ? 16u : ti.n_mma <= 32 ? 32u : ti.n_mma <= 64 ? 64u : (uint32_t)TOK_TILE;
+    const uint32_t tx = W_BYTES + box_rows * TILE_K + 2 * SF_BYTES;
+    // this lane's load: 0 weight tile (streamed once: evict first), 1 token tile (re-read by every weight tile of
+    // the expert: evict last), 2 weight scale atom, 3 token scale atom (512-byte records, index = atom number)
+    const int sfw_atom = (ti.e * n_tiles + ti.nt) * kt_count;
+    const int sfx_atom = (tab.scale0(ti.e) >> 7) * kt_count;
+    const CUtensorMap* my_map = lane == 0 ? &map_w : lane == 1 ? xm : lane == 2 ? &map_sfw : &map_sfx;
+    const uint32_t my_off = lane == 0 ? 0u : lane == 1 ? (uint32_t)W_BYTES
+                            : lane == 2 ? (uint32_t)(W_BYTES + X_BYTES) : (uint32_t)(W_BYTES + X_BYTES + SF_BYTES);
+    const int my_c1_first = lane == 0 ? ti.e * n + ti.nt * TILE_N : lane == 1 ? ti.row0 : lane == 2 ? sfw_atom : sfx_atom;
+    const int my_c1_step = lane == 0 ? TILE_N : lane == 2 ? kt_count : 0;     // per weight tile of the item
+    const uint64_t my_hint = lane == 0 ? ptx::kL2EvictFirst : lane == 1 ? ptx::kL2EvictLast : ptx::kL2EvictNormal;
+    bool ok = true;
+    for (int sub = 0; ok && sub < ti.n_sub; ++sub) {
+    const int my_c1 = my_c1_first + sub * my_c1_step;
+    for (int kt = 0; kt < kt_count; ++kt) {
+      if (!split_slots || (s & 1) == parity) {
+        ok = __all_sync(0xffffffffu, ptx::mbar_wait(&ctl->empty[s], ph ^ 1u, abort_flag));
+        if (!ok) break;
+        uint8_t* stage = smem + (size_t)s * STAGE_BYTES;
+        if (lane == 0) ptx::mbar_arrive_expect_tx(&ctl->full[s], tx);
+        __syncwarp();
+        if (lane < 4)
+          ptx::tma_load_2d_hint(stage + my_off, my_map, &ctl->full[s], lane < 2 ? kt * TILE_K : 0,
+                                lane < 2 ? my_c1 : my_c1 + kt, my_hint);
+      }
+      if (++s == STAGES) { s = 0; ph ^= 1u; }
+    }
+    }   // weight tiles of the item
+    return ok;
   };
 
   if (warp == 0) {
@@ -385,36 +432,7 @@ __device__ __forceinline__ void grouped_mm_cta(const CUtensorMap& map_w, const C
       }
       if (t < 0) break;
       const TileInfo ti = decode_tile(t, tab, num_experts, n_tiles, group);
-      const CUtensorMap* xm = ti.n_mma <= 16 ? &map_x16 : ti.n_mma <= 32 ? &map_x32 : ti.n_mma <= 64 ? &map_x64 : &map_xt;
-      const uint32_t box_rows = ti.n_mma <= 16 ? 16u : ti.n_mma <= 32 ? 32u : ti.n_mma <= 64 ? 64u : (uint32_t)TOK_TILE;
-      const uint32_t tx = W_BYTES + box_rows * TILE_K + 2 * SF_BYTES;
-      // this lane's load: 0 weight tile (streamed once: evict first), 1 token tile (re-read by every weight tile of
-      // the expert: evict last), 2 weight scale atom, 3 token scale atom (512-byte records, index = atom number)
-      const int sfw_atom = (ti.e * n_tiles + ti.nt) * kt_count;
-      const int sfx_atom = (tab.scale0(ti.e) >> 7) * kt_count;
-      const CUtensorMap* my_map = lane == 0 ? &map_w : lane == 1 ? xm : lane == 2 ? &map_sfw : &map_sfx;
-      const uint32_t my_off = lane == 0 ? 0u : lane == 1 ? (uint32_t)W_BYTES
-                              : lane == 2 ? (uint32_t)(W_BYTES + X_BYTES) : (uint32_t)(W_BYTES + X_BYTES + SF_BYTES);
-      const int my_c1_first = lane == 0 ? ti.e * n + ti.nt * TILE_N : lane == 1 ? ti.row0 : lane == 2 ? sfw_atom : sfx_atom;
-      const int my_c1_step = lane == 0 ? TILE_N : lane == 2 ? kt_count : 0;     // per weight tile of the item
-      const uint64_t my_hint = lane == 0 ? ptx::kL2EvictFirst : lane == 1 ? ptx::kL2EvictLast : ptx::kL2EvictNormal;
-      bool ok = true;
-      for (int sub = 0; ok && sub < ti.n_sub; ++sub) {
-      const int my_c1 = my_c1_first + sub * my_c1_step;
-      for (int kt = 0; kt < kt_count; ++kt) {
-        if (!(use_lsu && (s & 1))) {          // odd slots belong to the cp.async loaders
-          ok = __all_sync(0xffffffffu, ptx::mbar_wait(&ctl->empty[s], ph ^ 1u, abort_flag));
-          if (!ok) break;
-          uint8_t* stage = smem + (size_t)s * STAGE_BYTES;
-          if (lane == 0) ptx::mbar_arrive_expect_tx(&ctl->full[s], tx);
-          __syncwarp();
-          if (lane < 4)
-            ptx::tma_load_2d_hint(stage + my_off, my_map, &ctl->full[s], lane < 2 ? kt * TILE_K : 0,
-                                  lane < 2 ? my_c1 : my_c1 + kt, my_hint);
-        }
-        if (++s == STAGES) { s = 0; ph ^= 1u; }
-      }
-      }   // weight tiles of the item
+      const bool ok = load_item(ti, s, ph);
       if (!ok) {
         if (lane == 0) {
           *abort_flag = 1;
@@ -424,9 +442,25 @@ __device__ __forceinline__ void grouped_mm_cta(const CUtensorMap& map_w, const C
       }
     }
   } else if (mma_lane >= 0) {
-    // ------------------------------------------------------------------ MMA issue: lane l of LANES takes the K steps
-    // with kt % LANES == l and accumulates them in partial accumulator l of the tile's buffer
-    if (lane == 0 && mma_lane < LANES) {
+    // ------------------------------------------------------------------ MMA issue: lane l of `lanes` takes the K steps
+    // with kt % lanes == l and accumulates them in partial accumulator l of the tile's buffer
+    if (epi2 && warp == PRODUCER2_WARP) {
+      // ---------------------------------------------------------------- second producer (short K): the odd ring slots
+      QueueReader q;
+      int s = 0;
+      uint32_t ph = 0;
+      bool ok = true;
+      while (ok) {
+        int t;
+        if (!q.next<true>(ctl, abort_flag, lane, &t)) { ok = false; break; }
+        if (t < 0) break;
+        ok = load_item(decode_tile(t, tab, num_experts, n_tiles, group), s, ph);
+      }
+      if (!ok && lane == 0) {
+        *abort_flag = 1;
+        atomicOr(&g_status, ERR_PRODUCER);
+      }
+    } else if (lane == 0 && mma_lane < lanes) {
       QueueReader q;
       int s = 0;
       uint32_t ph = 0;
@@ -443,7 +477,7 @@ __device__ __forceinline__ void grouped_mm_cta(const CUtensorMap& map_w, const C
         ptx::tc_fence_after_sync();
         const uint32_t d_tmem = tmem_base + acc * S::ACC_COLS + mma_lane * TOK_TILE;
         for (int kt = 0; kt < kt_count; ++kt) {
-          if ((kt & (LANES - 1)) == mma_lane) {
+          if ((kt & (lanes - 1)) == mma_lane) {
             if (!ptx::mbar_wait(&ctl->full[s], ph, abort_flag)) { ok = false; break; }
             if (!ptx::mbar_wait(&ctl->sf_ready[s], ph, abort_flag)) { ok = false; break; }
             if (use_lsu && (s & 1)) ptx::fence_proxy_async_shared();   // slot written by cp.async (generic proxy)
@@ -511,7 +545,7 @@ __device__ __forceinline__ void grouped_mm_cta(const CUtensorMap& map_w, const C
     // slot (MMA lanes, copy lanes) issue a proxy fence after their wait: the data was written through the generic
     // proxy and is read by tcgen05 through the async proxy.
     if (epi2) {
-      run_epilogue(reinterpret_cast<OutT*>(epi_stage) + (4 + warp - LOADER_WARP0) * 1024, 32, 64);
+      run_epilogue(1, warp - LOADER_WARP0);
     } else if (use_lsu) {
       const int lt = threadIdx.x - LOADER_WARP0 * 32;        // 0..127
       const int c16 = lt & 7, r0 = lt >> 3;                   // this thread's 16-byte column and first row
@@ -568,7 +602,7 @@ __device__ __forceinline__ void grouped_mm_cta(const CUtensorMap& map_w, const C
       }
     }
   } else if (warp >= 2 && warp <= 5) {
-    run_epilogue(reinterpret_cast<OutT*>(epi_stage) + (warp - 2) * 1024, 0, epi2 ? 64 : 32);
+    run_epilogue(0, warp - 2);
   }
   // (warps of MMA lanes the shape does not use fall through)
 
@@ -678,8 +712,8 @@ int launch_streaming(const CallArgs& c, int tiny_max, int mid_max, bool want_tin
                      first_of_call ? 1 : 0, group, c.counters, last_of_call ? 1 : 0, *earlier_ctas};
   ES_CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, map_w, map_x[0], map_x[1], map_x[2], map_x[3], map_sfx, map_sfw, args,
                                  *c.scatter, first_ctas, mid_lead, tiny_max, mid_max,
-                                 (ShapeTiny::SECOND_LOAD_PATH && lsu) ? 1 : 0,
-                                 (ShapeMid::SECOND_EPILOGUE && kt_count < 8) ? 2 : (ShapeMid::SECOND_LOAD_PATH && lsu) ? 1 : 0));
+                                 kt_count <= 2 ? 2 : (ShapeTiny::SECOND_LOAD_PATH && lsu) ? 1 : 0,
+                                 kt_count < SHORT_K_STEPS ? 2 : (ShapeMid::SECOND_LOAD_PATH && lsu) ? 1 : 0));
   *earlier_ctas += (uint32_t)grid;
   return ES_B200_OK;
 }
