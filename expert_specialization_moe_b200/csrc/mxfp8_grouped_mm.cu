@@ -37,7 +37,7 @@
 //   warps 6, 14 scale copies, one lane each: the slot's weight / token scale atom smem -> the slot's TMEM columns
 //               (tcgen05.cp), tcgen05.commit to the slot's sf_ready barrier
 //   warps 7-10  second load path: the odd ring slots by cp.async — or, when K is short, a second epilogue group (every
-//               slot is then filled by TMA and the two groups take alternate tiles)
+//               slot is then filled by TMA)
 //
 // Work list: items (expert, 1..8 consecutive weight tiles of 128 — one tile when K is long, several when it is short, so
 // that an item spans ~16 K steps) found with a per-CTA prefix scan over the problem sizes (device resident: no host
@@ -88,10 +88,12 @@ struct Shape {
   static constexpr bool SECOND_LOAD_PATH = SECOND_LOAD_PATH_;
   // With few K steps per tile four epilogue warps set the pace (k = 256: 2050 cycles for a tile of up to 32 tokens, 1430
   // is what its bytes take at HBM speed; a 112-token tile ~10000, its loads ~1500).  The four loader warps are then a
-  // second epilogue group (every ring slot by TMA, from two producer warps): the groups take alternate tiles, one
-  // accumulator buffer each.  Reference benchmark's row distribution at n = 7168, k = 256: the 187 experts of <= 32 rows
+  // second epilogue group (every ring slot by TMA, from two producer warps).  A tile of up to 32 tokens is one 32-token
+  // chunk: the groups take alternate tiles, one accumulator buffer each.  A larger tile they share, alternate chunks each
+  // (where a CTA has only a few tiles, alternate tiles would leave one group idle).  Reference benchmark's row distribution at n = 7168, k = 256: the 187 experts of <= 32 rows
   // alone 98.8 -> 80.8 us, the whole call 187 -> 168.  The 32-token shape runs that way up to two K steps (with 3 to 5 its
   // second load path is worth more: E = 264, n = 3968, k = 384 54.5 us against 59.9), the 112-token shape below eight.
+  static constexpr bool GROUPS_SHARE_TILES = TOK_TILE > 32;
   static constexpr int STORE_TOK = STORE_TOK_;             // tokens per pass through a warp's store tile
   static constexpr int STORE_TILE_BYTES = STORE_TOK * 32 * 2;
   static constexpr int EPILOGUE_BYTES = 8 * STORE_TILE_BYTES;
@@ -120,7 +122,7 @@ struct SharedCtl {
   uint64_t empty[MAX_STAGES];           // 1 arrival: the commit of the MMA lane that owns the K step
   uint64_t sf_ready[MAX_STAGES];        // 2 arrivals: both scale atoms of the slot are in its TMEM columns
   uint64_t tmem_full[2];                // LANES arrivals: every MMA lane's share of the tile is complete
-  uint64_t tmem_empty[2];               // 4 arrivals: the warps of the epilogue group that owns the tile have read the buffer
+  uint64_t tmem_empty[2];               // 4 arrivals (8 when two groups share the tile): the epilogue warps have read it
   uint64_t q_full[QUEUE_DEPTH];         // 1 arrival: the producer lane has written q_tile[slot]
   uint64_t q_empty[QUEUE_DEPTH];        // every consuming role has read it
   int q_tile[QUEUE_DEPTH];              // tile index, or -1: no more work
@@ -255,7 +257,7 @@ __device__ __forceinline__ void grouped_mm_cta(const CUtensorMap& map_w, const C
     }
     for (int a = 0; a < 2; ++a) {
       ptx::mbar_init(&ctl->tmem_full[a], lanes);
-      ptx::mbar_init(&ctl->tmem_empty[a], 4);
+      ptx::mbar_init(&ctl->tmem_empty[a], epi2 && S::GROUPS_SHARE_TILES ? 8 : 4);
     }
     for (int q = 0; q < QUEUE_DEPTH; ++q) {
       ptx::mbar_init(&ctl->q_full[q], 1);
@@ -318,7 +320,8 @@ __device__ __forceinline__ void grouped_mm_cta(const CUtensorMap& map_w, const C
   const int mma_lane = warp == 1 ? 0 : (warp >= MMA_WARP1 && warp < MMA_WARP1 + MAX_LANES - 1) ? warp - MMA_WARP1 + 1 : -1;
 
   // ------------------------------------------------------------------ epilogue: warps 2..5 (group 0), and warps 7..10 as
-  // group 1 when the launch runs that way: buffer b, every second tile, then belongs to group b
+  // group 1 when the launch runs that way: the groups then share the 32-token chunks of a tile, or buffer b, every second
+  // tile, belongs to group b
   auto run_epilogue = [&](int group_id, int warp_in_group) {
     OutT* stage_warp = reinterpret_cast<OutT*>(epi_stage + (group_id * 4 + warp_in_group) * S::STORE_TILE_BYTES);
     const int quad = warp & 3;   // TMEM lane quadrant this warp may access
@@ -333,7 +336,7 @@ __device__ __forceinline__ void grouped_mm_cta(const CUtensorMap& map_w, const C
       const TileInfo ti = decode_tile(t, tab, num_experts, n_tiles, group);
       for (int sub = 0; ok && sub < ti.n_sub; ++sub) {
       const int nt = ti.nt + sub;
-      if (!epi2 || acc == group_id) {
+      if (!epi2 || S::GROUPS_SHARE_TILES || acc == group_id) {
       const bool got = ptx::mbar_wait(&ctl->tmem_full[acc], acc_ph, abort_flag);
       if (!__all_sync(0xffffffffu, got)) { ok = false; break; }
       ptx::tc_fence_after_sync();
@@ -348,8 +351,9 @@ __device__ __forceinline__ void grouped_mm_cta(const CUtensorMap& map_w, const C
             __syncwarp();
             if (lane == 0) ptx::mbar_arrive(&ctl->tmem_empty[acc]);
           },
-          scatter, ti.row0, nt * TILE_N + quad * 32, &g_status, kt_count >= SHORT_K_STEPS);
-      }   // this group's tile
+          scatter, ti.row0, nt * TILE_N + quad * 32, &g_status, kt_count >= SHORT_K_STEPS,
+          S::GROUPS_SHARE_TILES ? group_id * 32 : 0, epi2 && S::GROUPS_SHARE_TILES ? 64 : 32);
+      }   // a tile of this group
       acc ^= 1;
       if (acc == 0) acc_ph ^= 1u;
       }   // weight tiles of the item
@@ -684,6 +688,12 @@ int launch_streaming(const CallArgs& c, int tiny_max, int mid_max, bool want_tin
   if (item_k_steps < 1) item_k_steps = 1;
   int group = (item_k_steps + kt_count - 1) / kt_count;
   if (group > 8) group = 8;
+  // ... but as many items as half the SMs while there are the tiles for it: a call of few tiles is a matter of latency, and
+  // up to half the SMs the CTAs of both shapes are on an SM at once.  8 experts, 729 rows, n = 640, k = 384: 23.8 -> 15.7 us;
+  // 24, 3000, 896, 384: 32.0 -> 25.7 (one item per SM 29.1, per three SMs 25.4); 20, 600, 1024, 256: 22.5 -> 17.3 (22.0,
+  // 17.7); 16, 100, 4096, 256: 14.5 -> 13.6 (15.0, 14.6)
+  const int64_t tiles = (c.num_experts < c.num_rows ? c.num_experts : c.num_rows) * (c.n / TILE_N);
+  while (group > 1 && tiles / group < info.sm_count / 2) --group;
   // upper bound of the item count known on the host: one token tile per expert
   const int64_t max_tiles = (int64_t)c.num_experts * ((c.n / TILE_N + group - 1) / group);
   int per_shape = (int)(max_tiles < info.sm_count ? max_tiles : info.sm_count);
