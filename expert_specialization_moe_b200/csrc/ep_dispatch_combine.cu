@@ -147,31 +147,56 @@ dispatch_quant_push_kernel(const T* __restrict__ x, const int* __restrict__ dst_
   // that follows on the stream orders them before its flag
 }
 
-// One warp per received row: the side record's scale bytes go to their swizzled position, its return address to the
-// (GPU, slot) table.  Offsets are range-checked: a bad one is skipped and reported.
+// The received rows' scale bytes go to their swizzled position, their return addresses to the (GPU, slot) table.  Offsets
+// are range-checked: a bad one is skipped and reported.  One thread per (row, K tile), four of them in flight: the
+// records are 16 + k / 32 bytes, and a warp per row (one dependent pass of 16 useful lanes at k = 2048) took 16.8 us for
+// 131072 rows, the bytes are worth 3; this way 12.2.
+constexpr int UNPACK_UNROLL = 4;
 __global__ void __launch_bounds__(THREADS)
 unpack_side_kernel(const uint8_t* __restrict__ side, const int* __restrict__ num_rows_dev, uint8_t* __restrict__ scales,
                    int2* __restrict__ meta, int k, long long capacity_rows, long long scale_bytes) {
   pdl_wait_prior_grid();
   pdl_launch_dependents();
-  const int lane = threadIdx.x & 31;
-  const int warps_per_grid = gridDim.x * (THREADS / 32);
   const int side_bytes = side_record_bytes(k);
-  const int kt = k >> 7;
+  const unsigned kt = (unsigned)(k >> 7);
   long long rows = *num_rows_dev;
   if (rows > capacity_rows) rows = capacity_rows;
-  for (long long r = blockIdx.x * (THREADS / 32) + (threadIdx.x >> 5); r < rows; r += warps_per_grid) {
-    const uint8_t* rec = side + r * side_bytes;
-    const uint4 head = *reinterpret_cast<const uint4*>(rec);
-    const long long sf_off = (long long)head.z | ((long long)head.w << 32);
-    if (lane == 0) meta[r] = make_int2((int)head.x, (int)head.y);
-    const bool ok = sf_off >= 0 && (sf_off & 3) == 0 && sf_off + (long long)(kt - 1) * 512 + 4 <= scale_bytes;
-    if (!ok) {
-      if (lane == 0) atomicOr(&g_status, ERR_BAD_DESTINATION);
-      continue;
+  const long long words = rows * kt;                     // kt <= 128: below 2^38
+  const long long threads = (long long)gridDim.x * THREADS;
+  // 32-bit row arithmetic inside a stretch of the grid: (row, tile) of the thread's first word, then steps of the grid
+  const long long first = (long long)blockIdx.x * THREADS + threadIdx.x;
+  long long r = first / kt;
+  unsigned q = (unsigned)(first - r * kt);
+  const long long step_rows = threads / kt;
+  const unsigned step_q = (unsigned)(threads - step_rows * kt);
+  for (long long i0 = first; i0 < words; i0 += UNPACK_UNROLL * threads) {
+    uint4 head[UNPACK_UNROLL];
+    uint32_t word[UNPACK_UNROLL];
+    long long row[UNPACK_UNROLL];
+    unsigned tile[UNPACK_UNROLL];
+#pragma unroll
+    for (int u = 0; u < UNPACK_UNROLL; ++u) {
+      row[u] = r;
+      tile[u] = q;
+      if (i0 + u * threads < words) {
+        const uint8_t* rec = side + r * side_bytes;
+        head[u] = __ldg(reinterpret_cast<const uint4*>(rec));
+        word[u] = __ldg(reinterpret_cast<const uint32_t*>(rec + 16) + q);
+      }
+      r += step_rows;
+      q += step_q;
+      if (q >= kt) { q -= kt; ++r; }
     }
-    for (int q = lane; q < kt; q += 32)
-      *reinterpret_cast<uint32_t*>(scales + sf_off + (long long)q * 512) = *reinterpret_cast<const uint32_t*>(rec + 16 + q * 4);
+#pragma unroll
+    for (int u = 0; u < UNPACK_UNROLL; ++u) {
+      if (i0 + u * threads >= words) break;
+      if (tile[u] == 0) meta[row[u]] = make_int2((int)head[u].x, (int)head[u].y);
+      const long long sf_off = (long long)head[u].z | ((long long)head[u].w << 32);
+      if (sf_off >= 0 && (sf_off & 3) == 0 && sf_off + (long long)(kt - 1) * 512 + 4 <= scale_bytes)
+        *reinterpret_cast<uint32_t*>(scales + sf_off + (long long)tile[u] * 512) = word[u];
+      else if (tile[u] == 0)
+        atomicOr(&g_status, ERR_BAD_DESTINATION);
+    }
   }
 }
 
@@ -225,7 +250,11 @@ struct Pack2<__half> {
   }
 };
 
-// One warp per token; a lane accumulates 8 columns at a time in fp32 over the token's top-k rows, in order j = 0..topk-1.
+// A warp per (token, 256 columns); a lane accumulates 8 columns in fp32 over the token's top-k rows, in order
+// j = 0 .. topk-1.  Bound by HBM (topk + 1 rows per token): the rows are requested SUM_ROWS at a time before the first is
+// used, and the work is cut by columns too, so that the last round of warps is short.  A warp per token with one row in
+// flight took 130 us for 16384 tokens x top-8 at n = 2048 (0.60 GB), this way 96.
+constexpr int SUM_ROWS = 8;
 template <typename T>
 __global__ void __launch_bounds__(THREADS)
 topk_weighted_sum_kernel(const uint4* __restrict__ pairs, const float* __restrict__ weights, uint4* __restrict__ out,
@@ -233,15 +262,26 @@ topk_weighted_sum_kernel(const uint4* __restrict__ pairs, const float* __restric
   pdl_wait_prior_grid();
   pdl_launch_dependents();
   const int lane = threadIdx.x & 31;
-  const int warps_per_grid = gridDim.x * (THREADS / 32);
-  for (int t = blockIdx.x * (THREADS / 32) + (threadIdx.x >> 5); t < tokens; t += warps_per_grid) {
-    const float w_lane = lane < topk ? weights[(int64_t)t * topk + lane] : 0.f;
-    for (int c = lane; c < row_vec16; c += 32) {
-      float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-      for (int j = 0; j < topk; ++j) {
-        const float w = __shfl_sync(0xffffffffu, w_lane, j);
-        const uint4 v = pairs[((int64_t)t * topk + j) * row_vec16 + c];
-        const uint32_t vw[4] = {v.x, v.y, v.z, v.w};
+  const int col_chunks = (row_vec16 + 31) / 32;
+  const long long units = (long long)tokens * col_chunks;
+  const long long warps_per_grid = (long long)gridDim.x * (THREADS / 32);
+  for (long long u = (long long)blockIdx.x * (THREADS / 32) + (threadIdx.x >> 5); u < units; u += warps_per_grid) {
+    const int t = (int)(u / col_chunks);
+    const int c = (int)(u - (long long)t * col_chunks) * 32 + lane;
+    const bool on = c < row_vec16;
+    const float w_lane = lane < topk ? __ldg(weights + (int64_t)t * topk + lane) : 0.f;
+    const uint4* src = pairs + (int64_t)t * topk * row_vec16 + c;
+    float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    for (int j0 = 0; j0 < topk; j0 += SUM_ROWS) {
+      uint4 v[SUM_ROWS];
+#pragma unroll
+      for (int j = 0; j < SUM_ROWS; ++j)
+        if (on && j0 + j < topk) v[j] = ld_stream_16B(src + (int64_t)(j0 + j) * row_vec16);
+#pragma unroll
+      for (int j = 0; j < SUM_ROWS; ++j) {
+        if (j0 + j >= topk) break;
+        const float w = __shfl_sync(0xffffffffu, w_lane, j0 + j);
+        const uint32_t vw[4] = {v[j].x, v[j].y, v[j].z, v[j].w};
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
           const float2 f = Pack2<T>::unpack(vw[i]);
@@ -249,9 +289,10 @@ topk_weighted_sum_kernel(const uint4* __restrict__ pairs, const float* __restric
           acc[2 * i + 1] = fmaf(w, f.y, acc[2 * i + 1]);
         }
       }
+    }
+    if (on)
       out[(int64_t)t * row_vec16 + c] = make_uint4(Pack2<T>::pack(acc[0], acc[1]), Pack2<T>::pack(acc[2], acc[3]),
                                                    Pack2<T>::pack(acc[4], acc[5]), Pack2<T>::pack(acc[6], acc[7]));
-    }
   }
 }
 
@@ -374,7 +415,8 @@ extern "C" int es_b200_ep_unpack_side(const void* side, const int32_t* num_rows_
                  (reinterpret_cast<uintptr_t>(meta) & 7u) == 0,
              "side must be 16-byte, meta 8-byte and scales 4-byte aligned");
   int grid = 1;
-  int rc = ep::grid_for(capacity_rows, &grid);
+  // warps for the words of every row that fits; each thread takes several
+  int rc = ep::grid_for((capacity_rows * (k / 128) + 31) / 32, &grid);
   if (rc != ES_B200_OK) return rc;
   ep::unpack_side_kernel<<<grid, ep::THREADS, 0, static_cast<cudaStream_t>(stream)>>>(
       static_cast<const uint8_t*>(side), num_rows_dev, scales, reinterpret_cast<int2*>(meta), k, capacity_rows,
@@ -417,7 +459,7 @@ extern "C" int es_b200_ep_topk_weighted_sum(const void* pairs, int dtype, const 
   ES_REQUIRE(pairs && weights && out, "null pointer argument");
   ES_REQUIRE(aligned16(pairs) && aligned16(out), "pairs and out must be 16-byte aligned");
   int grid = 1;
-  int rc = ep::grid_for(tokens, &grid);
+  int rc = ep::grid_for((int64_t)tokens * ((n / 8 + 31) / 32), &grid);
   if (rc != ES_B200_OK) return rc;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   if (dtype == ES_B200_BF16)

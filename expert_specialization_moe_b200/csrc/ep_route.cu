@@ -114,7 +114,8 @@ tables_kernel(const void* __restrict__ ids, int ids_int64, int pairs, int num_ex
   pdl_launch_dependents();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int e_local = num_experts / world;
-  // per-expert totals; each owner's experts are then scanned serially by one thread (E / world entries: short)
+  // per-expert totals; each owner's experts are then scanned by a warp (one thread stepping through them took as long as
+  // the table look-ups of the block's pairs)
   for (int e = threadIdx.x; e < num_experts; e += THREADS) {
     int m = 0, before = 0;
     for (int s = 0; s < world; ++s) {
@@ -126,29 +127,38 @@ tables_kernel(const void* __restrict__ ids, int ids_int64, int pairs, int num_ex
     before_s[e] = before;
   }
   __syncthreads();
-  if (threadIdx.x < world) {
-    const int d = threadIdx.x;
-    int rows = 0, srows = 0;
-    for (int le = 0; le < e_local; ++le) {
-      const int e = d * e_local + le;
-      const int m = eo_s[e];
-      eo_s[e] = rows;
-      bo_s[e] = srows;
-      if (d == my_rank && blockIdx.x == 0) {
-        // Rows past the capacity of the receive buffers are dropped (the senders' stores to them are skipped by the
-        // dispatch kernel's own range check): the expert that straddles the end is cut, later ones get no rows.
-        long long room = capacity_rows - rows;
-        if (room < 0) room = 0;
-        const int kept = m < room ? m : (int)room;
-        if (kept != m) atomicOr(&g_status, ERR_CAPACITY);
-        rows_out[le] = kept;
-        eo_out[le] = rows;
-        bo_out[le] = srows;
+  for (int d = warp; d < world; d += WARPS) {
+    const bool mine = d == my_rank && blockIdx.x == 0;
+    int rows0 = 0, srows0 = 0;                              // before this step's 32 experts
+    for (int l0 = 0; l0 < e_local; l0 += 32) {
+      const int le = l0 + lane, e = d * e_local + le;
+      const int m = le < e_local ? eo_s[e] : 0;
+      int rows = m, srows = (m + 127) & ~127;               // inclusive scans
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int a = __shfl_up_sync(0xffffffffu, rows, o), b = __shfl_up_sync(0xffffffffu, srows, o);
+        if (lane >= o) { rows += a; srows += b; }
       }
-      rows += m;
-      srows += (m + 127) & ~127;
+      const int first = rows0 + rows - m, sfirst = srows0 + srows - ((m + 127) & ~127);
+      if (le < e_local) {
+        eo_s[e] = first;
+        bo_s[e] = sfirst;
+        if (mine) {
+          // Rows past the capacity of the receive buffers are dropped (the senders' stores to them are skipped by the
+          // dispatch kernel's own range check): the expert that straddles the end is cut, later ones get no rows.
+          long long room = capacity_rows - first;
+          if (room < 0) room = 0;
+          const int kept = m < room ? m : (int)room;
+          if (kept != m) atomicOr(&g_status, ERR_CAPACITY);
+          rows_out[le] = kept;
+          eo_out[le] = first;
+          bo_out[le] = sfirst;
+        }
+      }
+      rows0 += __shfl_sync(0xffffffffu, rows, 31);
+      srows0 += __shfl_sync(0xffffffffu, srows, 31);
     }
-    if (d == my_rank && blockIdx.x == 0) *total_rows_out = rows < capacity_rows ? rows : (int)capacity_rows;
+    if (mine && lane == 0) *total_rows_out = rows0 < capacity_rows ? rows0 : (int)capacity_rows;
   }
   const int seg = blockIdx.x * WARPS + warp;
   int* my_run = run + warp * num_experts;
@@ -160,10 +170,12 @@ tables_kernel(const void* __restrict__ ids, int ids_int64, int pairs, int num_ex
   const int len = segment_len(pairs);
   const int begin = seg * len;
   const int end = min(begin + len, pairs);
+  int next = begin + lane < end ? load_id(ids, ids_int64, begin + lane) : -1;      // one step ahead of its use
   for (int i0 = begin; i0 < end; i0 += 32) {
     const int i = i0 + lane;
-    int e = i < end ? load_id(ids, ids_int64, i) : -1;
-    if (e >= num_experts) e = -1;
+    int e = next;
+    next = i + 32 < end ? load_id(ids, ids_int64, i + 32) : -1;
+    if (e < 0 || e >= num_experts) e = -1;
     const unsigned peers = __match_any_sync(0xffffffffu, e);
     const int rank_in_step = __popc(peers & ((1u << lane) - 1u));
     int pos = 0;
