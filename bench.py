@@ -601,7 +601,7 @@ def bench_blockwise(args, E, T, N, K, desc, device, rank, world, dist):
                            "l2": "inputs larger than L2 (weights %.2f GB per GPU), no flush" % (el * N * K / 1e9)},
                 "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                              "traffic": read_traffic(f"{args.workload}_n{world}"), "peak_kind": peak_kind,
-                             "algorithmic_bytes": abytes_local, "kernel": "fp8_blockwise_grouped_mm_kernel (<= 32 rows) + fp8_blockwise_two_shapes_kernel",
+                             "algorithmic_bytes": abytes_local, "kernel": "fp8_blockwise_grouped_mm_kernel (<= 32 rows) + fp8_blockwise_many_rows_kernel",
                              "kernel_ms": ms},
                 "clocks": clocks, "gpu_launches": int(args.steps * buckets)}
         print(json.dumps(line))
