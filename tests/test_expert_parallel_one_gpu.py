@@ -277,3 +277,64 @@ def test_dropped_pairs_add_zero_to_the_weighted_sum():
     assert int(dropped.sum()) == pairs - capacity
     assert bool((slots[dropped] == 0).all()), "slots of dropped pairs were not cleared"
     assert bool((slots[~dropped] == 7.0).all()), "slots of delivered pairs must be left to the combine"
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("tokens,topk,n", [(1, 1, 8), (3, 3, 264), (37, 8, 2048), (5, 11, 776), (2, 32, 256)])
+def test_topk_weighted_sum_edges(tokens, topk, n, dtype):
+    """Column chunks with a ragged last one, top-k below, at and above the rows requested at a time: fp32 accumulation in
+    order j = 0 .. topk-1, so within one rounding of the output type of the same sum in fp64."""
+    from expert_specialization_moe_b200 import _cabi
+    lib, dev = _cabi.load(), torch.device("cuda", 0)
+    g = torch.Generator(device=dev).manual_seed(tokens * 100 + topk)
+    pairs = torch.randn((tokens * topk, n), generator=g, device=dev).to(dtype)
+    w = torch.rand((tokens, topk), generator=g, device=dev)
+    out = torch.full((tokens, n), 7.0, dtype=dtype, device=dev)
+    code = _cabi.BF16 if dtype == torch.bfloat16 else _cabi.FP16
+    _cabi.check(lib.es_b200_ep_topk_weighted_sum(pairs.data_ptr(), code, w.data_ptr(), out.data_ptr(), tokens, topk, n,
+                                                 torch.cuda.current_stream(dev).cuda_stream))
+    want = (pairs.view(tokens, topk, n).double() * w.double().unsqueeze(-1)).sum(1)
+    # half an ulp of the output (2^-8, 2^-11 relative at most), topk fp32 roundings of partial sums of at most
+    # sum |w x|, and half the fp16 subnormal spacing
+    mag = (pairs.view(tokens, topk, n).double().abs() * w.double().unsqueeze(-1)).sum(1)
+    ulp = 2.0 ** (-8 if dtype == torch.bfloat16 else -11)
+    assert ((out.double() - want).abs() <= want.abs() * ulp * 1.01 + mag * topk * 2.0 ** -23 + 2.0 ** -24).all()
+
+
+@pytest.mark.parametrize("rows,capacity,k", [(1, 4, 128), (1000, 1500, 384), (3000, 3000, 2048), (70, 80, 7168)])
+def test_unpack_side_edges(rows, capacity, k):
+    """K tiles per row that do and do not divide the grid; scale words to their offsets, return addresses to the table,
+    rows past the count untouched, a row with an offset out of range reported and skipped."""
+    from expert_specialization_moe_b200 import _cabi
+    lib, dev = _cabi.load(), torch.device("cuda", 0)
+    _status(lib, dev)
+    kt, rec = k // 128, int(lib.es_b200_ep_side_record_bytes(k))
+    g = torch.Generator().manual_seed(rows + k)
+    side = torch.randint(0, 256, (capacity, rec), generator=g, dtype=torch.uint8)
+    head = torch.zeros((capacity, 4), dtype=torch.int32)
+    head[:, 0] = torch.randint(0, 8, (capacity,), generator=g)
+    head[:, 1] = torch.randperm(capacity, generator=g)
+    r = torch.randperm(capacity, generator=g)
+    off = (r // 128) * kt * 512 + (r % 32) * 16 + ((r % 128) // 32) * 4
+    head[:, 2] = off.to(torch.int32)
+    side[:, :16] = head.view(torch.uint8).view(capacity, 16)
+    scale_bytes = (capacity + 127) // 128 * 128 * kt * 4
+    want = torch.full((scale_bytes,), 0xEE, dtype=torch.uint8)
+    at = (off[:rows].view(-1, 1, 1) + torch.arange(kt).view(1, -1, 1) * 512 + torch.arange(4).view(1, 1, -1)).reshape(-1)
+    want[at] = side[:rows, 16:16 + 4 * kt].reshape(-1)
+    scales = torch.full((scale_bytes,), 0xEE, dtype=torch.uint8, device=dev)
+    meta = torch.full((capacity, 2), -5, dtype=torch.int32, device=dev)
+    side_d, n = side.to(dev), torch.tensor([rows], dtype=torch.int32, device=dev)
+    s = torch.cuda.current_stream(dev).cuda_stream
+    _cabi.check(lib.es_b200_ep_unpack_side(side_d.data_ptr(), n.data_ptr(), scales.data_ptr(), meta.data_ptr(), k, capacity,
+                                           scale_bytes, s))
+    assert torch.equal(scales.cpu(), want)
+    assert torch.equal(meta.cpu()[:rows], head[:rows, :2]) and (meta.cpu()[rows:] == -5).all()
+    assert _status(lib, dev)[0] == 0
+    side[0, 8:16] = torch.tensor([scale_bytes], dtype=torch.int64).view(torch.uint8)
+    side_d = side.to(dev)
+    _cabi.check(lib.es_b200_ep_unpack_side(side_d.data_ptr(), n.data_ptr(), scales.data_ptr(), meta.data_ptr(), k, capacity,
+                                           scale_bytes, s))
+    rc, raw = _status(lib, dev)
+    assert rc != 0 and raw & ERR_BAD_DESTINATION
+    assert torch.equal(scales.cpu(), want)

@@ -160,3 +160,20 @@ def test_scatter_epilogue_equals_dense_output(counts, N, K, out_dtype):
     untouched = torch.ones(slots, dtype=torch.bool)
     untouched[rows] = False
     assert bool((out[untouched] == 7.0).all())
+
+
+@pytest.mark.parametrize("lo,hi,E,N,K", [
+    (1, 32, 96, 1152, 256),       # two K steps: two epilogue groups on alternate tiles, two producer warps; items of 8 + 1 tiles
+    (1, 16, 40, 640, 128),        # one K step: only one MMA lane has work; slots of both producers within a tile alternate
+    (15, 18, 200, 256, 256),      # around the 16-token store pass; two tiles per expert
+    (20, 112, 60, 1152, 384),     # odd number of K steps, both shapes
+    (33, 112, 12, 1408, 896),     # seven K steps: groups share the chunks of a tile; fewer items than half the SMs
+    (1, 112, 6, 2304, 512),       # few experts: items shortened for the sake of more of them
+])
+def test_mm_short_k_many_tiles(lo, hi, E, N, K):
+    """Tiles of few K steps, many per CTA: hand-over between the epilogue groups, the producers and the tile queue."""
+    import random
+    rnd = random.Random(E + K)
+    inp = C.mxfp8_gemm_inputs([rnd.randint(lo, hi) for _ in range(E)], N, K, seed=K)
+    d = C.run_mxfp8_mm_op(inp)
+    _check_against_oracle(inp, d, torch.bfloat16)
