@@ -45,28 +45,36 @@ constexpr int QUANT_MIN_BLOCKS = 4, QUANT_MIN_BLOCKS_SILU = 3;
 // exact arithmetic of an unfused silu(gate.float()) * up.float() -> T: accurate expf, IEEE division and multiply
 __device__ __forceinline__ float silu_mul_exact(float g, float u) { return (g / (1.0f + expf(-g))) * u; }
 
-// act = round_to_T( silu(gate) * up ) on 16 elements, bit for bit what silu_mul_exact gives, for a third of its
-// instructions: p = g * rcp(1 + 2^(-g log2 e)) * u with the hardware approximations is within `eps` (relative) of the
-// exact sequence's fp32 value, so wherever p (1 - eps) and p (1 + eps) round to the same 16-bit value, that value is the
-// answer (rounding is monotonic); the few pairs where they do not (bf16: 0.04 % of the elements) take the exact sequence.
-// Error of p against the exact sequence, in units of 2^-24: 2^x 4 (2 ulp), its argument |g| (one rounding of g log2 e
-// and of the constant), reciprocal 2 (1 ulp), sum and two products 3 x 1; exact sequence: expf 2 (1 ulp), sum, quotient
-// and product 3 x 1; rounding of the two bounds 2.  16 + |g| in all; eps = (24 + 1.5 |g|) 2^-24 with the lane's largest g.
-// Lanes with an element outside the range in which these relative bounds hold go the exact way altogether: |g| > 64
-// (1 + 2^x can leave the range of the approximate reciprocal), and in bf16 |g| or |u| < 2^-36 (zeros among them: with
-// g = -64 the product is then 2^-122, next to the fp32 subnormals).  fp16 values are zero, which is exact, or at least
-// 2^-24.
+// act = round_to_T( silu(gate) * up ) on 16 elements; the codes and scale of their block are bit for bit those of
+// silu_mul_exact's values, for a third of its instructions.  p = g * rcp(1 + 2^(-g log2 e)) * u with the hardware
+// approximations is within `eps` (relative) of the exact sequence's fp32 value, so wherever p (1 - eps) and p (1 + eps)
+// round to the same 16-bit value, that value is the answer (rounding is monotonic); the few pairs where they do not (of
+// N(0, 1) values 0.05 % of the elements in bf16, 0.4 % in fp16) take the exact sequence.
+// Error of p against the exact sequence, in units of 2^-24: 2^x 4 (2 ulp), its argument 1.22 |g| (the product g log2 e and
+// the constant; at most 0.45 for g > 0, where 2^x is at most e^-g of the sum), reciprocal 2 (1 ulp), sum and two products
+// 3 x 1; exact sequence: expf 2 (1 ulp), sum, quotient and product 3 x 1; the factors 1 +- eps and their products 2.
+// 16 + 1.22 |g| in all; eps = (20 + 1.25 |g|) 2^-24 with the lane's lowest g.  (|g| < 2^-124 makes g / 2 subnormal: at
+// most 5 more, and only where it is large enough for an error to round away from it.)
+// The bound does not hold for g < -64 (1 + 2^x may leave the range of the reciprocal, p is then accurate or a zero of the
+// right sign) and for |p| near the fp32 subnormals.  Both are values that the block's scale turns into a signed zero,
+// whatever their digits, unless all the lane's values are that small: |p| <= 2^-86 |u| for the former, so a largest value
+// above 2^20 times these limits settles it (scaled to 448, they are below 2^-11, half of the smallest code is 2^-10).  Lanes
+// that it does not settle — none in practice but those whose values are all zero — take the exact sequence for every
+// element that is not a zero by its factors.  (Whole lanes by the exact sequence because of one zero or one large gate cost
+// a warp's step eight serial turns: 131072 x 768 bf16 with 1 % of zeros 312 us, 96 this way; 50-fold outliers 226, 99.)
+// fp16 products are zero or at least 2^-110.
+// `largest`: magnitudes of the lane's largest values, as max_magnitude16 gives them.
 template <typename T>
-__device__ __forceinline__ void silu_mul16(const uint32_t (&g)[8], const uint32_t (&u)[8], uint32_t (&out)[8]) {
+__device__ __forceinline__ void silu_mul16(const uint32_t (&g)[8], const uint32_t (&u)[8], uint32_t (&out)[8],
+                                           uint32_t& largest) {
   using V2 = typename Vec2<T>::type;
-  const float g_max = max_abs16<T>(g);
-  bool irregular = !(g_max <= 64.0f);
-  if constexpr (std::is_same<T, __nv_bfloat16>::value) {
-    const uint32_t least = min_magnitude2(min_magnitude16(g), min_magnitude16(u)) & 0x7fff7fffu;
-    irregular |= (least & 0xffffu) < 0x2d80u || least < 0x2d800000u;      // 2^-36
-  }
-  const float eps = fmaf(g_max, 8.940696716e-8f, 1.430511475e-6f);      // (24 + 1.5 |g|) 2^-24
-  uint32_t undecided = irregular ? 0xffu : 0u;      // one bit per pair
+  const uint32_t low2 = max_u16x2(max_u16x2(max_u16x2(g[0], g[1]), max_u16x2(g[2], g[3])),
+                                  max_u16x2(max_u16x2(g[4], g[5]), max_u16x2(g[6], g[7])));
+  const float low = Vec2<T>::from_bits(max(low2 >> 16, low2 & 0xffffu));   // negative values sort highest, most negative last
+  const bool in_range = low >= -64.0f;                                     // no: a lower one or a NaN among them
+  const float eps = fmaf(in_range ? fmaxf(-low, 0.0f) : 64.0f, 7.450580597e-8f, 1.192092896e-6f);   // (20 + 1.25 |g|) 2^-24
+  const float2 up = make_float2(1.0f + eps, 1.0f + eps), down = make_float2(1.0f - eps, 1.0f - eps);
+  uint32_t undecided = 0u;      // one bit per pair
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
     const float2 gf = Vec2<T>::to_float2(*reinterpret_cast<const V2*>(&g[i]));
@@ -74,14 +82,25 @@ __device__ __forceinline__ void silu_mul16(const uint32_t (&g)[8], const uint32_
     const float2 t = mul2(gf, make_float2(-1.4426950408889634f, -1.4426950408889634f));
     const float2 d = add2(make_float2(ex2_approx_ftz(t.x), ex2_approx_ftz(t.y)), make_float2(1.0f, 1.0f));
     const float2 p = mul2(mul2(gf, make_float2(rcp_approx_ftz(d.x), rcp_approx_ftz(d.y))), uf);
-    const float2 hi = fma2(p, make_float2(eps, eps), p);
-    const float2 lo = fma2(p, make_float2(-eps, -eps), p);
+    const float2 hi = mul2(p, up), lo = mul2(p, down);      // a zero keeps its sign in both
     const V2 r_hi = Vec2<T>::from_floats(hi.x, hi.y), r_lo = Vec2<T>::from_floats(lo.x, lo.y);
     out[i] = *reinterpret_cast<const uint32_t*>(&r_hi);
     if (out[i] != *reinterpret_cast<const uint32_t*>(&r_lo)) undecided |= 1u << i;
   }
-  // no branch above: the sixteen chains overlap.  One undecided pair per turn here (a warp's step has one in 18 %).
-  while (undecided != 0) {
+  largest = max_magnitude16<T>(out);
+  float limit = std::is_same<T, __nv_bfloat16>::value ? 8.271806125530277e-25f : -1.0f;      // 2^-80
+  if (!in_range) limit = fmaxf(limit, max_abs16<T>(u) * 1.3552527156068805e-20f);            // 2^-66 |u|
+  if (!(magnitude_of_pair<T>(largest) > limit)) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const uint32_t gm = g[i] & 0x7fff7fffu, um = u[i] & 0x7fff7fffu;
+      if (((gm & 0xffffu) != 0u && (um & 0xffffu) != 0u) || (gm >> 16 != 0u && um >> 16 != 0u)) undecided |= 1u << i;
+    }
+  }
+  if (undecided == 0u) return;
+  // no branch above: the sixteen chains overlap.  One undecided pair per turn here (bf16: a turn in 21 % of a warp's steps;
+  // fp16: 0.9 turns per step).
+  do {
     const int i = __ffs((int)undecided) - 1;
     undecided &= undecided - 1;
     uint32_t gw = g[0], uw = u[0];
@@ -96,7 +115,8 @@ __device__ __forceinline__ void silu_mul16(const uint32_t (&g)[8], const uint32_
     for (int j = 0; j < 8; ++j) {
       if (i == j) out[j] = *reinterpret_cast<const uint32_t*>(&r);
     }
-  }
+  } while (undecided != 0u);
+  largest = max_magnitude16<T>(out);
 }
 
 // 32 bytes of input per lane (v is left alone where `on` is false): one 256-bit load where the tensor starts on a 32-byte
@@ -201,13 +221,13 @@ mxfp8_group_quant_kernel(const T* __restrict__ input, const int* __restrict__ pr
         uint4 codes;
         uint32_t sf;
         if constexpr (kSiluMul) {
-          uint32_t v[8];
-          silu_mul16<T>(g, up, v);
+          uint32_t v[8], largest;
+          silu_mul16<T>(g, up, v, largest);
           load(g, up);
-          sf = quantize16<T>(v, codes);
+          sf = quantize16<T>(v, largest, codes);
         } else {
           load(next, up);
-          sf = quantize16<T>(g, codes);
+          sf = quantize16<T>(g, max_magnitude16<T>(g), codes);
         }
         // the four scale bytes of the tile as one aligned 32-bit word (two lanes hold the byte of a 32-element block)
         uint32_t w = sf << ((l8 >> 1) * 8);

@@ -113,6 +113,7 @@ struct Vec2<__nv_bfloat16> {
   using type = __nv_bfloat162;
   static __device__ __forceinline__ float2 to_float2(type v) { return __bfloat1622float2(v); }
   static __device__ __forceinline__ float to_float(__nv_bfloat16 v) { return __bfloat162float(v); }
+  static __device__ __forceinline__ float from_bits(uint32_t v) { return __uint_as_float(v << 16); }
   static __device__ __forceinline__ type from_floats(float a, float b) { return __floats2bfloat162_rn(a, b); }
 };
 template <>
@@ -120,6 +121,7 @@ struct Vec2<__half> {
   using type = __half2;
   static __device__ __forceinline__ float2 to_float2(type v) { return __half22float2(v); }
   static __device__ __forceinline__ float to_float(__half v) { return __half2float(v); }
+  static __device__ __forceinline__ float from_bits(uint32_t v) { return __half2float(__ushort_as_half((unsigned short)v)); }
   static __device__ __forceinline__ type from_floats(float a, float b) { return __floats2half2_rn(a, b); }
 };
 
@@ -187,16 +189,11 @@ __device__ __forceinline__ uint32_t max_magnitude16(const uint32_t (&v)[8]) {
   return max_magnitude2<T>(a, b);
 }
 
-// min(|a|, |b|) per half, the sign of the result unspecified; NaN members dropped
-__device__ __forceinline__ uint32_t min_magnitude2(uint32_t a, uint32_t b) {
+// larger of the two halves, each pair compared as unsigned 16-bit numbers
+__device__ __forceinline__ uint32_t max_u16x2(uint32_t a, uint32_t b) {
   uint32_t r;
-  asm("min.xorsign.abs.bf16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+  asm("max.u16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
   return r;
-}
-__device__ __forceinline__ uint32_t min_magnitude16(const uint32_t (&v)[8]) {
-  const uint32_t a = min_magnitude2(min_magnitude2(v[0], v[1]), min_magnitude2(v[2], v[3]));
-  const uint32_t b = min_magnitude2(min_magnitude2(v[4], v[5]), min_magnitude2(v[6], v[7]));
-  return min_magnitude2(a, b);
 }
 
 // larger magnitude of the two halves as fp32 (NaN only if both are)
@@ -228,13 +225,12 @@ __device__ __forceinline__ uint32_t e4m3x4(float2 lo, float2 hi) {
   return r;
 }
 
-// Quantise the 16 elements this lane holds; two neighbouring lanes share one 32-element block.  Same arithmetic as
-// quantize8; returns the block's UE8M0 byte in both lanes.
+// Quantise the 16 elements this lane holds (largest = max_magnitude16 of them); two neighbouring lanes share one 32-element
+// block.  Same arithmetic as quantize8; returns the block's UE8M0 byte in both lanes.
 template <typename T>
-__device__ __forceinline__ uint32_t quantize16(const uint32_t (&v)[8], uint4& codes) {
+__device__ __forceinline__ uint32_t quantize16(const uint32_t (&v)[8], uint32_t largest, uint4& codes) {
   using V2 = typename Vec2<T>::type;
-  uint32_t mx = max_magnitude16<T>(v);
-  mx = max_magnitude2<T>(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
+  const uint32_t mx = max_magnitude2<T>(largest, __shfl_xor_sync(0xffffffffu, largest, 1));
   const float block_max = magnitude_of_pair<T>(mx);
   const uint32_t sf = __nv_cvt_float_to_e8m0(block_max * rcp_approx_ftz(448.0f), __NV_SATFINITE, cudaRoundPosInf);
   // rcp.approx.ftz(2^(sf - 127)): 2^(127 - sf); the subnormal 2^-127 (sf = 0) counts as zero, 1 / 2^127 (254) flushes to
