@@ -177,8 +177,10 @@ mxfp8_group_quant_kernel(const T* __restrict__ input, const int* __restrict__ pr
       const int last = m & 127;
       const int first_word = last <= lane ? 0 : (last - lane + 31) >> 5;      // 0 .. 4
       uint8_t* line = sf_expert + (int64_t)(m >> 7) * kt * 512 + lane * 16;
-      const int q0 = ((i - n_data) * QUANT_WARPS + warp) * QUANT_PAD_ATOMS;
-      for (int q = q0; q < min(kt, q0 + QUANT_PAD_ATOMS); ++q) {
+      // (atoms dealt to the warps one by one: in runs of sixteen, k <= 2048 left seven of the eight without any, 4.6 us
+      // against 2.9 for 16 rows x 2048)
+      const int q0 = (i - n_data) * QUANT_WARPS * QUANT_PAD_ATOMS;
+      for (int q = q0 + warp; q < min(kt, q0 + QUANT_WARPS * QUANT_PAD_ATOMS); q += QUANT_WARPS) {
         uint32_t* words = reinterpret_cast<uint32_t*>(line + (int64_t)q * 512);
         if (first_word == 0 && (reinterpret_cast<uintptr_t>(words) & 15u) == 0) {
           *reinterpret_cast<uint4*>(words) = make_uint4(0, 0, 0, 0);
