@@ -201,7 +201,8 @@ mxfp8_group_quant_kernel(const T* __restrict__ input, const int* __restrict__ pr
       // gate tiles of one row and the next are kt tiles further apart than those inside a row
       const T* src = input + (kSiluMul ? row0 * 2 * kt + t0 + (int64_t)row * kt : row0 * kt + t0) * 128 + l8 * 16;
       uint8_t* dst = quant_output + (row0 * kt + t0) * 128 + l8 * 16;
-      int left = warp_left - group, load_left = left;       // tiles from this lane group's next one on: to do / to load
+      int left = warp_left - group;                            // tiles from this lane group's next one on: to store,
+      int load_left = min(left, n_steps * QUANT_STEP_TILES);   // to load (of this run only: the next one loads its own)
 
       auto load = [&](uint32_t (&g)[8], uint32_t (&up)[8]) {
         const bool on = load_left > 0;
