@@ -140,9 +140,9 @@ struct TileWalk {
 template <typename OutT>
 __global__ void __launch_bounds__(FewRows::THREADS, 1)
 fp8_blockwise_grouped_mm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x16,
-                                const __grid_constant__ CUtensorMap map_x32, const float* __restrict__ scales_a,
-                                const float* __restrict__ scales_b, OutT* __restrict__ d,
-                                const int* __restrict__ problem_sizes, const int* __restrict__ expert_offsets,
+                                const __grid_constant__ CUtensorMap map_x32, const float* scales_a,
+                                const float* scales_b, OutT* __restrict__ d,
+                                const int* problem_sizes, const int* expert_offsets,
                                 int num_experts, int n, int k, int group) {
   using S = FewRows;
   const int block = (int)blockIdx.x, blocks = (int)gridDim.x;
@@ -295,14 +295,14 @@ fp8_blockwise_grouped_mm_kernel(const __grid_constant__ CUtensorMap map_w, const
         const int nk = kt_count - kt0 < CH_KT ? kt_count - kt0 : CH_KT;
         float sb[CH_KT];
 #pragma unroll
-        for (int i = 0; i < CH_KT; ++i) sb[i] = i < nk ? __ldg(sb_row + kt0 + i) : 0.f;
+        for (int i = 0; i < CH_KT; ++i) sb[i] = i < nk ? sb_row[kt0 + i] : 0.f;
         float sa[TOK / 32][CH_KT];
 #pragma unroll
         for (int u = 0; u < TOK / 32; ++u) {
           const int tok = u * 32 + lane;
           const float* sa_row = scales_a + (int64_t)(ti.row0 + tok) * kt_count + kt0;
 #pragma unroll
-          for (int i = 0; i < CH_KT; ++i) sa[u][i] = (tok < ti.valid && i < nk) ? __ldg(sa_row + i) : 0.f;
+          for (int i = 0; i < CH_KT; ++i) sa[u][i] = (tok < ti.valid && i < nk) ? sa_row[i] : 0.f;
         }
         if (!__all_sync(0xffffffffu, ptx::mbar_wait(&ctl->chunk_empty[cs], c_ph ^ 1u, abort_flag))) {
           ok = false;

@@ -132,10 +132,11 @@ __device__ __forceinline__ void load_16_elements(const void* p, bool on, uint32_
 }
 
 // kSiluMul = false: input [rows, k].  kSiluMul = true: input [rows, 2k] = gate | up, quantises silu(gate) * up.
+// The inputs are not __restrict__: the kernel may start while their producer still runs (programmatic launch), and the
+// read-only path wants memory that nothing writes during the kernel's life.
 template <typename T, bool kSiluMul, bool kWide>
 __global__ void __launch_bounds__(QUANT_THREADS, kSiluMul ? QUANT_MIN_BLOCKS_SILU : QUANT_MIN_BLOCKS)
-mxfp8_group_quant_kernel(const T* __restrict__ input, const int* __restrict__ problem_sizes,
-                         const int* __restrict__ expert_offsets, const int* __restrict__ blockscale_offsets,
+mxfp8_group_quant_kernel(const T* input, const int* problem_sizes, const int* expert_offsets, const int* blockscale_offsets,
                          uint8_t* __restrict__ quant_output, uint8_t* __restrict__ scale_factor, int num_experts,
                          int k) {
   __shared__ int table[ES_B200_MAX_EXPERTS + 1];

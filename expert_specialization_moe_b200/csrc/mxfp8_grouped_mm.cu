@@ -221,16 +221,16 @@ __device__ __forceinline__ void grouped_mm_cta(const CUtensorMap& map_w, const C
   // are a second epilogue group
   const bool use_lsu = load_mode == 1;
   const bool epi2 = load_mode == 2;
-  const uint8_t* __restrict__ a_codes = args.a_codes;
-  const uint8_t* __restrict__ w_codes = args.w_codes;
-  const uint8_t* __restrict__ sf_tokens = args.sf_tokens;
-  const uint8_t* __restrict__ sf_weights = args.sf_weights;
+  const uint8_t* a_codes = args.a_codes;
+  const uint8_t* w_codes = args.w_codes;
+  const uint8_t* sf_tokens = args.sf_tokens;
+  const uint8_t* sf_weights = args.sf_weights;
   const int num_rows = args.num_rows;
   const long long sf_token_bytes = args.sf_token_bytes;
   OutT* __restrict__ d = static_cast<OutT*>(args.d);
-  const int* __restrict__ problem_sizes = args.problem_sizes;
-  const int* __restrict__ expert_offsets = args.expert_offsets;
-  const int* __restrict__ blockscale_offsets = args.blockscale_offsets;
+  const int* problem_sizes = args.problem_sizes;
+  const int* expert_offsets = args.expert_offsets;
+  const int* blockscale_offsets = args.blockscale_offsets;
   const int num_experts = args.num_experts, n = args.n, k = args.k, group = args.group;
   const int wait_at_start = args.wait_at_start, last_of_call = args.last_of_call;
   // A kernel that is not the first of its call lets the next one launch at once (measured: 1.6 % on a 0.19 ms call,

@@ -156,8 +156,8 @@ struct Maps {
 template <typename OutT, bool HOLD>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
 mxfp8_grouped_mm_pair_kernel(const __grid_constant__ Maps maps, OutT* __restrict__ d,
-                             const int* __restrict__ problem_sizes, const int* __restrict__ expert_offsets,
-                             const int* __restrict__ blockscale_offsets, int num_experts, int n, int k, int min_rows,
+                             const int* problem_sizes, const int* expert_offsets,
+                             const int* blockscale_offsets, int num_experts, int n, int k, int min_rows,
                              int wait_at_start, const __grid_constant__ RowScatter scatter, uint32_t* counters,
                              int last_of_call, uint32_t earlier_ctas) {
   if (!wait_at_start) pdl_launch_dependents();   // not the first kernel of its call: the next one may launch at once

@@ -20,6 +20,8 @@ __device__ __forceinline__ float rcp_approx_ftz(float a) {
   return b;
 }
 
+// (ld.global.nc: for kernels that start after the producer of the memory has finished, not for those launched with
+// programmatic stream serialisation, during whose life it may still be written)
 __device__ __forceinline__ uint4 ld_stream_16B(const void* p) {
   uint4 v;
   asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];"
@@ -35,7 +37,7 @@ __device__ __forceinline__ void ld_stream_32B_if(const void* p, bool on, uint32_
       "{\n\t"
       ".reg .pred P;\n\t"
       "setp.ne.b32 P, %9, 0;\n\t"
-      "@P ld.global.nc.L1::no_allocate.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];\n\t"
+      "@P ld.global.L1::no_allocate.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];\n\t"
       "}"
       : "+r"(v[0]), "+r"(v[1]), "+r"(v[2]), "+r"(v[3]), "+r"(v[4]), "+r"(v[5]), "+r"(v[6]), "+r"(v[7])
       : "l"(p), "r"((int)on));
@@ -45,7 +47,7 @@ __device__ __forceinline__ void ld_stream_16B_if(const void* p, bool on, uint32_
       "{\n\t"
       ".reg .pred P;\n\t"
       "setp.ne.b32 P, %5, 0;\n\t"
-      "@P ld.global.nc.L1::no_allocate.v4.b32 {%0,%1,%2,%3}, [%4];\n\t"
+      "@P ld.global.L1::no_allocate.v4.b32 {%0,%1,%2,%3}, [%4];\n\t"
       "}"
       : "+r"(a), "+r"(b), "+r"(c), "+r"(d)
       : "l"(p), "r"((int)on));
