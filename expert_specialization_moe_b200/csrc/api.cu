@@ -5,6 +5,7 @@
 #include <mutex>
 
 #include "common.cuh"
+#include "work_items.cuh"
 
 namespace es_b200 {
 
@@ -62,7 +63,7 @@ Tunables& tunables() {
       env_or("ES_B200_MM_PAIR_FIRST_CLUSTERS", 32), env_or("ES_B200_MM_SPLIT_MIN_ROWS", 256),
       env_or("ES_B200_MM_STREAM_MAX_CTAS", 0),     env_or("ES_B200_MM_PAIR_MAX_CLUSTERS", 0),
       env_or("ES_B200_MM_DYNAMIC", 1),             env_or("ES_B200_MM_STREAM_LSU", 1),
-      env_or("ES_B200_MM_ITEM_K_STEPS", 16), env_or("ES_B200_MM_STREAM_MID_LEAD_CTAS", -1),
+      env_or("ES_B200_MM_ITEM_K_STEPS", kDefaultItemKSteps), env_or("ES_B200_MM_STREAM_MID_LEAD_CTAS", -1),
   };
   return t;
 }

@@ -55,6 +55,7 @@
 #include "grouped_mm_call.cuh"
 #include "sm100_ptx.cuh"
 #include "tensormap.cuh"
+#include "work_items.cuh"
 
 namespace es_b200 {
 namespace mm {
@@ -683,17 +684,8 @@ int launch_streaming(const CallArgs& c, int tiny_max, int mid_max, bool want_tin
     ES_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_BYTES));
     configured[dev & 63] = true;
   }
-  // weight tiles per work item: ~mm_item_k_steps K steps per item
-  int item_k_steps = tunables().mm_item_k_steps;
-  if (item_k_steps < 1) item_k_steps = 1;
-  int group = (item_k_steps + kt_count - 1) / kt_count;
-  if (group > 8) group = 8;
-  // ... but as many items as half the SMs while there are the tiles for it: a call of few tiles is a matter of latency, and
-  // up to half the SMs the CTAs of both shapes are on an SM at once.  8 experts, 729 rows, n = 640, k = 384: 23.8 -> 15.7 us;
-  // 24, 3000, 896, 384: 32.0 -> 25.7 (one item per SM 29.1, per three SMs 25.4); 20, 600, 1024, 256: 22.5 -> 17.3 (22.0,
-  // 17.7); 16, 100, 4096, 256: 14.5 -> 13.6 (15.0, 14.6)
   const int64_t tiles = (c.num_experts < c.num_rows ? c.num_experts : c.num_rows) * (c.n / TILE_N);
-  while (group > 1 && tiles / group < info.sm_count / 2) --group;
+  const int group = weight_tiles_per_item(tunables().mm_item_k_steps, kt_count, tiles, info.sm_count);
   // upper bound of the item count known on the host: one token tile per expert
   const int64_t max_tiles = (int64_t)c.num_experts * ((c.n / TILE_N + group - 1) / group);
   int per_shape = (int)(max_tiles < info.sm_count ? max_tiles : info.sm_count);

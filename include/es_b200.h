@@ -239,7 +239,8 @@ int es_b200_ep_route_count_static(const void* topk_ids, int ids_are_int64, int p
  * "mm_dynamic" (0: ignore the work counters), "mm_stream_lsu" (0: the streaming CTAs load by TMA only),
  * "mm_stream_mid_lead_ctas" (CTAs of the 112-token shape that start before the 32-token shape's; negative = built-in
  * default), "mm_item_k_steps" (K steps that a streaming work item should span: it takes that many weight tiles, at
- * most 8).  Unknown name: ES_B200_ERR_INVALID_ARGUMENT.
+ * most 8; at the default, 16, fewer where a call has too few tiles to occupy half the SMs, any other value is taken as
+ * it is).  Unknown name: ES_B200_ERR_INVALID_ARGUMENT.
  */
 int es_b200_set_tunable(const char* name, int value);
 

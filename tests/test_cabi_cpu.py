@@ -103,3 +103,32 @@ def test_product_does_not_import_the_oracle():
     for f in (ROOT / "expert_specialization_moe_b200").rglob("*.py"):
         txt = f.read_text()
         assert "import oracle" not in txt and "from oracle" not in txt, f
+
+
+def test_item_length_setting_is_honoured(tmp_path):
+    """A streaming work item spans the K steps that mm_item_k_steps asks for; only the default is shortened in calls of
+    few weight tiles (the host function of the launch, compiled alone)."""
+    import shutil
+    import subprocess
+    cxx = shutil.which("g++")
+    if cxx is None:
+        pytest.skip("no host compiler")
+    (tmp_path / "t.cpp").write_text('''
+#include <cstdio>
+#include "work_items.cuh"
+int main() {
+  const int steps[] = {-3, 0, 1, 4, 15, 16, 17, 64}, k_steps[] = {1, 2, 3, 7, 16, 56}, tiles[] = {1, 5, 73, 74, 148, 600};
+  for (int s : steps) for (int k : k_steps) for (int t : tiles)
+    std::printf("%d %d %d %d\\n", s, k, t, es_b200::weight_tiles_per_item(s, k, t, 148));
+}''')
+    csrc = ROOT / "expert_specialization_moe_b200" / "csrc"
+    subprocess.run([cxx, "-std=c++17", "-x", "c++", f"-I{csrc}", str(tmp_path / "t.cpp"), "-o", str(tmp_path / "t")], check=True)
+    lines = subprocess.run([str(tmp_path / "t")], check=True, capture_output=True, text=True).stdout.split("\n")
+    rows = [tuple(map(int, l.split())) for l in lines if l]
+    assert len(rows) == 8 * 6 * 6
+    for steps, k_steps, tiles, group in rows:
+        asked = min(-(-max(steps, 1) // k_steps), 8)
+        if steps == 16:      # the most tiles per item, up to the asked, that leave as many items as half the SMs
+            assert group == max([g for g in range(1, asked + 1) if tiles // g >= 74], default=1)
+        else:
+            assert group == asked
