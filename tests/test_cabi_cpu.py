@@ -132,3 +132,19 @@ int main() {
             assert group == max([g for g in range(1, asked + 1) if tiles // g >= 74], default=1)
         else:
             assert group == asked
+
+
+def test_build_with_an_empty_reference_folder(tmp_path, monkeypatch):
+    """build() makes the checker from the reference's sources where they are; a folder without them is no error."""
+    import sys
+    sys.path.insert(0, str(ROOT))
+    import __graft_entry__ as entry
+    monkeypatch.setenv("ES_REFERENCE_DIR", str(tmp_path))
+    run = entry.subprocess.run
+
+    def only_the_product(cmd, *args, **kwargs):
+        assert not any("build_ref" in str(c) for c in cmd), cmd
+        return run(cmd, *args, **kwargs)
+
+    monkeypatch.setattr(entry.subprocess, "run", only_the_product)
+    entry.build()
