@@ -171,8 +171,8 @@ def test_fused_silu_mul_quant_every_gate_value(is_bf16):
 @pytest.mark.parametrize("counts,K", [([1], 128), ([3, 0, 2], 128), ([37, 129, 1], 640), ([33] * 9, 768),
                                       ([700, 1, 260], 2176)])
 def test_quant_unit_edges_and_alignment(counts, K):
-    """Units of one to sixteen steps with ragged last steps (K tiles per row that do not divide a step), an input that
-    starts 16 bytes past a 32-byte boundary, and scale offsets whose padding words are only 4-byte aligned."""
+    """Ragged last steps (K tiles per row that do not divide a step of 32), at most one step per CTA; an input that starts
+    16 bytes past a 32-byte boundary, and scale offsets whose padding words are only 4-byte aligned."""
     import torch
     from expert_specialization_moe_b200 import es_sm100_mxfp8_blockscaled_grouped_quant as quant
     T = sum(counts)
@@ -269,3 +269,83 @@ def test_fused_silu_mul_quant_time_does_not_depend_on_the_values(is_bf16):
         took[name] = sorted(times)[4]
     # measured: up to 1.03 (outliers); 1.4 leaves room for a busy GPU
     assert max(took.values()) < 1.4 * took["plain"], took
+
+
+# Rows that give every CTA several steps of 32 K tiles: a grid is at most 4 CTAs (3 with silu) on each of up to 160 SMs.
+def _rows_for_steps(steps, K, ctas_per_sm):
+    return steps * ctas_per_sm * 160 * 32 * 128 // K + 3
+
+
+def _silu_bits_on_gpu(gu, K):
+    import torch
+    return (torch.nn.functional.silu(gu[:, :K].float()) * gu[:, K:].float()).to(gu.dtype)
+
+
+def _quantise_on_gpu(x, counts, lists, sf_rows, op, K):
+    import torch
+    codes = torch.zeros((x.shape[0], K), dtype=torch.uint8, device="cuda").view(torch.float8_e4m3fn)
+    sf = torch.full((sf_rows, K // 32), 0xCD, dtype=torch.uint8, device="cuda")
+    op(x, *lists, codes, sf)
+    torch.cuda.synchronize()
+    return codes.view(torch.uint8), sf
+
+
+@pytest.mark.parametrize("K,is_bf16", [(128, True), (640, True), (640, False), (2176, False)])
+def test_quant_several_steps_per_cta(K, is_bf16):
+    """Five to six steps per CTA (the loads two steps ahead, the carry of row and tile from step to step, every place of
+    the register rotation), an expert's end and another's start inside a CTA's stretch: against the CPU oracle; and from
+    an input that starts 16 bytes past a 32-byte boundary."""
+    import torch
+    from expert_specialization_moe_b200 import es_sm100_mxfp8_blockscaled_grouped_quant as quant
+    T = _rows_for_steps(6, K, 4)
+    counts = [T // 3, 0, T - T // 3 - 1, 1]
+    x_bits = C.activations_bits(T, K, seed=K, is_bf16=is_bf16)
+    _compare(x_bits, is_bf16, counts)
+    ps, eo, bo, sf_rows = Q.offsets_from_counts(counts, 0, K)
+    lists = [torch.from_numpy(a).to("cuda") for a in (ps, eo, bo)]
+    x = C.bits_to_tensor(x_bits, is_bf16, "cuda")
+    shifted = torch.empty(T * K + 8, dtype=x.dtype, device="cuda")[8:].view(T, K)
+    shifted.copy_(x)
+    assert x.data_ptr() % 32 == 0 and shifted.data_ptr() % 32 == 16
+    for a, b in zip(_quantise_on_gpu(x, counts, lists, sf_rows, quant, K),
+                    _quantise_on_gpu(shifted, counts, lists, sf_rows, quant, K)):
+        assert torch.equal(a, b)
+
+
+def test_quant_long_share_from_a_shifted_input():
+    """More than 48 steps per CTA (dealt eight at a time): the input 16 bytes past a 32-byte boundary gives the bits of
+    the aligned one, which test_quant_full_size_digest_matches_reference covers."""
+    import torch
+    from expert_specialization_moe_b200 import es_sm100_mxfp8_blockscaled_grouped_quant as quant
+    K = 7168
+    T = _rows_for_steps(52, K, 4)
+    counts = [int(c) for c in Q.zipf_counts(T, 64, 1.2, 5)]
+    ps, eo, bo, sf_rows = Q.offsets_from_counts(counts, 0, K)
+    lists = [torch.from_numpy(a).to("cuda") for a in (ps, eo, bo)]
+    x = torch.randn((T, K), device="cuda", generator=torch.Generator(device="cuda").manual_seed(1)).to(torch.bfloat16)
+    shifted = torch.empty(T * K + 8, dtype=x.dtype, device="cuda")[8:].view(T, K)
+    shifted.copy_(x)
+    for a, b in zip(_quantise_on_gpu(x, counts, lists, sf_rows, quant, K),
+                    _quantise_on_gpu(shifted, counts, lists, sf_rows, quant, K)):
+        assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("shift", [0, 8])
+@pytest.mark.parametrize("is_bf16", [True, False])
+@pytest.mark.parametrize("K", [128, 640, 2176])
+def test_fused_silu_mul_quant_several_steps_per_cta(K, is_bf16, shift):
+    """As above for the fused form, against the unfused GPU sequence (whose quantisation the tests above pin)."""
+    import torch
+    from expert_specialization_moe_b200 import es_sm100_mxfp8_blockscaled_grouped_quant as quant
+    from expert_specialization_moe_b200 import es_sm100_mxfp8_silu_mul_grouped_quant as fused
+    T = _rows_for_steps(6, K, 3)
+    counts = [T // 3, 0, T - T // 3 - 1, 1]
+    ps, eo, bo, sf_rows = Q.offsets_from_counts(counts, 0, K)
+    lists = [torch.from_numpy(a).to("cuda") for a in (ps, eo, bo)]
+    gen = torch.Generator(device="cuda").manual_seed(K)
+    gu = torch.empty(T * 2 * K + 8, dtype=torch.bfloat16 if is_bf16 else torch.float16, device="cuda")[shift:shift + T * 2 * K]
+    gu = gu.view(T, 2 * K)
+    gu.copy_(torch.randn((T, 2 * K), device="cuda", generator=gen))
+    for a, b in zip(_quantise_on_gpu(gu, counts, lists, sf_rows, fused, K),
+                    _quantise_on_gpu(_silu_bits_on_gpu(gu, K), counts, lists, sf_rows, quant, K)):
+        assert torch.equal(a, b)
