@@ -99,10 +99,11 @@ def test_blockwise_rejects_bad_arguments():
     ([33], 128, 128),                                    # one K block, one tile
     ([32, 33, 64, 65, 128, 129, 256, 257], 384, 640),    # edges of the split, of the token boxes and of the 128-row tiles
     ([96] * 40, 1024, 1280),                             # ten K blocks: scales read four at a time with a rest of two
-    ([40] * 160, 640, 256),                              # short tiles: more than 32 tiles per CTA in the work list
+    ([40] * 160, 640, 256),                              # short tiles: five or six per CTA
 ])
 def test_blockwise_many_rows_edges(counts, N, K):
-    """Experts of more than 32 rows; an output and scales whose base is only 16- and 4-byte aligned gives the same bits."""
+    """Experts of more than 32 rows; an output that is only 16-byte aligned (and token scales that start elsewhere) gives the
+    same bits."""
     from expert_specialization_moe_b200 import es_fp8_blockwise_scaled_grouped_mm as op
     inp = C.fp8_blockwise_inputs(counts, N, K, seed=17)
     d = C.run_fp8_blockwise_op(inp)
@@ -115,5 +116,42 @@ def test_blockwise_many_rows_edges(counts, N, K):
     op(out, inp["a_q"].to(dev), inp["w_q"].to(dev).transpose(1, 2), sa, inp["sb"].to(dev).transpose(1, 2), ld, ld, ld,
        torch.from_numpy(inp["ps"]).to(dev), torch.from_numpy(inp["eo"]).to(dev),
        torch.empty(16, dtype=torch.uint8, device=dev))
+    torch.cuda.synchronize()
+    assert torch.equal(out.cpu(), d)
+
+
+@pytest.mark.parametrize("E,N", [(220, 3072), (148, 4096)])
+def test_blockwise_many_rows_long_work_list(E, N):
+    """Over 32 tiles per CTA — a second batch of the work list — and, with 148 SMs, exactly 32 (a batch without an end
+    mark), at one K block per tile."""
+    counts = [40] * E
+    inp = C.fp8_blockwise_inputs(counts, N, 128, seed=23)
+    d = C.run_fp8_blockwise_op(inp)
+    _check(inp, d, torch.bfloat16)
+
+
+@pytest.mark.parametrize("shift_a,shift_b", [(1, 0), (0, 1), (1, 1)])
+@pytest.mark.parametrize("K", [512, 1024])
+def test_blockwise_scales_only_4_byte_aligned(K, shift_a, shift_b):
+    """K blocks that the many-rows kernel reads four scales at a time where they start on 16 bytes: scales that do not
+    give the same bits."""
+    from expert_specialization_moe_b200 import es_fp8_blockwise_scaled_grouped_mm as op
+    counts, N = [20, 40, 129, 33], 256
+    inp = C.fp8_blockwise_inputs(counts, N, K, seed=29)
+    d = C.run_fp8_blockwise_op(inp)
+    _check(inp, d, torch.bfloat16)
+    dev = "cuda"
+
+    def shifted(t, by):
+        out = torch.zeros(t.numel() + 4, device=dev)[by:by + t.numel()].view(t.shape)
+        out.copy_(t)
+        assert out.data_ptr() % 16 == 4 * by
+        return out
+
+    out = torch.zeros((sum(counts), N), dtype=torch.bfloat16, device=dev)
+    ld = torch.full((len(counts),), K, dtype=torch.int64, device=dev)
+    op(out, inp["a_q"].to(dev), inp["w_q"].to(dev).transpose(1, 2), shifted(inp["sa"], shift_a),
+       shifted(inp["sb"], shift_b).transpose(1, 2), ld, ld, torch.full_like(ld, N), torch.from_numpy(inp["ps"]).to(dev),
+       torch.from_numpy(inp["eo"]).to(dev), torch.empty(16, dtype=torch.uint8, device=dev))
     torch.cuda.synchronize()
     assert torch.equal(out.cpu(), d)
