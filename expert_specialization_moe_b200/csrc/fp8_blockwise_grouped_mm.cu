@@ -39,25 +39,34 @@
 namespace es_b200 {
 namespace bw {
 
-constexpr int TILE_N = 128;
+constexpr int TILE_N = 128;          // weight rows per tile
 constexpr int TILE_K = 128;
+constexpr int TOK = FEW_ROWS;        // token rows per tile = columns of one TMEM partial
 constexpr int W_BYTES = TILE_N * TILE_K;
+constexpr int STAGE_BYTES = W_BYTES + TOK * TILE_K;
+constexpr int STAGES = 10;
 constexpr int NPART = 4;             // TMEM partial buffers
+constexpr uint32_t TMEM_COLS = NPART * TOK;
 constexpr int CH_KT = 8;             // K blocks per scale chunk
-constexpr int MAX_NCH = 4;           // scale chunks in the ring (per shape: 2 or 4)
-constexpr int MAX_STAGES = 10;
+constexpr int NCH = 4;               // scale chunks in the ring
+constexpr int CHUNK_FLOATS = CH_KT * TOK;
+constexpr int LOADER_WARP0 = 3;      // two scale loaders
+constexpr int EPI_WARP0 = 5;
+constexpr int GROUP_WARPS = 4;       // epilogue group: the four TMEM lane quadrants; two groups take alternate tiles
+constexpr int EPI_WARPS = 2 * GROUP_WARPS;
+constexpr int THREADS = 32 * (EPI_WARP0 + EPI_WARPS);
 constexpr int EPI_TOK = 16;                          // tokens per pass through an epilogue warp's transposition tile
 constexpr int EPI_TILE_BYTES = EPI_TOK * 32 * 2;     // 1 KB
 
 constexpr uint32_t ERR_PRODUCER = 0x1000u, ERR_MMA = 0x2000u, ERR_EPILOGUE = 0x4000u, ERR_SCALES = 0x8000u;
 
 struct SharedCtl {
-  uint64_t full[MAX_STAGES];
-  uint64_t empty[MAX_STAGES];
+  uint64_t full[STAGES];
+  uint64_t empty[STAGES];
   uint64_t part_full[NPART];
   uint64_t part_empty[NPART];     // one arrival per warp of the epilogue group that owns the tile
-  uint64_t chunk_full[MAX_NCH];   // 1 arrival: the chunk's scale loader
-  uint64_t chunk_empty[MAX_NCH];  // one arrival per warp of the epilogue group that owns the tile
+  uint64_t chunk_full[NCH];       // 1 arrival: the chunk's scale loader
+  uint64_t chunk_empty[NCH];      // one arrival per warp of the epilogue group that owns the tile
   uint64_t turn[2];               // turn[x]: epilogue group x may enter the K loop of its next tile
   uint32_t tmem_base;
   int abort_flag;
@@ -65,47 +74,25 @@ struct SharedCtl {
   int tile_prefix[ES_B200_MAX_EXPERTS + 1];   // item prefix [0, E], then the per-expert tables (fill_expert_table)
 };
 
-template <int TOK_TILE_, int STAGES_, int NCH_, int LOADERS_, int GROUPS_>
-struct Shape {
-  static constexpr int GROUPS = GROUPS_;                   // epilogue groups; consecutive tiles alternate between them
-  static constexpr int LOADERS = LOADERS_;                 // scale loader warps (1 or 2)
-  static constexpr int FIRST_EPI_WARP = 3 + LOADERS;
-  static constexpr int TOK_TILE = TOK_TILE_;               // token rows per tile = columns of one TMEM partial
-  static constexpr int STAGES = STAGES_;
-  static constexpr int NCH = NCH_;
-  static constexpr int GROUP_WARPS = 4 * (TOK_TILE / 32);  // 4 lane quadrants x sets of 32 token columns
-  static constexpr int EPI_WARPS = GROUPS * GROUP_WARPS;
-  static constexpr int THREADS = 32 * (FIRST_EPI_WARP + EPI_WARPS);
-  static constexpr int X_BYTES = TOK_TILE * TILE_K;
-  static constexpr int STAGE_BYTES = W_BYTES + X_BYTES;
-  static constexpr uint32_t TMEM_COLS = NPART * TOK_TILE;  // 128 / 256 / 512
-  static constexpr int CHUNK_FLOATS = CH_KT * TOK_TILE;
-  static constexpr size_t SMEM_BYTES = 1024 + (size_t)STAGES * STAGE_BYTES + (size_t)NCH * CHUNK_FLOATS * 4 +
-                                       (size_t)EPI_WARPS * EPI_TILE_BYTES + sizeof(SharedCtl);
-  static_assert(NCH == 2 || NCH == 4, "ring slots are taken modulo a power of two");
-  static_assert(LOADERS == 1 || LOADERS == 2, "chunks alternate between at most two loaders");
-  static_assert(GROUPS == 1 || GROUPS == 2, "tiles alternate between at most two epilogue groups");
-  static_assert(STAGES <= MAX_STAGES, "ring too deep for the control block");
-  // A waiter may be at most one phase ahead of its mbarrier.  Each ring barrier therefore has ONE waiting role per
-  // revolution: K blocks (and chunks) alternate between two lanes (warps), so ring sizes must be even.
-  static_assert(STAGES % 2 == 0 && NPART % 2 == 0, "alternating owners need even rings");
-  static_assert(STAGE_BYTES % 1024 == 0, "stages must keep the 1024-byte alignment of the swizzled tiles");
-  static_assert(SMEM_BYTES <= 232448, "shared memory of one CTA per SM");
-};
-using FewRows = Shape<FEW_ROWS, 10, 4, 2, 2>;    // 20 KB stages, 200 KB in flight; 13 warps
+constexpr size_t SMEM_BYTES = 1024 + (size_t)STAGES * STAGE_BYTES + (size_t)NCH * CHUNK_FLOATS * 4 +
+                              (size_t)EPI_WARPS * EPI_TILE_BYTES + sizeof(SharedCtl);
+static_assert((NCH & (NCH - 1)) == 0 && (NPART & (NPART - 1)) == 0, "ring slots are taken modulo a power of two");
+// A waiter may be at most one phase ahead of its mbarrier.  Each ring barrier therefore has ONE waiting role per
+// revolution: K blocks (and chunks) alternate between two lanes (warps), so ring sizes must be even.
+static_assert(STAGES % 2 == 0 && NPART % 2 == 0 && NCH % 2 == 0, "alternating owners need even rings");
+static_assert(STAGE_BYTES % 1024 == 0, "stages must keep the 1024-byte alignment of the swizzled tiles");
+static_assert(SMEM_BYTES <= 232448, "shared memory of one CTA per SM");
 
 __device__ uint32_t g_status = 0;
 
 struct TileInfo {
-  int e, tt, nt, valid, n_mma, row0;
+  int e, nt, valid, n_mma, row0;
 };
 
-// A work item is `group` consecutive weight tiles of one (expert, token tile); CTA `block` of the `blocks` CTAs of its
-// shape takes the items block, block + blocks, ... and every role walks their tiles in the same order.  The item is
-// decoded once (binary search over the item prefix, a division) and the tiles inside it only advance `nt`: with two
-// K blocks per tile (k = 256) every role spent more time per tile finding out what the tile was than working on it
-// (measured: the producer lane and both MMA lanes ~2200 cycles per tile, almost none of it waiting).
-template <int TOK_TILE>
+// A work item is `group` consecutive weight tiles of one expert; CTA `block` of `blocks` takes the items block, block +
+// blocks, ... and every role walks their tiles in the same order.  The item is decoded once (binary search over the item
+// prefix) and the tiles inside it only advance `nt`: with two K blocks per tile (k = 256) a decode per tile costs every
+// role more time than its work on the tile (the producer lane and both MMA lanes ~2200 cycles, almost none of it waiting).
 struct TileWalk {
   TileInfo ti;
   int item, left, blocks;
@@ -120,16 +107,10 @@ struct TileWalk {
     item += blocks;
     if (item >= total_items) return false;
     ti.e = upper_bound_expert(tab.prefix, num_experts, item);
-    const int i = item - tab.prefix[ti.e];
-    const int m = tab.m(ti.e);
-    const int token_tiles = (m + TOK_TILE - 1) / TOK_TILE;
-    const int ng = i / token_tiles;
-    ti.tt = i - ng * token_tiles;
-    ti.nt = ng * group;
-    const int rem = m - ti.tt * TOK_TILE;
-    ti.valid = rem < TOK_TILE ? rem : TOK_TILE;
+    ti.nt = (item - tab.prefix[ti.e]) * group;
+    ti.valid = tab.m(ti.e);
     ti.n_mma = (ti.valid + 15) & ~15;
-    ti.row0 = tab.row0(ti.e) + ti.tt * TOK_TILE;
+    ti.row0 = tab.row0(ti.e);
     const int rest = n_tiles - ti.nt;
     left = (rest < group ? rest : group) - 1;
     return true;
@@ -138,22 +119,18 @@ struct TileWalk {
 
 // One CTA per SM; serves the experts with 1 .. FEW_ROWS rows.  First kernel of its call.
 template <typename OutT>
-__global__ void __launch_bounds__(FewRows::THREADS, 1)
+__global__ void __launch_bounds__(THREADS, 1)
 fp8_blockwise_grouped_mm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x16,
                                 const __grid_constant__ CUtensorMap map_x32, const float* scales_a,
                                 const float* scales_b, OutT* __restrict__ d,
                                 const int* problem_sizes, const int* expert_offsets,
                                 int num_experts, int n, int k, int group) {
-  using S = FewRows;
   const int block = (int)blockIdx.x, blocks = (int)gridDim.x;
-  constexpr int TOK = S::TOK_TILE;
-  constexpr int STAGES = S::STAGES;
-  constexpr int NCH = S::NCH;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = ptx::align1024(smem_raw);
-  float* chunks = reinterpret_cast<float*>(smem + (size_t)STAGES * S::STAGE_BYTES);        // [NCH][CH_KT][TOK]
-  uint8_t* epi_stage = reinterpret_cast<uint8_t*>(chunks + NCH * S::CHUNK_FLOATS);        // 1 KB per epilogue warp
-  SharedCtl* ctl = reinterpret_cast<SharedCtl*>(epi_stage + (size_t)S::EPI_WARPS * EPI_TILE_BYTES);
+  float* chunks = reinterpret_cast<float*>(smem + (size_t)STAGES * STAGE_BYTES);        // [NCH][CH_KT][TOK]
+  uint8_t* epi_stage = reinterpret_cast<uint8_t*>(chunks + NCH * CHUNK_FLOATS);        // 1 KB per epilogue warp
+  SharedCtl* ctl = reinterpret_cast<SharedCtl*>(epi_stage + (size_t)EPI_WARPS * EPI_TILE_BYTES);
   const int kt_count = k / TILE_K;
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -165,14 +142,14 @@ fp8_blockwise_grouped_mm_kernel(const __grid_constant__ CUtensorMap map_w, const
     }
     for (int p = 0; p < NPART; ++p) {
       ptx::mbar_init(&ctl->part_full[p], 1);
-      ptx::mbar_init(&ctl->part_empty[p], S::GROUP_WARPS);
+      ptx::mbar_init(&ctl->part_empty[p], GROUP_WARPS);
     }
     for (int c = 0; c < NCH; ++c) {
       ptx::mbar_init(&ctl->chunk_full[c], 1);
-      ptx::mbar_init(&ctl->chunk_empty[c], S::GROUP_WARPS);
+      ptx::mbar_init(&ctl->chunk_empty[c], GROUP_WARPS);
     }
-    ptx::mbar_init(&ctl->turn[0], S::GROUP_WARPS);
-    ptx::mbar_init(&ctl->turn[1], S::GROUP_WARPS);
+    ptx::mbar_init(&ctl->turn[0], GROUP_WARPS);
+    ptx::mbar_init(&ctl->turn[1], GROUP_WARPS);
     ctl->abort_flag = 0;
     ptx::fence_mbar_init();
     ptx::prefetch_tensormap(&map_w);
@@ -180,7 +157,7 @@ fp8_blockwise_grouped_mm_kernel(const __grid_constant__ CUtensorMap map_w, const
     ptx::prefetch_tensormap(&map_x32);
   }
   if (warp == 1) {
-    ptx::tmem_alloc(&ctl->tmem_base, S::TMEM_COLS);
+    ptx::tmem_alloc(&ctl->tmem_base, TMEM_COLS);
     ptx::tmem_relinquish();
   }
   // This kernel waits for the stream's earlier work and then lets the many-rows kernel of the call start; that one writes
@@ -196,7 +173,7 @@ fp8_blockwise_grouped_mm_kernel(const __grid_constant__ CUtensorMap map_w, const
     pdl_launch_dependents();
     ptx::tc_fence_before_sync();
     __syncthreads();
-    if (warp == 1) ptx::tmem_dealloc(ctl->tmem_base, S::TMEM_COLS);
+    if (warp == 1) ptx::tmem_dealloc(ctl->tmem_base, TMEM_COLS);
     return;
   }
   const ExpertTable tab = fill_expert_table(ctl->tile_prefix, num_experts, problem_sizes, expert_offsets, nullptr);
@@ -215,7 +192,7 @@ fp8_blockwise_grouped_mm_kernel(const __grid_constant__ CUtensorMap map_w, const
       int s = 0;
       uint32_t ph = 0;
       bool ok = true;
-      TileWalk<TOK> walk(block, blocks);
+      TileWalk walk(block, blocks);
       while (ok && walk.next(tab, num_experts, total_items, n_tiles, group)) {
         const TileInfo& ti = walk.ti;
         const CUtensorMap* xm = ti.n_mma <= 16 ? &map_x16 : &map_x32;
@@ -229,7 +206,7 @@ fp8_blockwise_grouped_mm_kernel(const __grid_constant__ CUtensorMap map_w, const
             atomicOr(&g_status, ERR_PRODUCER);
             break;
           }
-          uint8_t* stage = smem + (size_t)s * S::STAGE_BYTES;
+          uint8_t* stage = smem + (size_t)s * STAGE_BYTES;
           ptx::mbar_arrive_expect_tx(&ctl->full[s], tx);
           ptx::tma_load_2d(stage, &map_w, &ctl->full[s], kt * TILE_K, w_row);
           ptx::tma_load_2d(stage + W_BYTES, xm, &ctl->full[s], kt * TILE_K, ti.row0);
@@ -244,7 +221,7 @@ fp8_blockwise_grouped_mm_kernel(const __grid_constant__ CUtensorMap map_w, const
       const int mine = warp - 1;
       int g = 0;
       bool ok = true;
-      TileWalk<TOK> walk(block, blocks);
+      TileWalk walk(block, blocks);
       while (ok && walk.next(tab, num_experts, total_items, n_tiles, group)) {
         const TileInfo& ti = walk.ti;
         const uint32_t idesc = ptx::make_idesc_f8(TILE_N, ti.n_mma);
@@ -257,7 +234,7 @@ fp8_blockwise_grouped_mm_kernel(const __grid_constant__ CUtensorMap map_w, const
           if (!ptx::mbar_wait(&ctl->part_empty[p], p_ph ^ 1u, abort_flag)) { ok = false; break; }
           if (!ptx::mbar_wait(&ctl->full[s], ph, abort_flag)) { ok = false; break; }
           ptx::tc_fence_after_sync();
-          const uint32_t stage = ptx::smem_u32(smem + (size_t)s * S::STAGE_BYTES);
+          const uint32_t stage = ptx::smem_u32(smem + (size_t)s * STAGE_BYTES);
           const uint64_t a_desc = ptx::make_desc_k_sw128(stage);
           const uint64_t b_desc = ptx::make_desc_k_sw128(stage + W_BYTES);
           const uint32_t d_tmem = tmem_base + p * TOK;
@@ -273,22 +250,21 @@ fp8_blockwise_grouped_mm_kernel(const __grid_constant__ CUtensorMap map_w, const
         }
       }
     }
-  } else if (warp < S::FIRST_EPI_WARP) {
+  } else if (warp < EPI_WARP0) {
     // ------------------------------------------------------------------ scale loaders: chunks alternate between the
     // two warps; c counts chunks over all tiles of this CTA (ring slot = c mod NCH)
-    constexpr int LMASK = S::LOADERS - 1;     // 0: one loader takes every chunk; 1: the two loaders alternate
-    const int mine = warp - 3;
+    const int mine = warp - LOADER_WARP0;
     int c = 0;
     bool ok = true;
-    TileWalk<TOK> walk(block, blocks);
+    TileWalk walk(block, blocks);
     while (ok && walk.next(tab, num_experts, total_items, n_tiles, group)) {
       const int chunks_in_tile = (kt_count + CH_KT - 1) / CH_KT;
       // this warp's chunks of the tile: c, c+1, .. with (c & 1) == mine
-      if (chunks_in_tile == 1 && (c & LMASK) != mine) { ++c; continue; }   // common for small K
+      if (chunks_in_tile == 1 && (c & 1) != mine) { ++c; continue; }   // common for small K
       const TileInfo& ti = walk.ti;
       const float* sb_row = scales_b + ((int64_t)ti.e * n_tiles + ti.nt) * kt_count;
       for (int kt0 = 0; kt0 < kt_count; kt0 += CH_KT, ++c) {
-        if ((c & LMASK) != mine) continue;
+        if ((c & 1) != mine) continue;
         const int cs = c & (NCH - 1);
         const uint32_t c_ph = (uint32_t)(c / NCH) & 1u;
         // the loads do not depend on the ring slot: issue them before waiting for it
@@ -296,14 +272,10 @@ fp8_blockwise_grouped_mm_kernel(const __grid_constant__ CUtensorMap map_w, const
         float sb[CH_KT];
 #pragma unroll
         for (int i = 0; i < CH_KT; ++i) sb[i] = i < nk ? sb_row[kt0 + i] : 0.f;
-        float sa[TOK / 32][CH_KT];
+        float sa[CH_KT];                           // of token `lane`
+        const float* sa_row = scales_a + (int64_t)(ti.row0 + lane) * kt_count + kt0;
 #pragma unroll
-        for (int u = 0; u < TOK / 32; ++u) {
-          const int tok = u * 32 + lane;
-          const float* sa_row = scales_a + (int64_t)(ti.row0 + tok) * kt_count + kt0;
-#pragma unroll
-          for (int i = 0; i < CH_KT; ++i) sa[u][i] = (tok < ti.valid && i < nk) ? sa_row[i] : 0.f;
-        }
+        for (int i = 0; i < CH_KT; ++i) sa[i] = (lane < ti.valid && i < nk) ? sa_row[i] : 0.f;
         if (!__all_sync(0xffffffffu, ptx::mbar_wait(&ctl->chunk_empty[cs], c_ph ^ 1u, abort_flag))) {
           ok = false;
           if (lane == 0) {
@@ -312,15 +284,9 @@ fp8_blockwise_grouped_mm_kernel(const __grid_constant__ CUtensorMap map_w, const
           }
           break;
         }
-        float* chunk = chunks + cs * S::CHUNK_FLOATS;
+        float* chunk = chunks + cs * CHUNK_FLOATS;
 #pragma unroll
-        for (int u = 0; u < TOK / 32; ++u) {
-          const int tok = u * 32 + lane;
-          if (u * 32 < ti.n_mma) {                 // columns past n_mma are never read (warp-uniform)
-#pragma unroll
-            for (int i = 0; i < CH_KT; ++i) chunk[i * TOK + tok] = sa[u][i] * sb[i];
-          }
-        }
+        for (int i = 0; i < CH_KT; ++i) chunk[i * TOK + lane] = sa[i] * sb[i];
         __syncwarp();
         if (lane == 0) ptx::mbar_arrive(&ctl->chunk_full[cs]);
       }
@@ -332,30 +298,27 @@ fp8_blockwise_grouped_mm_kernel(const __grid_constant__ CUtensorMap map_w, const
     // are strictly serial (turn barriers): a group that waited on part_full / chunk_full for a tile further ahead
     // would be more than one phase ahead of those barriers, and a parity wait cannot tell phases n and n+2 apart.
     const int q = warp & 3;                           // TMEM lane quadrant of this warp
-    const int egroup = (warp - S::FIRST_EPI_WARP) / S::GROUP_WARPS;
-    const int col0 = (((warp - S::FIRST_EPI_WARP) % S::GROUP_WARPS) >> 2) * 32;   // this warp's 32 token columns
-    OutT* stage_warp = reinterpret_cast<OutT*>(epi_stage) + (warp - S::FIRST_EPI_WARP) * (EPI_TOK * 32);
+    const int egroup = (warp - EPI_WARP0) / GROUP_WARPS;
+    OutT* stage_warp = reinterpret_cast<OutT*>(epi_stage) + (warp - EPI_WARP0) * (EPI_TOK * 32);
     const int part = lane & 3;
     int g = 0;                                        // K blocks over all tiles of this CTA
     int c = 0;                                        // scale chunks over all tiles of this CTA
     bool alive = true;
     uint32_t turn_ph = 0;
     int tile_index = 0;
-    TileWalk<TOK> walk(block, blocks);
+    TileWalk walk(block, blocks);
     while (alive && walk.next(tab, num_experts, total_items, n_tiles, group)) {
       const int my_index = tile_index++;
-      if ((my_index & (S::GROUPS - 1)) != egroup) {   // the other group's tile
+      if ((my_index & 1) != egroup) {   // the other group's tile
         g += kt_count;
         c += (kt_count + CH_KT - 1) / CH_KT;
         continue;
       }
       const TileInfo& ti = walk.ti;
-      const bool has_cols = col0 < ti.n_mma;          // warp-uniform: a set past the tile's tokens only keeps the
-                                                      // barriers moving
       float acc[32];
 #pragma unroll
       for (int j = 0; j < 32; ++j) acc[j] = 0.f;
-      if (S::GROUPS == 2 && my_index > 0) {            // the other group has left the K loop of the previous tile
+      if (my_index > 0) {                              // the other group has left the K loop of the previous tile
         if (!__all_sync(0xffffffffu, ptx::mbar_wait(&ctl->turn[egroup], turn_ph, abort_flag))) {
           if (lane == 0) {
             *abort_flag = 1;
@@ -382,24 +345,20 @@ fp8_blockwise_grouped_mm_kernel(const __grid_constant__ CUtensorMap map_w, const
           break;
         }
         uint32_t v[32];
-        if (has_cols) {
-          ptx::tc_fence_after_sync();
-          ptx::tc_ld_32x32b_x32(tmem_base + p * TOK + col0 + ((uint32_t)(q * 32) << 16), v);
-          ptx::tc_wait_ld();
-          ptx::tc_fence_before_sync();
-        }
+        ptx::tc_fence_after_sync();
+        ptx::tc_ld_32x32b_x32(tmem_base + p * TOK + ((uint32_t)(q * 32) << 16), v);
+        ptx::tc_wait_ld();
+        ptx::tc_fence_before_sync();
         __syncwarp();
         if (lane == 0) ptx::mbar_arrive(&ctl->part_empty[p]);      // the tensor core may overwrite this partial
-        if (has_cols) {
-          const float4* srow = reinterpret_cast<const float4*>(chunks + cs * S::CHUNK_FLOATS + ki * TOK + col0);
+        const float4* srow = reinterpret_cast<const float4*>(chunks + cs * CHUNK_FLOATS + ki * TOK);
 #pragma unroll
-          for (int j4 = 0; j4 < 8; ++j4) {
-            const float4 sc = srow[j4];                // same address in every lane: broadcast
-            acc[j4 * 4 + 0] = fmaf(__uint_as_float(v[j4 * 4 + 0]), sc.x, acc[j4 * 4 + 0]);
-            acc[j4 * 4 + 1] = fmaf(__uint_as_float(v[j4 * 4 + 1]), sc.y, acc[j4 * 4 + 1]);
-            acc[j4 * 4 + 2] = fmaf(__uint_as_float(v[j4 * 4 + 2]), sc.z, acc[j4 * 4 + 2]);
-            acc[j4 * 4 + 3] = fmaf(__uint_as_float(v[j4 * 4 + 3]), sc.w, acc[j4 * 4 + 3]);
-          }
+        for (int j4 = 0; j4 < 8; ++j4) {
+          const float4 sc = srow[j4];                  // same address in every lane: broadcast
+          acc[j4 * 4 + 0] = fmaf(__uint_as_float(v[j4 * 4 + 0]), sc.x, acc[j4 * 4 + 0]);
+          acc[j4 * 4 + 1] = fmaf(__uint_as_float(v[j4 * 4 + 1]), sc.y, acc[j4 * 4 + 1]);
+          acc[j4 * 4 + 2] = fmaf(__uint_as_float(v[j4 * 4 + 2]), sc.z, acc[j4 * 4 + 2]);
+          acc[j4 * 4 + 3] = fmaf(__uint_as_float(v[j4 * 4 + 3]), sc.w, acc[j4 * 4 + 3]);
         }
         if (ki == CH_KT - 1 || kt == kt_count - 1) {          // done with this scale chunk
           __syncwarp();
@@ -408,28 +367,24 @@ fp8_blockwise_grouped_mm_kernel(const __grid_constant__ CUtensorMap map_w, const
         }
       }
       if (!alive) break;
-      if (S::GROUPS == 2) {
-        __syncwarp();
-        if (lane == 0) ptx::mbar_arrive(&ctl->turn[egroup ^ 1]);
-      }
-      // output: this warp's 32 tokens x 32 n, 16 tokens at a time through its 1 KB tile, 128-bit stores (4 lanes per
+      __syncwarp();
+      if (lane == 0) ptx::mbar_arrive(&ctl->turn[egroup ^ 1]);
+      // output: this warp's 32 n of up to 32 tokens, 16 tokens at a time through its 1 KB tile, 128-bit stores (4 lanes per
       // 64-byte row piece)
-      if (col0 < ti.valid) {
-        OutT* dst = d + (int64_t)(ti.row0 + col0) * n + (ti.nt * TILE_N + q * 32);
+      OutT* dst = d + (int64_t)ti.row0 * n + (ti.nt * TILE_N + q * 32);
 #pragma unroll
-        for (int h = 0; h < 32 / EPI_TOK; ++h) {
+      for (int h = 0; h < TOK / EPI_TOK; ++h) {
 #pragma unroll
-          for (int j = 0; j < EPI_TOK; ++j) stage_warp[j * 32 + lane] = out_from_f32<OutT>(acc[h * EPI_TOK + j]);
-          __syncwarp();
+        for (int j = 0; j < EPI_TOK; ++j) stage_warp[j * 32 + lane] = out_from_f32<OutT>(acc[h * EPI_TOK + j]);
+        __syncwarp();
 #pragma unroll
-          for (int it = 0; it < EPI_TOK / 8; ++it) {
-            const int tok = it * 8 + (lane >> 2);
-            const uint4 val = *reinterpret_cast<const uint4*>(stage_warp + tok * 32 + part * 8);
-            const int row = col0 + h * EPI_TOK + tok;
-            if (row < ti.valid) *reinterpret_cast<uint4*>(dst + (int64_t)(h * EPI_TOK + tok) * n + part * 8) = val;
-          }
-          __syncwarp();
+        for (int it = 0; it < EPI_TOK / 8; ++it) {
+          const int tok = it * 8 + (lane >> 2);
+          const uint4 val = *reinterpret_cast<const uint4*>(stage_warp + tok * 32 + part * 8);
+          const int row = h * EPI_TOK + tok;
+          if (row < ti.valid) *reinterpret_cast<uint4*>(dst + (int64_t)row * n + part * 8) = val;
         }
+        __syncwarp();
       }
     }
   }
@@ -438,7 +393,7 @@ fp8_blockwise_grouped_mm_kernel(const __grid_constant__ CUtensorMap map_w, const
   __syncthreads();
   if (warp == 1) {
     __syncwarp();
-    ptx::tmem_dealloc(tmem_base, S::TMEM_COLS);
+    ptx::tmem_dealloc(tmem_base, TMEM_COLS);
   }
 }
 
@@ -451,7 +406,6 @@ static int tiles_per_item(int k) {
 
 template <typename OutT>
 int launch_few_rows(const CallArgs& c) {
-  using S = FewRows;
   DeviceInfo info;
   int rc = get_device_info(&info);
   if (rc != ES_B200_OK) return rc;
@@ -465,7 +419,7 @@ int launch_few_rows(const CallArgs& c) {
   int dev = 0;
   ES_CUDA_TRY(cudaGetDevice(&dev));
   if (!configured[dev & 63]) {
-    ES_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::SMEM_BYTES));
+    ES_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_BYTES));
     configured[dev & 63] = true;
   }
   const int group = tiles_per_item(c.k);
@@ -474,8 +428,8 @@ int launch_few_rows(const CallArgs& c) {
   const int64_t max_items = experts * ((c.n / TILE_N + group - 1) / group);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)(max_items < info.sm_count ? max_items : info.sm_count));
-  cfg.blockDim = dim3(S::THREADS);
-  cfg.dynamicSmemBytes = S::SMEM_BYTES;
+  cfg.blockDim = dim3(THREADS);
+  cfg.dynamicSmemBytes = SMEM_BYTES;
   cfg.stream = c.stream;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;

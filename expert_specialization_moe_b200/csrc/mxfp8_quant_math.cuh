@@ -104,10 +104,6 @@ __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
   return unpack_f32x2(r);
 }
 
-__device__ __forceinline__ void st_stream_8B(void* p, uint2 v) {
-  asm volatile("st.global.cs.v2.u32 [%0], {%1,%2};" ::"l"(p), "r"(v.x), "r"(v.y) : "memory");
-}
-
 template <typename T>
 struct Vec2;
 template <>
