@@ -591,7 +591,7 @@ def bench_blockwise(args, E, T, N, K, desc, device, rank, world, dist):
         peak, peak_kind = peak_hbm()
         achieved = abytes_local / (ms * 1e-3) / 1e9
         value = 2.0 * T * N * K / (float(stats[0]) * 1e-3) / 1e12
-        buckets = 1 + (rows > 32)        # launches: the <= 32-row shape, then the two larger shapes in one launch
+        buckets = 1 + (rows > 32)        # launches: the few-rows kernel, then the many-rows kernel
         line = {"metric": "FP8-blockwise grouped GEMM TFLOPS", "value": value, "unit": "TFLOP/s", "n_gpus": world,
                 "steps": args.steps, "warmup": args.warmup, "ms_per_step": float(stats[0]), "higher_is_better": True,
                 "scaling": "strong", "vs_baseline": value / PUBLISHED_H200_TFLOPS[args.workload],

@@ -149,8 +149,8 @@ dispatch_quant_push_kernel(const T* __restrict__ x, const int* __restrict__ dst_
 
 // The received rows' scale bytes go to their swizzled position, their return addresses to the (GPU, slot) table.  Offsets
 // are range-checked: a bad one is skipped and reported.  One thread per (row, K tile), four of them in flight: the
-// records are 16 + k / 32 bytes, and a warp per row (one dependent pass of 16 useful lanes at k = 2048) took 16.8 us for
-// 131072 rows, the bytes are worth 3; this way 12.2.
+// records are 16 + k / 32 bytes, and a warp per row would be one dependent pass of 16 useful lanes at k = 2048 (131072 rows:
+// 16.8 us, this way 12.2, the bytes are worth 3).
 constexpr int UNPACK_UNROLL = 4;
 __global__ void __launch_bounds__(THREADS)
 unpack_side_kernel(const uint8_t* __restrict__ side, const int* __restrict__ num_rows_dev, uint8_t* __restrict__ scales,
@@ -163,7 +163,7 @@ unpack_side_kernel(const uint8_t* __restrict__ side, const int* __restrict__ num
   if (rows > capacity_rows) rows = capacity_rows;
   const long long words = rows * kt;                     // kt <= 128: below 2^38
   const long long threads = (long long)gridDim.x * THREADS;
-  // 32-bit row arithmetic inside a stretch of the grid: (row, tile) of the thread's first word, then steps of the grid
+  // (row, tile) of the thread's first word by one division, of the next ones by steps of the grid
   const long long first = (long long)blockIdx.x * THREADS + threadIdx.x;
   long long r = first / kt;
   unsigned q = (unsigned)(first - r * kt);
@@ -252,8 +252,8 @@ struct Pack2<__half> {
 
 // A warp per (token, 256 columns); a lane accumulates 8 columns in fp32 over the token's top-k rows, in order
 // j = 0 .. topk-1.  Bound by HBM (topk + 1 rows per token): the rows are requested SUM_ROWS at a time before the first is
-// used, and the work is cut by columns too, so that the last round of warps is short.  A warp per token with one row in
-// flight took 130 us for 16384 tokens x top-8 at n = 2048 (0.60 GB), this way 96.
+// used, and the work is cut by columns too, so that the last round of warps is short.  16384 tokens x top-8 at n = 2048
+// (0.60 GB): 96 us; a warp per token with one row in flight 130.
 constexpr int SUM_ROWS = 8;
 template <typename T>
 __global__ void __launch_bounds__(THREADS)

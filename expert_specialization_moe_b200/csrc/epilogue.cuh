@@ -13,7 +13,6 @@
 
 namespace es_b200 {
 
-
 // Optional destination map of the output rows (expert-parallel combine fused into the GEMM): output row r goes to row
 // meta[r].y of the [slots, n] array base[meta[r].x] — another GPU's buffer mapped into this process, or a local one —
 // instead of row r of d.  meta == nullptr: dense output.  Entries out of range are skipped and reported.

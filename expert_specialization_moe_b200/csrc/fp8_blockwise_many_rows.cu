@@ -10,8 +10,9 @@
 // (a quarter less traffic) hold 64 accumulators a thread, spill, and were 14 % slower; two K blocks per stage and
 // hand-over 13 % slower; the kernel serving the experts of <= 32 rows too (128 MMA rows for a few tokens) 4-8 % slower
 // there than the few-rows kernel.
-// At that size the call takes 155 us (burst; 0.189 ms in a second-long loop), 211 (0.235) before this kernel; E = 256,
-// n = 7168, k = 256, 24576 rows 165 us, 228 before; E = 64, n = k = 2048, 32768 rows 226 us, 308 before.
+// At that size the whole call takes 151 us back to back; with the tokens on N (this kernel's predecessor) 212.  Experts of
+// 33 to 64 rows, whose MMAs are half empty, gain as well, at long K too (bound by HBM): E = 256, 48 rows, n = 512, k = 7168
+// 175 and 213 us; E = 32, 48 rows, n = 4096, k = 7168 167 and 242; E = 128, 33 rows, n = 4096, k = 2048 197 and 286.
 //
 //   warp 0     producer: TMA loads of the token tile and the weight tile per K block
 //   warps 1, 2 MMA issue, one lane each: warp 1 (which also owns the TMEM allocation) takes the even K blocks, warp 2

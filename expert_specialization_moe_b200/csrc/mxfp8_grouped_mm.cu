@@ -91,9 +91,10 @@ struct Shape {
   // is what its bytes take at HBM speed; a 112-token tile ~10000, its loads ~1500).  The four loader warps are then a
   // second epilogue group (every ring slot by TMA, from two producer warps).  A tile of up to 32 tokens is one 32-token
   // chunk: the groups take alternate tiles, one accumulator buffer each.  A larger tile they share, alternate chunks each
-  // (where a CTA has only a few tiles, alternate tiles would leave one group idle).  Reference benchmark's row distribution at n = 7168, k = 256: the 187 experts of <= 32 rows
-  // alone 98.8 -> 80.8 us, the whole call 187 -> 168.  The 32-token shape runs that way up to two K steps (with 3 to 5 its
-  // second load path is worth more: E = 264, n = 3968, k = 384 54.5 us against 59.9), the 112-token shape below eight.
+  // (where a CTA has only a few tiles, alternate tiles would leave one group idle).  The reference benchmark's row
+  // distribution at n = 7168, k = 256: the 187 experts of <= 32 rows alone 81 us, 99 with one group, the whole call 168
+  // and 187.  The 32-token shape runs that way up to two K steps (with 3 to 5 its second load path is worth more: E = 264,
+  // n = 3968, k = 384 54.5 us against 59.9), the 112-token shape below eight.
   static constexpr bool GROUPS_SHARE_TILES = TOK_TILE > 32;
   static constexpr int STORE_TOK = STORE_TOK_;             // tokens per pass through a warp's store tile
   static constexpr int STORE_TILE_BYTES = STORE_TOK * 32 * 2;
@@ -336,27 +337,27 @@ __device__ __forceinline__ void grouped_mm_cta(const CUtensorMap& map_w, const C
       if (t < 0) break;
       const TileInfo ti = decode_tile(t, tab, num_experts, n_tiles, group);
       for (int sub = 0; ok && sub < ti.n_sub; ++sub) {
-      const int nt = ti.nt + sub;
-      if (!epi2 || S::GROUPS_SHARE_TILES || acc == group_id) {
-      const bool got = ptx::mbar_wait(&ctl->tmem_full[acc], acc_ph, abort_flag);
-      if (!__all_sync(0xffffffffu, got)) { ok = false; break; }
-      ptx::tc_fence_after_sync();
-      const uint32_t taddr = tmem_base + acc * S::ACC_COLS + ((uint32_t)(quad * 32) << 16);
-      OutT* dst = d + (int64_t)ti.row0 * n + (nt * TILE_N + quad * 32);
-      drain_partial_sums<OutT, S::LANES, S::STORE_TOK>(
-          taddr, TOK_TILE, kt_count < lanes ? kt_count : lanes, ti.n_mma, ti.valid,
-          stage_warp, dst, n, lane,
-          [&] {
-            // all of this warp's accumulator reads are done: hand the buffer back to the MMA lanes
-            ptx::tc_fence_before_sync();
-            __syncwarp();
-            if (lane == 0) ptx::mbar_arrive(&ctl->tmem_empty[acc]);
-          },
-          scatter, ti.row0, nt * TILE_N + quad * 32, &g_status, kt_count >= SHORT_K_STEPS,
-          S::GROUPS_SHARE_TILES ? group_id * 32 : 0, epi2 && S::GROUPS_SHARE_TILES ? 64 : 32);
-      }   // a tile of this group
-      acc ^= 1;
-      if (acc == 0) acc_ph ^= 1u;
+        const int nt = ti.nt + sub;
+        if (!epi2 || S::GROUPS_SHARE_TILES || acc == group_id) {
+          const bool got = ptx::mbar_wait(&ctl->tmem_full[acc], acc_ph, abort_flag);
+          if (!__all_sync(0xffffffffu, got)) { ok = false; break; }
+          ptx::tc_fence_after_sync();
+          const uint32_t taddr = tmem_base + acc * S::ACC_COLS + ((uint32_t)(quad * 32) << 16);
+          OutT* dst = d + (int64_t)ti.row0 * n + (nt * TILE_N + quad * 32);
+          drain_partial_sums<OutT, S::LANES, S::STORE_TOK>(
+              taddr, TOK_TILE, kt_count < lanes ? kt_count : lanes, ti.n_mma, ti.valid,
+              stage_warp, dst, n, lane,
+              [&] {
+                // all of this warp's accumulator reads are done: hand the buffer back to the MMA lanes
+                ptx::tc_fence_before_sync();
+                __syncwarp();
+                if (lane == 0) ptx::mbar_arrive(&ctl->tmem_empty[acc]);
+              },
+              scatter, ti.row0, nt * TILE_N + quad * 32, &g_status, kt_count >= SHORT_K_STEPS,
+              S::GROUPS_SHARE_TILES ? group_id * 32 : 0, epi2 && S::GROUPS_SHARE_TILES ? 64 : 32);
+        }   // a tile of this group
+        acc ^= 1;
+        if (acc == 0) acc_ph ^= 1u;
       }   // weight tiles of the item
     }
     if (!ok && lane == 0) {
@@ -386,20 +387,20 @@ __device__ __forceinline__ void grouped_mm_cta(const CUtensorMap& map_w, const C
     const uint64_t my_hint = lane == 0 ? ptx::kL2EvictFirst : lane == 1 ? ptx::kL2EvictLast : ptx::kL2EvictNormal;
     bool ok = true;
     for (int sub = 0; ok && sub < ti.n_sub; ++sub) {
-    const int my_c1 = my_c1_first + sub * my_c1_step;
-    for (int kt = 0; kt < kt_count; ++kt) {
-      if (!split_slots || (s & 1) == parity) {
-        ok = __all_sync(0xffffffffu, ptx::mbar_wait(&ctl->empty[s], ph ^ 1u, abort_flag));
-        if (!ok) break;
-        uint8_t* stage = smem + (size_t)s * STAGE_BYTES;
-        if (lane == 0) ptx::mbar_arrive_expect_tx(&ctl->full[s], tx);
-        __syncwarp();
-        if (lane < 4)
-          ptx::tma_load_2d_hint(stage + my_off, my_map, &ctl->full[s], lane < 2 ? kt * TILE_K : 0,
-                                lane < 2 ? my_c1 : my_c1 + kt, my_hint);
+      const int my_c1 = my_c1_first + sub * my_c1_step;
+      for (int kt = 0; kt < kt_count; ++kt) {
+        if (!split_slots || (s & 1) == parity) {
+          ok = __all_sync(0xffffffffu, ptx::mbar_wait(&ctl->empty[s], ph ^ 1u, abort_flag));
+          if (!ok) break;
+          uint8_t* stage = smem + (size_t)s * STAGE_BYTES;
+          if (lane == 0) ptx::mbar_arrive_expect_tx(&ctl->full[s], tx);
+          __syncwarp();
+          if (lane < 4)
+            ptx::tma_load_2d_hint(stage + my_off, my_map, &ctl->full[s], lane < 2 ? kt * TILE_K : 0,
+                                  lane < 2 ? my_c1 : my_c1 + kt, my_hint);
+        }
+        if (++s == STAGES) { s = 0; ph ^= 1u; }
       }
-      if (++s == STAGES) { s = 0; ph ^= 1u; }
-    }
     }   // weight tiles of the item
     return ok;
   };
