@@ -391,6 +391,7 @@ fp8_blockwise_grouped_mm_kernel(const __grid_constant__ CUtensorMap map_w, const
 
   ptx::tc_fence_before_sync();
   __syncthreads();
+  ptx::settle_if_aborted(abort_flag);
   if (warp == 1) {
     __syncwarp();
     ptx::tmem_dealloc(tmem_base, TMEM_COLS);

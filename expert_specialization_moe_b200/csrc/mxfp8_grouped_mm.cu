@@ -614,6 +614,7 @@ __device__ __forceinline__ void grouped_mm_cta(const CUtensorMap& map_w, const C
 
   ptx::tc_fence_before_sync();
   __syncthreads();
+  ptx::settle_if_aborted(abort_flag);
   if (warp == 1) {
     __syncwarp();
     ptx::tmem_dealloc(tmem_base, TMEM_COLS);

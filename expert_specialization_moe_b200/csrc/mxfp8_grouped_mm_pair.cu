@@ -539,6 +539,8 @@ mxfp8_grouped_mm_pair_kernel(const __grid_constant__ Maps maps, OutT* __restrict
 
   // neither CTA may leave (or free TMEM) while its partner can still signal it or read its shared memory
   ptx::tc_fence_before_sync();
+  __syncthreads();
+  ptx::settle_if_aborted(abort_flag);
   ptx::cluster_sync();
   if (warp == 1) {
     __syncwarp();

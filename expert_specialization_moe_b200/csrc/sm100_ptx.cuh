@@ -81,6 +81,16 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
   }
 }
 
+// Called by all threads of a CTA once its roles have ended (block barrier in front), before TMEM is freed.  After a wait
+// that gave up, loads into the CTA's shared memory and MMAs that read it and write TMEM may still be on their way: the
+// CTA keeps both for a millisecond, a thousand times what they take, before the next one on the SM gets them.
+constexpr uint64_t kSettleNs = 1000000ull;
+__device__ __forceinline__ void settle_if_aborted(volatile int* abort_flag) {
+  if (*abort_flag == 0) return;
+  const uint64_t t0 = globaltimer_ns();
+  while (globaltimer_ns() - t0 < kSettleNs) __nanosleep(1000);
+}
+
 // ---- TMA / bulk copies (no cluster multicast anywhere) -----------------------------------------
 // L2 eviction-priority hints (createpolicy encodings: evict_first / evict_last / evict_normal)
 constexpr uint64_t kL2EvictFirst = 0x12F0000000000000ull;

@@ -39,3 +39,17 @@ def test_kernels_with_read_only_loads_are_launched_without_programmatic_serialis
         code = _code(path.name)
         if "ld_stream_16B(" in code:
             assert "cudaLaunchAttributeProgrammaticStreamSerialization" not in code, path.name
+
+
+@pytest.mark.parametrize("name", [p.name for p in sorted(CSRC.glob("*.cu")) if "mbar_wait(" in p.read_text()])
+def test_a_kernel_that_gave_up_lets_its_copies_land(name):
+    """Between the end of the roles and the release of TMEM: a CTA whose roles gave up may have loads into its shared
+    memory and MMAs in flight.  (A wait cannot be made to run out in a test without withholding an arrival from a running
+    pipeline, so the sources are checked.)"""
+    code = re.sub(r"\s+", " ", _code(name))
+    last_free = max(m.start() for m in re.finditer(r"ptx::tmem_dealloc(_pair)?\(tmem_base", code))
+    tail = code[:last_free]
+    settle = tail.rfind("ptx::settle_if_aborted(abort_flag);")
+    assert settle > 0, "no settling before the release of TMEM"
+    assert tail[:settle].rstrip().endswith("__syncthreads();"), "all roles must have ended"
+    assert "mbar_wait" not in tail[settle:] and "tma_load" not in tail[settle:]
