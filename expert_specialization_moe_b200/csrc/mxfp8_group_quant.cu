@@ -34,11 +34,13 @@ constexpr int QUANT_WARPS = QUANT_THREADS / 32;
 constexpr int QUANT_WARP_TILES = 4;           // a warp's four groups of eight lanes, one 128-element K tile each
 constexpr int QUANT_STEP_TILES = QUANT_WARPS * QUANT_WARP_TILES;
 constexpr int QUANT_PAD_ATOMS = 16;           // scale atoms per warp and step of padding work
-// Consecutive steps that a CTA takes before it moves on by a grid's worth: an equal share of the list in one stretch, but
-// eight steps where the share is long and the kernel is bound by memory — 592 streams 0.8 MB apart cost it 10 % of the
-// bandwidth (32768 x 7168: 134 us in one stretch, 121 in chunks of 8, 125 of 4, 140 of 2; with silu, bound by its
-// arithmetic, 106 us either way, and the last round of chunks is not paid for).
-constexpr int QUANT_CHUNK = 8, QUANT_LONG_SHARE = 48;
+// Consecutive steps that a CTA takes before it moves on by a grid's worth: its equal share of the list in one stretch, or
+// eight where the share is long and the kernel is bound by memory: 592 streams far apart cost bandwidth, the uneven last
+// round of chunks costs the most where there are few rounds.  One stretch / chunks of 8, us: share 16 23.6 / 26.7, 20
+// 28.3 / 30.0, 24 33.5 / 34.3, 26 36.1 / 36.8, 28 38.6 / 38.2, 30 41.2 / 38.7, 36 48.9 / 46.7, 48 65.5 / 60.5 (k = 768;
+// k = 2048 and 7168 cross between 22 and 28 too); 97 (32768 x 7168) 128 / 125.  Chunks of 4 and 2 are slower than of 8
+// there.  With silu, bound by its arithmetic, one stretch is never slower.
+constexpr int QUANT_CHUNK = 8, QUANT_LONG_SHARE = 27;
 // registers: two steps of input in flight per warp; the fused variant holds gate and up of both
 constexpr int QUANT_MIN_BLOCKS = 4, QUANT_MIN_BLOCKS_SILU = 3;
 
