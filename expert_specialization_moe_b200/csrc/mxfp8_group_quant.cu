@@ -39,7 +39,7 @@ constexpr int QUANT_PAD_ATOMS = 16;           // scale atoms per warp and step o
 // round of chunks costs the most where there are few rounds.  One stretch / chunks of 8, us: share 16 23.6 / 26.7, 20
 // 28.3 / 30.0, 24 33.5 / 34.3, 26 36.1 / 36.8, 28 38.6 / 38.2, 30 41.2 / 38.7, 36 48.9 / 46.7, 48 65.5 / 60.5 (k = 768;
 // k = 2048 and 7168 cross between 22 and 28 too); 97 (32768 x 7168) 128 / 125.  Chunks of 4 and 2 are slower than of 8
-// there.  With silu, bound by its arithmetic, one stretch is never slower.
+// there.  With silu, bound by its arithmetic, no difference (131072 x 768), and the last round is not paid for.
 constexpr int QUANT_CHUNK = 8, QUANT_LONG_SHARE = 27;
 // registers: two steps of input in flight per warp; the fused variant holds gate and up of both
 constexpr int QUANT_MIN_BLOCKS = 4, QUANT_MIN_BLOCKS_SILU = 3;

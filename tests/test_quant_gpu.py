@@ -312,22 +312,32 @@ def test_quant_several_steps_per_cta(K, is_bf16):
         assert torch.equal(a, b)
 
 
-def test_quant_long_share_from_a_shifted_input():
-    """More than 48 steps per CTA (dealt eight at a time): the input 16 bytes past a 32-byte boundary gives the bits of
-    the aligned one, which test_quant_full_size_digest_matches_reference covers."""
+@pytest.mark.parametrize("steps,K", [(30, 640), (52, 7168)])
+def test_quant_long_share(steps, K):
+    """More than 27 steps per CTA, dealt eight at a time, over several experts: the bits of one call per expert, whose
+    CTAs have fewer; and the same from an input that starts 16 bytes past a 32-byte boundary."""
     import torch
     from expert_specialization_moe_b200 import es_sm100_mxfp8_blockscaled_grouped_quant as quant
-    K = 7168
-    T = _rows_for_steps(52, K, 4)
-    counts = [int(c) for c in Q.zipf_counts(T, 64, 1.2, 5)]
+    T = _rows_for_steps(steps, K, 4)
+    counts = [T // 5, T // 4, 1, T - T // 5 - T // 4 - 1]
     ps, eo, bo, sf_rows = Q.offsets_from_counts(counts, 0, K)
     lists = [torch.from_numpy(a).to("cuda") for a in (ps, eo, bo)]
     x = torch.randn((T, K), device="cuda", generator=torch.Generator(device="cuda").manual_seed(1)).to(torch.bfloat16)
+    whole = _quantise_on_gpu(x, counts, lists, sf_rows, quant, K)
+    parts = [torch.zeros((T, K), dtype=torch.uint8, device="cuda").view(torch.float8_e4m3fn),
+             torch.full((sf_rows, K // 32), 0xCD, dtype=torch.uint8, device="cuda")]
+    for e in range(len(counts)):
+        for first in range(0, counts[e], T // 8 // 128 * 128):       # whole scale atoms
+            rows = min(counts[e] - first, T // 8 // 128 * 128)
+            one = [torch.tensor(v, dtype=torch.int32, device="cuda")
+                   for v in ([[rows, 0, K]], [int(eo[e]) + first], [int(bo[e]) + first])]
+            quant(x, *one, *parts)
+    torch.cuda.synchronize()
     shifted = torch.empty(T * K + 8, dtype=x.dtype, device="cuda")[8:].view(T, K)
     shifted.copy_(x)
-    for a, b in zip(_quantise_on_gpu(x, counts, lists, sf_rows, quant, K),
-                    _quantise_on_gpu(shifted, counts, lists, sf_rows, quant, K)):
-        assert torch.equal(a, b)
+    again = _quantise_on_gpu(shifted, counts, lists, sf_rows, quant, K)
+    for a, b, c in zip(whole, parts, again):
+        assert torch.equal(a, b.view(torch.uint8)) and torch.equal(a, c)
 
 
 @pytest.mark.parametrize("shift", [0, 8])
