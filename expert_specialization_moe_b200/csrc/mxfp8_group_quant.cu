@@ -11,9 +11,8 @@
 // Schedule: an expert's rows are one contiguous stream of 128-element K tiles (rows are densely packed), whatever k is.
 // Eight lanes take a tile, sixteen elements each, a CTA 32 consecutive tiles per step.  The steps of all experts form one
 // flat list (a per-CTA prefix scan over the row counts) that the resident CTAs share evenly: neither the split of the rows
-// between experts nor k leaves lanes or CTAs idle.  (Work units of 16 steps of a warp dealt round-robin came to 6.05 units
-// per warp, so 7, at 32768 x 7168.)  Zeroing the scale bytes of the padding rows is steps of its own, in 16-byte pieces: in
-// a decode call they are as many bytes as the codes.
+// between experts nor k leaves lanes or CTAs idle.  Zeroing the scale bytes of the padding rows is steps of its own, in
+// 16-byte pieces: in a decode call they are as many bytes as the codes.
 //
 // What bounds it: HBM (3 + 1/32 bytes per element; with silu 5 + 1/32).  One lane per 8 elements and a warp per row
 // cost 10.5 instructions per element, enough to keep the issue slots 62 % busy; 16 elements per lane halve the scale
