@@ -78,8 +78,8 @@ WORKLOADS = {
                                                  "(n=4096, k=384, E=128), the benchmark's row distribution"),
     "ref_dist_ep16": (16, None, 4096, 7168, "MXFP8 grouped GEMM on the reference's SM100 benchmark: DeepSeek-R1 gate_up "
                                             "EP16 decode (n=4096, k=7168, E=16), the benchmark's row distribution"),
-    # weight-streaming probe: 128 experts of 1..32 rows, every tile streams a [128 x 7168] slab once; with
-    # --tunable mm_stream_max_ctas=<n> it gives the per-SM ingest rate of the streaming kernel at n CTAs
+    # weight-streaming probe: 128 experts of 1..32 rows, every work item streams a [256 x 7168] slab once; with
+    # --tunable mm_pair_max_clusters=<n> it gives the ingest rate of n CTA pairs
     "stream_probe": (128, None, 4096, 7168, "weight-streaming probe: E=128 experts of 1..32 rows (uniform), N=4096, K=7168"),
     "quant_small": (64, 8192, 0, 7168, "grouped MXFP8 quantisation at 1/4 scale for profiler captures: bf16 "
                                        "[8192, 7168], E=64"),
@@ -421,9 +421,9 @@ def bench_ep_layer(args, device, rank, world, dist):
                                        else "NCCL all-to-all dispatch/combine"),
                            "experts_per_gpu": e_local},
                 "clocks": clocks, "device_status": status,
-                # ours per step: route count + tables, dispatch-quant-push, unpack, 2 barriers, 3 + 3 GEMM launches,
-                # silu-quant, weighted sum (fused) / 2 quant kernels + GEMMs (all-to-all path)
-                "gpu_launches": args.steps * ((28 if args.workload == "qwen3_ep_pipelined" else 14) if fused else 9)}
+                # ours per step: route count + tables, dispatch-quant-push, unpack, 2 barriers, 1 + 1 GEMM launches,
+                # silu-quant, weighted sum (fused) / 2 quant kernels + 2 GEMMs (all-to-all path)
+                "gpu_launches": args.steps * ((20 if args.workload == "qwen3_ep_pipelined" else 10) if fused else 4)}
     del shard, x
     torch.cuda.empty_cache()
     return line
@@ -807,7 +807,7 @@ def main():
                          "replicated (see place_experts)")
     ap.add_argument("--tunable", action="append", default=[], metavar="NAME=VALUE",
                     help="set a dispatcher tunable of the library before the run (es_b200_set_tunable), e.g. "
-                         "mm_pair_first_clusters=0, mm_stream_max_ctas=64, mm_stream_lsu=0; repeatable")
+                         "mm_pair_max_clusters=32, mm_dynamic=0; repeatable")
     ap.add_argument("--ep-layer-steps", type=int, default=10,
                     help="N > 1, default workload: steps of the expert-parallel layer run after the headline (0 = skip)")
     args = ap.parse_args()
@@ -944,11 +944,7 @@ def main():
     elapsed_ms, e2e_ms = float(stats[0]), float(stats[1])
     flops_total, h2d_total, d2h_total = float(sums[0]), float(sums[1]), float(sums[2])
 
-    # one call launches the streaming kernel (both shapes in one launch), the CTA-pair kernel when the host-known row
-    # count can reach its bucket (>= 113 rows at most shapes), and a leading capped CTA-pair launch when the call is split
-    # (256 rows or more)
-    rows_local = int(counts.sum())
-    launches_per_step = 1 + (rows_local >= 113) + (rows_local >= 256)
+    launches_per_step = 1          # one kernel per call, whatever the row counts are
     line = None
     if rank == 0:
         ms_per_step = elapsed_ms / args.steps
@@ -965,10 +961,7 @@ def main():
             "config": config,
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                          "traffic": traffic, "peak_kind": peak_kind, "algorithmic_bytes": abytes,
-                         "kernel": ("mxfp8_grouped_mm_pair_kernel (capped) | mxfp8_grouped_mm_kernel (32- and 112-token "
-                                    "shapes in one launch) | mxfp8_grouped_mm_pair_kernel: one PDL chain per call, "
-                                    "buckets side by side"
-                                    if launches_per_step == 3 else "mxfp8_grouped_mm_kernel chain"),
+                         "kernel": "mxfp8_grouped_mm_pair_kernel (one launch per call)",
                          "kernel_ms": my_ms},
             "clocks": clocks, "gpu_launches": args.steps * launches_per_step, "host_us_per_call": host_us,
         }

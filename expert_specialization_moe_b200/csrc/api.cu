@@ -59,11 +59,8 @@ static int env_or(const char* name, int fallback) {
 
 Tunables& tunables() {
   static Tunables t = {
-      env_or("ES_B200_MM_HEAVY_MIN_ROWS", 0),      env_or("ES_B200_MM_TINY_MAX_ROWS", 0),
-      env_or("ES_B200_MM_PAIR_FIRST_CLUSTERS", 32), env_or("ES_B200_MM_SPLIT_MIN_ROWS", 256),
-      env_or("ES_B200_MM_STREAM_MAX_CTAS", 0),     env_or("ES_B200_MM_PAIR_MAX_CLUSTERS", 0),
-      env_or("ES_B200_MM_DYNAMIC", 1),             env_or("ES_B200_MM_STREAM_LSU", 1),
-      env_or("ES_B200_MM_ITEM_K_STEPS", kDefaultItemKSteps), env_or("ES_B200_MM_STREAM_MID_LEAD_CTAS", -1),
+      env_or("ES_B200_MM_HEAVY_MIN_ROWS", 0), env_or("ES_B200_MM_PAIR_MAX_CLUSTERS", 0), env_or("ES_B200_MM_DYNAMIC", 1),
+      env_or("ES_B200_MM_ITEM_K_STEPS", kDefaultItemKSteps),
   };
   return t;
 }

@@ -1,39 +1,35 @@
-// MXFP8 block-scaled grouped GEMM for sm_100a on CTA PAIRS, for experts with many token rows:
-// tcgen05.mma.cta_group::2 with M = 256 and a weight-stationary K step over up to 384 token rows.
+// The kernel of the MXFP8 block-scaled grouped GEMM for sm_100a: CTA pairs (tcgen05.mma.cta_group::2), persistent, one
+// launch per call for experts of any row count.
 //
-// Same mapping as the single-CTA kernel (weights on the MMA M axis, the expert's token rows on the runtime-sized
-// MMA N axis).  Two CTAs of a cluster share every work item: each CTA holds 128 of the 256 weight rows and HALF of
-// the token rows in its own shared memory, and the pair's tensor cores exchange the token halves (no multicast
-// load anywhere).  One work item covers up to 384 token rows as two sub-tiles of <=192 rows with one accumulator
-// each: every 16 KB weight stage that a CTA pulls through L2 feeds BOTH sub-tiles' MMAs.  Per CTA and K step that
-// is 16 KB of weights + 2 x 12 KB of tokens for 128 x 384 x 128 MACs — 2.4x fewer operand bytes per FLOP than
-// 128 x 128 single-CTA tiles, which is what bounds experts with many rows (the operand feed, not the tensor pipe).
-// Sub-tiles are 192 rows because two 192-column fp32 accumulators plus per-stage scale slots fit the 512 TMEM
-// columns, and the second sub-tile starts on a 64-row boundary of the 128-row scale atoms, which a TMEM column
-// offset addresses.
+// Mapping: weights on the MMA M axis, the expert's token rows on the runtime-sized N axis (a multiple of 16: 3 rows cost an
+// N = 16 MMA, no padding of the ragged dimension to 128).  Two CTAs of a cluster share every work item: 256 weight rows —
+// each CTA holds 128 — times up to 384 token rows, half of them in each CTA's shared memory; the pair's tensor cores exchange
+// the halves (no multicast load anywhere).  More than 192 token rows are two sub-tiles with an accumulator each, so that
+// every 16 KB weight tile that a CTA pulls through L2 feeds both; up to 192 rows are one sub-tile and the two accumulators
+// take turns.  An expert's rows are divided into token tiles of whole 128-row scale atoms, as evenly as they go.
 //
-//   warp 0    producer (both CTAs): per K step lanes 0..4 each issue one TMA load (own weight rows, own halves of
-//             the two token sub-tiles, own weight scale atom, the item's token scale atoms); all completion bytes
-//             are credited to the leader CTA's barrier
-//   warp 1    TMEM allocation (both CTAs); in the leader CTA one lane issues sub-tile 0's four tcgen05.mma per K step
-//   warps 2-17  epilogue (both CTAs): own 128 accumulator lanes -> registers (bf16/fp16) -> accumulators handed back
-//               -> global; four warps per TMEM lane quadrant share the 32-column chunks of both accumulators
-//   warp 18     leader CTA, one lane: sub-tile 1's four tcgen05.mma per K step
-//   warp 19     leader CTA, one lane: the K step's four tcgen05.cp (scales smem -> TMEM of both CTAs)
+// What bounds it.  Experts of few rows stream their weights from HBM once: 1.69 GB in 239 us = 7.1 TB/s (256 experts, 512
+// rows, n = 7168, k = 2048).  Experts of many rows: the tensor pipe (a K step of 384 rows is 768 cycles of it, 782 measured),
+// then the power cap.  In between (about 256 rows): the K steps of token rows in flight (128 experts x 256 rows, n = 1536,
+// k = 2048: 158 us with 2 K steps, 124 with 3, 117 with 4).
 //
-// Work items come from the bucket's work counter in the caller's scratch (atomicAdd by lane 0 of the leader's producer
-// warp; round-robin over the clusters without scratch).  The index travels to every other role of BOTH CTAs through a
-// four-deep queue: the leader writes it into its own and its partner's shared memory and arrives on both CTAs'
-// q_full barriers; every consuming role arrives on the leader's q_empty barrier.  Two launches of this kernel may
-// serve one call (a small one in front of the streaming kernels, a full-width one behind them): they drain the same
-// counter.
+// What it took, measured cycle by cycle on its predecessor (three launches per call, 72 to 105 us more for the layer's two
+// GEMMs):
+//   * tcgen05 and TMA instructions are issued by a thread that elect.sync picked.  Guarded by lane == 0 the same code
+//     needs 137 cycles per MMA and 550 per K step; elected, MMAs go out at the pipe's rate (40 cycles at N = 16);
+//   * one barrier wait (130 cycles) and one commit (90) per K step: what a K step cannot have is several of them in a row;
+//   * arrivals at the partner CTA that publish no memory are relaxed: a releasing one first waits for the epilogue's
+//     stores, 2000 to 3000 cycles before every hand-back of an accumulator;
+//   * work items are decoded once, by a warp that does nothing else, and queued four deep (every role decoded for
+//     itself: 2000 cycles per item);
+//   * the output leaves as 16-byte stores: matrix fragments from TMEM (16x256b), transposed by stmatrix.
 //
-// Three issuing lanes instead of one because a tcgen05 instruction costs the thread that issues it ~90 cycles (mma)
-// or ~65 cycles (cp) whatever its size (measured: the K step of a single issuing lane took the same ~1000 cycles with
-// N = 64 and with N = 256 MMAs), while the tensor pipe needs 96 cycles for a 256 x 192 x 32 MMA.  One lane issuing
-// 8 MMAs + 4 copies + a commit per K step is therefore issue-bound at ~1260 cycles for 768 cycles of tensor work;
-// split three ways every lane stays below the pipe's time.  The lanes meet only through mbarriers: the copy lane
-// commits to sf_ready[stage], both MMA lanes commit to empty[stage] (2 arrivals) and to their accumulator's barrier.
+//   warp 0      producer of weights and scales (both CTAs): per K step one thread loads its 128 weight rows, their scale atom
+//               and the item's token scale atoms; all bytes are credited to the leader CTA's barrier
+//   warp 1      TMEM allocation; in the leader CTA one thread issues the K step's scale copies (tcgen05.cp) and MMAs
+//   warp 2      scheduler (leader): takes item indices from the work counter and queues the items in both CTAs
+//   warp 3      producer of token rows (both CTAs): this CTA's half of each sub-tile
+//   warps 4-15  epilogue (both CTAs)
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
@@ -42,102 +38,95 @@
 #include "grouped_mm_call.cuh"
 #include "sm100_ptx.cuh"
 #include "tensormap.cuh"
+#include "work_items.cuh"
 
 namespace es_b200 {
-namespace mm2 {
+namespace mm {
 
-constexpr int THREADS = 640;
+constexpr int THREADS = 512;
 constexpr int TILE_N = 128;      // weight rows per CTA (the pair covers 256)
 constexpr int TILE_K = 128;
 constexpr int SUB_TILE = 192;    // token rows per accumulator (MMA N, runtime multiple of 16)
-constexpr int TOK_TILE = 2 * SUB_TILE;   // token rows per work item
-constexpr int STAGES = 5;
+constexpr int ITEM_ATOMS = 3;    // 128-row scale atoms per work item: up to 384 token rows
 constexpr int W_BYTES = TILE_N * TILE_K;               // 16384
-constexpr int X_BYTES = (SUB_TILE / 2) * TILE_K;       // 12288: this CTA's half of one token sub-tile
-constexpr int SFW_BYTES = 512;
-constexpr int SFX_BYTES = 1536;                        // three 512-byte atoms cover 384 rows
-constexpr int STAGE_BYTES = 43008;                     // 42 KB: W | X0 | X1 | SFW | SFX  (multiple of 1024)
-static_assert(W_BYTES + 2 * X_BYTES + SFW_BYTES + SFX_BYTES <= STAGE_BYTES, "stage layout");
+constexpr int SF_BYTES = 512;
+constexpr int SFX_BYTES = ITEM_ATOMS * SF_BYTES;
+constexpr int W_SLOT = W_BYTES + SF_BYTES + SFX_BYTES; // 18432: W | SFW | SFX
+constexpr int X_SLOT = (SUB_TILE / 2) * TILE_K;        // 12288: this CTA's half of one token sub-tile
+static_assert(W_SLOT % 1024 == 0 && X_SLOT % 1024 == 0, "128-byte swizzle atoms are 1024 bytes");
+// The two rings share what shared memory there is: W weight slots (one per K step), X token slots (one per sub-tile of a K
+// step).  Few rows per expert: seven K steps in flight.  Many: eight token slots are four K steps of two sub-tiles.
+struct FewRows { static constexpr int W = 7, X = 7; };
+struct ManyRows { static constexpr int W = 6, X = 8; };
 constexpr uint32_t TMEM_COLS = 512;
 constexpr uint32_t ACC_COLS = 192;        // accumulators at columns [0,192) and [192,384)
-constexpr uint32_t SF_COL0 = 384;         // per-stage scale slots of 16 columns: 4 (weights) + 12 (tokens)
+constexpr uint32_t SF_COL0 = 384;         // per weight slot 16 columns: 4 (weight scales) + 12 (token scales)
 constexpr uint32_t SF_SLOT_COLS = 16;
-static_assert(SF_COL0 + STAGES * SF_SLOT_COLS <= TMEM_COLS, "TMEM budget");
+static_assert(SF_COL0 + FewRows::W * SF_SLOT_COLS <= TMEM_COLS && ManyRows::W <= FewRows::W, "TMEM budget");
 
-constexpr uint32_t ERR_PRODUCER = 0x10u, ERR_MMA = 0x20u, ERR_EPILOGUE = 0x40u;
-constexpr uint32_t ERR_SCALE_COPY = 0x100u;
-constexpr int EPI_WARPS = 16;                              // 4 TMEM lane quadrants x 4 warps
-constexpr int EPI_BYTES_PER_WARP = 8 * 32 * 2;             // 512 bytes: 8 tokens x 32 n (scattered output only)
-constexpr int MMA_B_WARP = 2 + EPI_WARPS;                  // 18
-constexpr int COPY_WARP = MMA_B_WARP + 1;                  // 19
+constexpr int MAX_W = 7, MAX_X = 8;
+constexpr uint32_t ERR_PRODUCER = 0x10u, ERR_MMA = 0x20u, ERR_EPILOGUE = 0x40u, ERR_SCHEDULER = 0x100u;
+constexpr int W_WARP = 0, MMA_WARP = 1, SCHED_WARP = 2, X_WARP = 3, EPI_WARP0 = 4;
+constexpr int EPI_WARPS = 12;                              // 4 TMEM lane quadrants x 3 warps
+constexpr int EPI_BYTES_PER_WARP = 8 * 32 * 2;             // 8 tokens x 32 n
 constexpr int QUEUE_DEPTH = 4;
-// readers of a queue slot: in the leader CTA the two MMA lanes, the copy lane and 16 epilogue warps; in the partner CTA
-// the producer warp and 16 epilogue warps
-constexpr int Q_CONSUMERS = (3 + EPI_WARPS) + (1 + EPI_WARPS);
+// readers of a queue entry: both producers and the epilogue warps of each CTA, the MMA warp of the leader
+constexpr int Q_CONSUMERS = 2 * (2 + EPI_WARPS) + 1;
+
+struct Item {      // one work item as the scheduler hands it out
+  int valid;       // token rows of the item (<= 384); -1: no more work
+  int row0;        // first token row in a / d
+  int n01;         // MMA N of the two sub-tiles, n0 | n1 << 16 (multiples of 16; n1 == 0: one sub-tile)
+  int np0;         // first weight pair
+  int units;       // weight pairs of the item
+  int e;           // expert
+  int sfx_row;     // first 128-row block of the token scales
+  int one_tile;    // 1: the expert has one token tile (its weights are read once)
+};
+static_assert(sizeof(Item) == 32, "two 16-byte words");
 
 struct SharedCtl {
-  uint64_t full[STAGES];        // used in the leader CTA only
-  uint64_t empty[STAGES];       // 2 arrivals: one commit from each MMA lane
-  uint64_t sf_ready[STAGES];    // leader only: the stage's scales are in the TMEM of both CTAs
-  uint64_t tmem_full[2];
-  uint64_t tmem_empty[2];       // used in the leader CTA only (32 arrivals: 16 epilogue warps x 2 CTAs)
-                                // index = accumulator (sub-tile 0 / 1)
-  uint64_t q_full[QUEUE_DEPTH];   // 1 arrival from the leader's producer lane (in the partner CTA also the 8 bytes of
-                                  // the entry, sent with the arrival): q_item[slot] is written
-  uint64_t q_empty[QUEUE_DEPTH];  // leader only: Q_CONSUMERS arrivals, every consuming role of both CTAs has read it
-  int2 q_item[QUEUE_DEPTH];       // x: work item index, or -1: no more work; y: the item's expert (found once, by
-                                  // the leader's producer lane)
-  uint32_t tmem_base;
+  uint64_t full[MAX_W];           // leader only: both producers' arrivals and all bytes of a K step
+  uint64_t empty[MAX_W];          // the step's MMAs have completed: its weight slot and its token slots are free
+  uint64_t acc_full[2];
+  uint64_t acc_empty[2];          // leader only: one arrival per epilogue warp of both CTAs
+  uint64_t q_full[QUEUE_DEPTH];
+  uint64_t q_empty[QUEUE_DEPTH];  // leader only
+  alignas(16) Item q_item[QUEUE_DEPTH];
+  int x_user[MAX_X];              // token producer: the K step that used the slot last
+  alignas(16) uint32_t tmem_base;
   int abort_flag;
-  int warp_sums[32];
-  // [0, E]: exclusive prefix of the experts' item counts; behind it the per-expert tables (fill_expert_table)
-  int table[ES_B200_MAX_EXPERTS + 1];
+  int warp_heavy[32], warp_light[32];
+  int prefix_heavy[ES_B200_MAX_EXPERTS + 1];   // exclusive prefix of the experts' work items
+  int prefix_light[ES_B200_MAX_EXPERTS + 1];
 };
 
-constexpr size_t SMEM_BYTES = 1024 + (size_t)STAGES * STAGE_BYTES + EPI_WARPS * EPI_BYTES_PER_WARP + sizeof(SharedCtl);
-static_assert(SMEM_BYTES <= 232448, "shared memory of one CTA per SM");
+template <class S>
+constexpr size_t smem_bytes() {
+  return 1024 + (size_t)S::W * W_SLOT + (size_t)S::X * X_SLOT + EPI_WARPS * EPI_BYTES_PER_WARP + sizeof(SharedCtl);
+}
+static_assert(smem_bytes<FewRows>() <= 232448 && smem_bytes<ManyRows>() <= 232448, "shared memory of one CTA per SM");
 
 __device__ uint32_t g_status = 0;
 
-struct TileInfo {
-  int e, tt, np;
-  int valid;       // token rows of this item that belong to the expert (<= 384)
-  int n0, n1;      // MMA N of the two sub-tiles (multiples of 16; n1 == 0 when the item has <= 192 rows)
-  int v0, v1;      // valid rows of the two sub-tiles
-  int row0;        // first token row of the item in a / d
-  int atom0;       // first 128-row scale atom of the item inside the expert (items start on atom boundaries)
-  int n_atoms;     // 1..3 atoms cover the item's valid rows
+struct Maps {
+  CUtensorMap w;        // weights  [E*N, K] bytes, box 128 rows x 128 B, 128-byte swizzle
+  CUtensorMap x[5];     // tokens   [T, K]   bytes, boxes of 8 / 16 / 32 / 64 / 96 rows
+  CUtensorMap sfw;      // weight scale atoms, 512-byte records
+  CUtensorMap sfx1;     // token scale atoms as [128-row block][K block] of 512-byte records; box = 1 row block
+  CUtensorMap sfx3;     // the same, box = 3 row blocks
 };
 
-__device__ __forceinline__ TileInfo decode_tile(int t, int e, const ExpertTable& tab, int n, int n_pairs) {
-  TileInfo ti;
-  ti.e = e;
-  const int i = t - tab.prefix[e];
-  const int m = tab.m(e);
-  const int token_tiles = (m + TOK_TILE - 1) / TOK_TILE;
-  // Consecutive items run at the same time on different CTA pairs and share one operand in L2 while they sweep the
-  // other: the swept operand should be the SMALLER one.  Token tile fastest (items share a weight slab and sweep the
-  // expert's m x k tokens) unless the expert has more token rows than weight rows; then weight pair fastest (items
-  // share a token tile and sweep the n x k weights).
-  if (m <= n) {
-    ti.np = i / token_tiles;
-    ti.tt = i - ti.np * token_tiles;
-  } else {
-    ti.tt = i / n_pairs;
-    ti.np = i - ti.tt * n_pairs;
-  }
-  const int r_local = ti.tt * TOK_TILE;
-  const int rem = m - r_local;
-  ti.valid = rem < TOK_TILE ? rem : TOK_TILE;
-  ti.v0 = ti.valid < SUB_TILE ? ti.valid : SUB_TILE;
-  ti.v1 = ti.valid - ti.v0;
-  ti.n0 = (ti.v0 + 15) & ~15;
-  ti.n1 = (ti.v1 + 15) & ~15;
-  ti.row0 = tab.row0(e) + r_local;
-  ti.atom0 = r_local >> 7;
-  ti.n_atoms = (ti.valid + 127) >> 7;
-  return ti;
-}
+struct KernelArgs {
+  void* d;
+  const int* problem_sizes;
+  const int* expert_offsets;
+  const int* blockscale_offsets;
+  int num_experts, n, k;
+  int heavy_min;             // experts with at least this many rows come first in the work list
+  int group_heavy, group_light;   // weight pairs per work item
+  uint32_t* counters;
+};
 
 __device__ __forceinline__ int box_index(int half_rows) {   // token tensor maps: boxes of 8 / 16 / 32 / 64 / 96 rows
   return half_rows <= 8 ? 0 : half_rows <= 16 ? 1 : half_rows <= 32 ? 2 : half_rows <= 64 ? 3 : 4;
@@ -146,40 +135,99 @@ __device__ __forceinline__ uint32_t box_rows_of(int idx) {
   return idx == 0 ? 8u : idx == 1 ? 16u : idx == 2 ? 32u : idx == 3 ? 64u : 96u;
 }
 
-struct Maps {
-  CUtensorMap w;        // weights  [E*N, K] bytes, box 128 rows x 128 B, 128-byte swizzle
-  CUtensorMap x[5];     // tokens   [T, K]   bytes, boxes of 8 / 16 / 32 / 64 / 96 rows
-  CUtensorMap sfw;      // weight scale atoms, 512-byte records
-  CUtensorMap sfx;      // token scale atoms as [128-row block][K block] of 512-byte records; box = 3 row blocks
-};
+// largest e in [0, n) with prefix[e] <= u, found by a converged warp (prefix non-decreasing, prefix[0] = 0 <= u < prefix[n])
+__device__ __forceinline__ int warp_find_expert(const int* prefix, int n, int u, int lane) {
+  const int stride = (n + 31) >> 5;
+  const int i = lane * stride;
+  const uint32_t above = __ballot_sync(0xffffffffu, i < n && prefix[i] <= u);
+  const int lo = (31 - __clz((int)above)) * stride;
+  const int j = lo + lane;
+  const uint32_t in = __ballot_sync(0xffffffffu, lane < stride && j < n && prefix[j] <= u);
+  return lo + 31 - __clz((int)in);
+}
 
-template <typename OutT, bool HOLD>
+// 8 tokens per pass through the warp's shared-memory tile: held[4 g + b] is the 8x8 fragment (n 8b .. 8b+7, tokens
+// 8g .. 8g+7) of a 32-token chunk; stored transposed, read back as 16-byte pieces of a token row, stored as 128-bit words,
+// four lanes per 64-byte segment.  `tok`: first token of the chunk within the item.
+template <typename OutT>
+__device__ __forceinline__ void store_chunk_16B(const uint32_t (&held)[16], uint32_t stage, int tok, int valid, OutT* out,
+                                                int64_t ld, int lane, bool scattered, OutT* dest_row) {
+  const uint32_t wr = stage + (lane & 7) * 64 + (((lane >> 3) ^ ((lane & 7) >> 1)) << 4);
+  const uint32_t rd = stage + (lane >> 2) * 64 + (((lane & 3) ^ ((lane >> 3) & 3)) << 4);
+#pragma unroll
+  for (int g = 0; g < 4; ++g) {
+    if (tok + g * 8 >= valid) break;       // warp-uniform
+    ptx::stmatrix_x4_trans(wr, held[g * 4], held[g * 4 + 1], held[g * 4 + 2], held[g * 4 + 3]);
+    __syncwarp();
+    const int t = g * 8 + (lane >> 2);
+    const uint4 val = ptx::ld_shared_16B(rd);
+    if (!scattered) {
+      if (tok + t < valid) *reinterpret_cast<uint4*>(out + (int64_t)(tok + t) * ld + (lane & 3) * 8) = val;
+    } else {
+      OutT* row = reinterpret_cast<OutT*>(__shfl_sync(0xffffffffu, reinterpret_cast<unsigned long long>(dest_row), t));
+      if (row != nullptr) *reinterpret_cast<uint4*>(row + (lane & 3) * 8) = val;
+    }
+    __syncwarp();
+  }
+}
+
+// 32-column chunks of the warp's 32 accumulator lanes as 16-bit 8x8 fragments (see store_chunk_16B): one chunk, or two with
+// all four reads in flight
+template <typename OutT>
+__device__ __forceinline__ void pack_chunk(const uint32_t (&lo)[16], const uint32_t (&hi)[16], uint32_t (&held)[16]) {
+#pragma unroll
+  for (int g = 0; g < 4; ++g) {
+    held[4 * g + 0] = pack_pair_from_f32<OutT>(__uint_as_float(lo[4 * g]), __uint_as_float(lo[4 * g + 1]));
+    held[4 * g + 1] = pack_pair_from_f32<OutT>(__uint_as_float(lo[4 * g + 2]), __uint_as_float(lo[4 * g + 3]));
+    held[4 * g + 2] = pack_pair_from_f32<OutT>(__uint_as_float(hi[4 * g]), __uint_as_float(hi[4 * g + 1]));
+    held[4 * g + 3] = pack_pair_from_f32<OutT>(__uint_as_float(hi[4 * g + 2]), __uint_as_float(hi[4 * g + 3]));
+  }
+}
+template <typename OutT>
+__device__ __forceinline__ void read_chunk(uint32_t taddr, uint32_t (&held)[16]) {
+  uint32_t lo[16], hi[16];
+  ptx::tc_ld_16x256b_x4(taddr, lo);
+  ptx::tc_ld_16x256b_x4(taddr + (16u << 16), hi);
+  ptx::tc_wait_ld();
+  pack_chunk<OutT>(lo, hi, held);
+}
+template <typename OutT>
+__device__ __forceinline__ void read_two_chunks(uint32_t taddr0, uint32_t taddr1, uint32_t (&held0)[16], uint32_t (&held1)[16]) {
+  uint32_t lo0[16], hi0[16], lo1[16], hi1[16];
+  ptx::tc_ld_16x256b_x4(taddr0, lo0);
+  ptx::tc_ld_16x256b_x4(taddr0 + (16u << 16), hi0);
+  ptx::tc_ld_16x256b_x4(taddr1, lo1);
+  ptx::tc_ld_16x256b_x4(taddr1 + (16u << 16), hi1);
+  ptx::tc_wait_ld();
+  pack_chunk<OutT>(lo0, hi0, held0);
+  pack_chunk<OutT>(lo1, hi1, held1);
+}
+
+template <typename OutT, class S>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
-mxfp8_grouped_mm_pair_kernel(const __grid_constant__ Maps maps, OutT* __restrict__ d,
-                             const int* problem_sizes, const int* expert_offsets,
-                             const int* blockscale_offsets, int num_experts, int n, int k, int min_rows,
-                             int wait_at_start, const __grid_constant__ RowScatter scatter, uint32_t* counters,
-                             int last_of_call, uint32_t earlier_ctas) {
-  if (!wait_at_start) pdl_launch_dependents();   // not the first kernel of its call: the next one may launch at once
+mxfp8_grouped_mm_pair_kernel(const __grid_constant__ Maps maps, const __grid_constant__ KernelArgs args,
+                             const __grid_constant__ RowScatter scatter) {
+  constexpr int W_STAGES = S::W, X_STAGES = S::X;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = ptx::align1024(smem_raw);
-  uint8_t* epi_stage = smem + (size_t)STAGES * STAGE_BYTES;      // 16 x 512 bytes, one per epilogue warp
+  uint8_t* x_ring = smem + (size_t)W_STAGES * W_SLOT;
+  uint8_t* epi_stage = x_ring + (size_t)X_STAGES * X_SLOT;
   SharedCtl* ctl = reinterpret_cast<SharedCtl*>(epi_stage + EPI_WARPS * EPI_BYTES_PER_WARP);
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
-  const uint32_t rank = ptx::cluster_ctarank();      // 0 = leader (issues the MMAs), 1 = peer
+  const uint32_t rank = ptx::cluster_ctarank();      // 0 = leader (schedules, issues the MMAs), 1 = peer
   const int pair = blockIdx.x >> 1;
   const int num_pairs = gridDim.x >> 1;
+  const int num_experts = args.num_experts, n = args.n, k = args.k;
 
-  if (threadIdx.x == 0) {
-    for (int s = 0; s < STAGES; ++s) {
-      ptx::mbar_init(&ctl->full[s], 1);
-      ptx::mbar_init(&ctl->empty[s], 2);
-      ptx::mbar_init(&ctl->sf_ready[s], 1);
+  if (threadIdx.x == SCHED_WARP * 32) {
+    for (int s = 0; s < W_STAGES; ++s) {
+      ptx::mbar_init(&ctl->full[s], 2);
+      ptx::mbar_init(&ctl->empty[s], 1);
     }
     for (int a = 0; a < 2; ++a) {
-      ptx::mbar_init(&ctl->tmem_full[a], 1);
-      ptx::mbar_init(&ctl->tmem_empty[a], 2 * EPI_WARPS);
+      ptx::mbar_init(&ctl->acc_full[a], 1);
+      ptx::mbar_init(&ctl->acc_empty[a], 2 * EPI_WARPS);
     }
     for (int q = 0; q < QUEUE_DEPTH; ++q) {
       ptx::mbar_init(&ctl->q_full[q], 1);
@@ -187,371 +235,454 @@ mxfp8_grouped_mm_pair_kernel(const __grid_constant__ Maps maps, OutT* __restrict
     }
     ctl->abort_flag = 0;
     ptx::fence_mbar_init();
-    ptx::prefetch_tensormap(&maps.w);
-    ptx::prefetch_tensormap(&maps.sfw);
-    ptx::prefetch_tensormap(&maps.sfx);
-#pragma unroll
-    for (int i = 0; i < 5; ++i) ptx::prefetch_tensormap(&maps.x[i]);
   }
-  // This kernel is chained with the single-CTA kernels of the same call by programmatic dependent launch — behind
-  // them, and for a large call also in front of them with a capped grid.  The first kernel of the call waits for
-  // everything before it (griddepcontrol.wait) before it lets the others start, so the operands are final; the
-  // kernels write disjoint rows of d.  A launch that is not first therefore starts on SMs as they become free; stream
-  // order for whatever follows the call is kept at the end (end_of_kernel).
-  // (a launch that is not first has let the next kernel of the call launch at entry; the first one does so after its
-  // prologue, below)
-  if (wait_at_start) pdl_wait_prior_grid();
-  const int n_tiles = n / TILE_N;
-  const int n_pairs = (n_tiles + 1) >> 1;
-  // only experts with at least min_rows rows belong to this kernel (the single-CTA kernel takes the others)
-  // (an expert whose scales do not start on a 128-row atom cannot be addressed: reported and skipped)
-  block_exclusive_scan(num_experts, ctl->table, ctl->warp_sums, [&](int e) {
-    const int m = problem_sizes[e * 3];
-    if (!(m > 0 && m >= min_rows)) return 0;
-    if ((blockscale_offsets[e] & 127) != 0) {
-      atomicOr(&g_status, ERR_SCALE_OFFSET_BIT);
-      return 0;
-    }
-    return ((m + TOK_TILE - 1) / TOK_TILE) * n_pairs;
-  });
-  // A launch without work (the host only knows an upper bound of the rows per expert) ends here, before it holds
-  // TMEM or has signalled its partner CTA; both CTAs of a pair see the same total.
-  if (ctl->table[num_experts] == 0) {
-    if (wait_at_start) pdl_launch_dependents();
-    end_of_kernel(counters, wait_at_start != 0, last_of_call != 0, earlier_ctas, scatter.meta != nullptr, &g_status);
-    return;
-  }
-  if (warp == 1) {
+  if (warp == MMA_WARP) {
     ptx::tmem_alloc_pair(&ctl->tmem_base, TMEM_COLS);
     ptx::tmem_relinquish_pair();
   }
-  const ExpertTable tab = fill_expert_table(ctl->table, num_experts, problem_sizes, expert_offsets, blockscale_offsets);
-  // barriers, TMEM and tables of both CTAs must exist before either CTA signals the other
+  if (warp == W_WARP && lane < 9) {
+    const CUtensorMap* m = lane == 0 ? &maps.w : lane < 6 ? &maps.x[lane - 1] : lane == 6 ? &maps.sfw : lane == 7 ? &maps.sfx1 : &maps.sfx3;
+    ptx::prefetch_tensormap(m);
+  }
+  // (the wait for the partner's barriers is in the middle of the prologue: cluster_wait below)
+  __syncthreads();
+  ptx::cluster_arrive();
+  pdl_wait_prior_grid();
+  const int n_tiles = n / TILE_N;
+  const int n_pairs = (n_tiles + 1) >> 1;
+  const int kt_count = k / TILE_K;
+  // rows, first row and first scale row of every expert, for the scheduler's first look-up: in the ring, which no load uses
+  // before that
+  int* const facts = reinterpret_cast<int*>(smem);
+  if (rank == 0) {
+    // exclusive prefixes of the experts' work items, heavy and light experts apart (an expert whose scales do not start
+    // on a 128-row atom cannot be addressed: reported and skipped)
+    const int per = (num_experts + THREADS - 1) / THREADS;      // 1 or 2 consecutive experts per thread
+    const int heavy_groups = (n_pairs + args.group_heavy - 1) / args.group_heavy;
+    const int light_groups = (n_pairs + args.group_light - 1) / args.group_light;
+    int h[2] = {0, 0}, l[2] = {0, 0};
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const int e = (int)threadIdx.x * per + i;
+      if (i < per && e < num_experts) {
+        const int m = args.problem_sizes[e * 3];
+        const int bs = args.blockscale_offsets[e];
+        facts[e] = m;
+        facts[ES_B200_MAX_EXPERTS + e] = args.expert_offsets[e];
+        facts[2 * ES_B200_MAX_EXPERTS + e] = bs;
+        if (m > 0) {
+          if ((bs & 127) != 0) atomicOr(&g_status, ERR_SCALE_OFFSET_BIT);
+          else if (m >= args.heavy_min) h[i] = (int)(((int64_t)m + 128 * ITEM_ATOMS - 1) / (128 * ITEM_ATOMS)) * heavy_groups;
+          else l[i] = (int)(((int64_t)m + 128 * ITEM_ATOMS - 1) / (128 * ITEM_ATOMS)) * light_groups;
+        }
+      }
+    }
+    int hs = h[0] + h[1], ls = l[0] + l[1];
+#pragma unroll
+    for (int dlt = 1; dlt < 32; dlt <<= 1) {
+      const int a = __shfl_up_sync(0xffffffffu, hs, dlt), b = __shfl_up_sync(0xffffffffu, ls, dlt);
+      if (lane >= dlt) { hs += a; ls += b; }
+    }
+    if (lane == 31) { ctl->warp_heavy[warp] = hs; ctl->warp_light[warp] = ls; }
+    __syncthreads();
+    int hb = 0, lb = 0;
+    for (int w = 0; w < warp; ++w) { hb += ctl->warp_heavy[w]; lb += ctl->warp_light[w]; }
+    hb += hs - h[0] - h[1];
+    lb += ls - l[0] - l[1];
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const int e = (int)threadIdx.x * per + i;
+      if (i < per && e < num_experts) {
+        ctl->prefix_heavy[e] = hb;
+        ctl->prefix_light[e] = lb;
+        hb += h[i];
+        lb += l[i];
+      }
+    }
+    if (threadIdx.x == THREADS - 1) { ctl->prefix_heavy[num_experts] = hb; ctl->prefix_light[num_experts] = lb; }
+  }
+  // barriers, TMEM and prefixes must exist before either CTA signals the other
   ptx::tc_fence_before_sync();
-  ptx::cluster_sync();
+  __syncthreads();
+  ptx::cluster_wait();
   ptx::tc_fence_after_sync();
-  if (wait_at_start) pdl_launch_dependents();
+  pdl_launch_dependents();
 
   const uint32_t tmem_base = ctl->tmem_base;
-  const int total_tiles = tab.prefix[num_experts];
-  const int kt_count = k / TILE_K;
-  const int sfw_atoms_per_expert = n_tiles * kt_count;
   volatile int* abort_flag = &ctl->abort_flag;
+  int qs = 0;
+  uint32_t qph = 0;
+  // the next work item, read by a whole warp; false: a wait gave up
+  auto next_item_one = [&](Item* it) {
+    const bool have = rank == 0 ? ptx::mbar_wait(&ctl->q_full[qs], qph, abort_flag)
+                                : ptx::mbar_wait_cluster(&ctl->q_full[qs], qph, abort_flag);
+    if (!have) return false;
+    const int4* src = reinterpret_cast<const int4*>(&ctl->q_item[qs]);
+    *reinterpret_cast<int4*>(it) = src[0];
+    *(reinterpret_cast<int4*>(it) + 1) = src[1];
+    ptx::mbar_arrive_cluster_relaxed(&ctl->q_empty[qs], 0);
+    if (++qs == QUEUE_DEPTH) { qs = 0; qph ^= 1u; }
+    return true;
+  };
+  auto next_item = [&](Item* it) {
+    const bool have = rank == 0 ? ptx::mbar_wait(&ctl->q_full[qs], qph, abort_flag)
+                                : ptx::mbar_wait_cluster(&ctl->q_full[qs], qph, abort_flag);
+    if (!__all_sync(0xffffffffu, have)) return false;
+    const int4* src = reinterpret_cast<const int4*>(&ctl->q_item[qs]);
+    *reinterpret_cast<int4*>(it) = src[0];
+    *(reinterpret_cast<int4*>(it) + 1) = src[1];
+    __syncwarp();
+    if (lane == 0) ptx::mbar_arrive_cluster_relaxed(&ctl->q_empty[qs], 0);
+    if (++qs == QUEUE_DEPTH) { qs = 0; qph ^= 1u; }
+    return true;
+  };
+  auto give_up = [&](uint32_t bit) {
+    *abort_flag = 1;
+    atomicOr(&g_status, bit);
+  };
 
-  if (warp == 0) {
-    // ------------------------------------------------------------------ producer (warp 0 of each CTA)
-    // The whole warp walks the work list; per K step lanes 0..4 each issue ONE of the stage's loads in the same
-    // instruction (a TMA issue costs the issuing thread ~80 cycles, five in a row would be a third of a stage time).
-    int s = 0, qs = 0;
-    uint32_t ph = 0, qph = 0;
-    uint32_t* counter = counters ? counters + 2 : nullptr;
-    int t_mine = 0;                   // leader, lane 0: the index that goes out next
-    if (rank == 0 && lane == 0) t_mine = counter ? (int)atomicAdd(counter, 1u) : pair;
-    while (true) {
-      // the leader publishes the next item (or the end mark) to both CTAs; the partner's producer reads its copy
-      int t = -1, e = 0;
-      bool q_ok = true;
-      if (rank == 0) {
-        if (lane == 0) {
-          q_ok = ptx::mbar_wait(&ctl->q_empty[qs], qph ^ 1u, abort_flag);
-          if (q_ok) {
-            t = t_mine < total_tiles ? t_mine : -1;
-            e = t >= 0 ? upper_bound_expert(tab.prefix, num_experts, t) : 0;
-            ctl->q_item[qs] = make_int2(t, e);
-            ptx::mbar_arrive(&ctl->q_full[qs]);
-            ptx::send_u64_to_cluster_cta(&ctl->q_item[qs], &ctl->q_full[qs], 1, (uint32_t)t, (uint32_t)e);
-            // the following index is requested now; its round trip to L2 hides behind this item's loads
-            if (t >= 0) t_mine = counter ? (int)atomicAdd(counter, 1u) : t_mine + num_pairs;
+  if (warp == SCHED_WARP) {
+    // ------------------------------------------------------------------ scheduler (leader): work item index -> item
+    if (rank == 0) {
+      const int total_heavy = ctl->prefix_heavy[num_experts], total = total_heavy + ctl->prefix_light[num_experts];
+      // the first item of a pair is its own index, the counter deals the items from num_pairs on
+      int t_next = pair;               // lane 0: the index that goes out next
+      // The heavy items are dealt out evenly over the first 95 % of the list: next to one another they are bound by the
+      // tensor pipe and the others by HBM (32768 Zipf rows, 256 experts, n = 4096, k = 7168: 1604 us with the heavy ones
+      // first, 1521 so).  A long item must not be the last one.
+      const bool mixed = total_heavy > 0 && total_heavy < total;
+      const int64_t span = max((int64_t)total_heavy, (int64_t)total * 95 / 100);
+      auto heavy_before = [&](int t) { return (int)min((int64_t)total_heavy, ((int64_t)t * total_heavy + span - 1) / span); };
+      while (true) {
+        const int t = __shfl_sync(0xffffffffu, t_next, 0);
+        Item it = {-1, 0, 0, 0, 0, 0, 0, 0};
+        if (t < total) {
+          // the following index is requested now; its round trip to L2 hides behind this item
+          if (lane == 0) t_next = args.counters ? num_pairs + (int)atomicAdd(args.counters, 1u) : t + num_pairs;
+          bool heavy = total_heavy > 0;
+          int u = t;
+          if (mixed) {
+            const int hb = heavy_before(t);
+            heavy = heavy_before(t + 1) > hb;
+            u = heavy ? hb : t - hb;
           }
+          const int* prefix = heavy ? ctl->prefix_heavy : ctl->prefix_light;
+          const int group = heavy ? args.group_heavy : args.group_light;
+          const int e = warp_find_expert(prefix, num_experts, u, lane);
+          const int i = u - prefix[e];
+          const int m = t == pair ? facts[e] : args.problem_sizes[e * 3];
+          const int row_first = t == pair ? facts[ES_B200_MAX_EXPERTS + e] : args.expert_offsets[e];
+          const int sf_first = (t == pair ? facts[2 * ES_B200_MAX_EXPERTS + e] : args.blockscale_offsets[e]) >> 7;
+          const int groups = (n_pairs + group - 1) / group;
+          const int atoms = (m + 127) >> 7;
+          const int tiles = (atoms + ITEM_ATOMS - 1) / ITEM_ATOMS;
+          // Consecutive items run at the same time on different CTA pairs and share one operand in L2 while they sweep
+          // the other: the swept operand should be the SMALLER one.
+          int tt, g;
+          if (tiles == 1) { tt = 0; g = i; }
+          else if (m <= n) { g = i / tiles; tt = i - g * tiles; }
+          else { tt = i / groups; g = i - tt * groups; }
+          const int base = atoms / tiles, rem = atoms - base * tiles;      // the atoms in tiles of base or base + 1
+          const int atom0 = tt * base + (tt < rem ? tt : rem);
+          const int rows = (base + (tt < rem ? 1 : 0)) * 128;
+          const int left = m - atom0 * 128;
+          it.valid = left < rows ? left : rows;
+          it.row0 = row_first + atom0 * 128;
+          const int n0 = it.valid <= SUB_TILE ? (it.valid + 15) & ~15 : it.valid <= 256 ? 128 : SUB_TILE;
+          const int n1 = it.valid > n0 ? (it.valid - n0 + 15) & ~15 : 0;
+          it.n01 = n0 | (n1 << 16);
+          it.np0 = g * group;
+          it.units = n_pairs - it.np0 < group ? n_pairs - it.np0 : group;
+          it.e = e;
+          it.sfx_row = sf_first + atom0;
+          it.one_tile = tiles == 1;
         }
-        q_ok = __shfl_sync(0xffffffffu, (int)q_ok, 0) != 0;
-        t = __shfl_sync(0xffffffffu, t, 0);
-        e = __shfl_sync(0xffffffffu, e, 0);
-      } else {
-        q_ok = __all_sync(0xffffffffu, ptx::mbar_wait_cluster(&ctl->q_full[qs], qph, abort_flag));
-        if (q_ok) {
-          t = ctl->q_item[qs].x;
-          e = ctl->q_item[qs].y;
-          __syncwarp();
-          if (lane == 0) ptx::mbar_arrive_cluster(&ctl->q_empty[qs], 0);
-        }
-      }
-      if (++qs == QUEUE_DEPTH) { qs = 0; qph ^= 1u; }
-      if (!q_ok) {
-        if (lane == 0) {
-          *abort_flag = 1;
-          atomicOr(&g_status, ERR_PRODUCER);
-        }
-        break;
-      }
-      if (t < 0) break;
-      const TileInfo ti = decode_tile(t, e, tab, n, n_pairs);
-      const int half0 = ti.n0 >> 1, half1 = ti.n1 >> 1;     // token rows of each sub-tile held by each CTA
-      const int xi0 = box_index(half0), xi1 = box_index(half1);
-      const uint32_t tx = 2u * (W_BYTES + box_rows_of(xi0) * TILE_K + (ti.n1 ? box_rows_of(xi1) * TILE_K : 0u) +
-                                SFW_BYTES + SFX_BYTES);
-      int nt = ti.np * 2 + (int)rank;
-      const int w_row = ti.e * n + nt * TILE_N;             // may run past the expert when n/128 is odd: not stored
-      if (nt >= n_tiles) nt = n_tiles - 1;                  // keep the scale-atom load inside the buffer
-      const int sfw_atom = ti.e * sfw_atoms_per_expert + nt * kt_count;
-      const int bs_off = tab.scale0(ti.e);                  // a multiple of 128 (checked by the scan)
-      const int sfx_atom_row = (bs_off >> 7) + ti.atom0;
-      // this lane's load: 0 weights, 1 tokens of sub-tile 0, 2 tokens of sub-tile 1, 3 weight scales, 4 the three
-      // token scale atoms of the item (one load: the lanes of a warp issue their loads one after the other, ~75
-      // cycles each, and the producer's issue time per K step is part of every stage's turnaround)
-      const bool active = lane == 0 || lane == 1 || (lane == 2 && ti.n1 > 0) || lane == 3 || lane == 4;
-      const CUtensorMap* my_map = lane == 0 ? &maps.w : lane == 1 ? &maps.x[xi0] : lane == 2 ? &maps.x[xi1]
-                                  : lane == 3 ? &maps.sfw : &maps.sfx;
-      const uint32_t my_off = lane == 0 ? 0u : lane == 1 ? (uint32_t)W_BYTES : lane == 2 ? (uint32_t)(W_BYTES + X_BYTES)
-                              : lane == 3 ? (uint32_t)(W_BYTES + 2 * X_BYTES)
-                                          : (uint32_t)(W_BYTES + 2 * X_BYTES + SFW_BYTES);
-      const int my_c1 = lane == 0 ? w_row : lane == 1 ? ti.row0 + (int)rank * half0
-                        : lane == 2 ? ti.row0 + SUB_TILE + (int)rank * half1
-                        : lane == 3 ? sfw_atom : sfx_atom_row;
-      const uint64_t my_hint = lane < 3 ? ptx::kL2EvictLast : ptx::kL2EvictNormal;
-      bool ok = true;
-      for (int kt = 0; kt < kt_count; ++kt) {
-        ok = __all_sync(0xffffffffu, ptx::mbar_wait(&ctl->empty[s], ph ^ 1u, abort_flag));
-        if (!ok) break;
-        uint8_t* stage = smem + (size_t)s * STAGE_BYTES;
-        if (rank == 0 && lane == 0) ptx::mbar_arrive_expect_tx(&ctl->full[s], tx);
-        __syncwarp();
-        if (active)
-          ptx::tma_load_2d_pair_hint(stage + my_off, my_map, &ctl->full[s],
-                                     lane < 3 ? kt * TILE_K : lane == 3 ? 0 : kt * 128,
-                                     lane == 3 ? my_c1 + kt : my_c1, my_hint);
-        if (++s == STAGES) { s = 0; ph ^= 1u; }
-      }
-      if (!ok) {
-        if (lane == 0) {
-          *abort_flag = 1;
-          atomicOr(&g_status, ERR_PRODUCER);
-        }
-        break;
-      }
-    }
-  } else if (warp == 1 || warp == MMA_B_WARP) {
-    // ------------------------------------------------------------------ MMA issue (leader CTA): warp 1 issues the
-    // MMAs of sub-tile 0 into accumulator 0, warp 18 those of sub-tile 1 into accumulator 1
-    if (lane == 0 && rank == 0) {
-      const int sub = warp == 1 ? 0 : 1;
-      int s = 0, qs = 0;
-      uint32_t ph = 0, qph = 0;
-      uint32_t acc_ph = 0;             // phase of this accumulator's empty barrier (advances once per use)
-      bool ok = true;
-      while (ok) {
-        if (!ptx::mbar_wait(&ctl->q_full[qs], qph, abort_flag)) {
-          *abort_flag = 1;
-          atomicOr(&g_status, ERR_MMA);
+        if (!__all_sync(0xffffffffu, ptx::mbar_wait(&ctl->q_empty[qs], qph ^ 1u, abort_flag))) {
+          if (lane == 0) give_up(ERR_SCHEDULER);
           break;
         }
-        const int t = ctl->q_item[qs].x;
-        const int e = ctl->q_item[qs].y;
-        ptx::mbar_arrive(&ctl->q_empty[qs]);
+        if (t == pair) ptx::fence_proxy_async_shared();     // the facts have been read: loads may overwrite them
+        if (lane == 0) {
+          const int4 a = make_int4(it.valid, it.row0, it.n01, it.np0), b = make_int4(it.units, it.e, it.sfx_row, it.one_tile);
+          int4* dst = reinterpret_cast<int4*>(&ctl->q_item[qs]);
+          dst[0] = a;
+          dst[1] = b;
+          ptx::mbar_arrive(&ctl->q_full[qs]);
+          ptx::send_32B_to_cluster_cta(&ctl->q_item[qs], &ctl->q_full[qs], 1, a, b);
+        }
+        __syncwarp();
         if (++qs == QUEUE_DEPTH) { qs = 0; qph ^= 1u; }
-        if (t < 0) break;
-        const TileInfo ti = decode_tile(t, e, tab, n, n_pairs);
-        const uint32_t n_mma = sub == 0 ? ti.n0 : ti.n1;
-        const uint32_t d_acc = tmem_base + sub * ACC_COLS;
-        for (int kt = 0; ok && kt < kt_count; ++kt) {
-          if (!ptx::mbar_wait(&ctl->full[s], ph, abort_flag)) { ok = false; break; }
-          if (n_mma > 0) {
-            if (!ptx::mbar_wait(&ctl->sf_ready[s], ph, abort_flag)) { ok = false; break; }
-            if (kt == 0) {   // the previous item's epilogue must have drained this accumulator
-              if (!ptx::mbar_wait(&ctl->tmem_empty[sub], acc_ph ^ 1u, abort_flag)) { ok = false; break; }
-              acc_ph ^= 1u;
+        if (it.valid < 0) break;
+      }
+    }
+  } else if (warp == W_WARP) {
+    // ------------------------------------------------------------------ weights and both scales of every K step (one thread)
+    if (ptx::elect_one()) {
+      int s = 0;
+      uint32_t ph = 0;
+      bool ok = true;
+      while (ok) {
+        Item it;
+        ok = next_item_one(&it);
+        if (!ok || it.valid < 0) break;
+        const bool three = it.valid > 128;
+        const uint32_t mine = W_BYTES + SF_BYTES + (three ? SFX_BYTES : SF_BYTES);
+        const uint64_t hint = it.one_tile ? ptx::kL2EvictFirst : ptx::kL2EvictLast;
+        const CUtensorMap* sfx_map = three ? &maps.sfx3 : &maps.sfx1;
+        for (int u = 0; ok && u < it.units; ++u) {
+          const int nt = (it.np0 + u) * 2 + (int)rank;
+          const bool have = nt < n_tiles;          // n / 128 odd: the last pair's second half does not exist
+          const uint32_t tx = mine * ((it.np0 + u) * 2 + 1 < n_tiles ? 2u : 1u);
+          const int w_row = it.e * n + nt * TILE_N;
+          const int sfw_atom = (it.e * n_tiles + nt) * kt_count;
+          for (int kt = 0; kt < kt_count; ++kt) {
+            ok = ptx::mbar_wait(&ctl->empty[s], ph ^ 1u, abort_flag);
+            if (!ok) break;
+            uint8_t* slot = smem + (size_t)s * W_SLOT;
+            if (rank == 0) ptx::mbar_arrive_expect_tx(&ctl->full[s], tx);
+            if (have) {
+              ptx::tma_load_2d_pair_hint(slot, &maps.w, &ctl->full[s], kt * TILE_K, w_row, hint);
+              ptx::tma_load_2d_pair_hint(slot + W_BYTES, &maps.sfw, &ctl->full[s], 0, sfw_atom + kt, ptx::kL2EvictNormal);
+              ptx::tma_load_2d_pair_hint(slot + W_BYTES + SF_BYTES, sfx_map, &ctl->full[s], kt * 128, it.sfx_row,
+                                         ptx::kL2EvictNormal);
             }
+            if (++s == W_STAGES) { s = 0; ph ^= 1u; }
+          }
+        }
+      }
+      if (!ok) give_up(ERR_PRODUCER);
+    }
+    __syncwarp();
+  } else if (warp == X_WARP) {
+    // ------------------------------------------------------------------ token rows (one thread): one slot per sub-tile of a
+    // K step.  A slot is free when the K step that used it last has completed, whose barrier is empty[] of that step's
+    // weight slot.  A step further back than W_STAGES is not waited for but the one W_STAGES back is, whose weight slot this
+    // step takes anyway: a parity wait cannot tell a phase from the one two further.
+    if (ptx::elect_one()) {
+      int s = 0, x = 0, step = 0;
+      uint32_t ph = 0;
+      for (int i = 0; i < X_STAGES; ++i) ctl->x_user[i] = -W_STAGES;
+      bool ok = true;
+      while (ok) {
+        Item it;
+        ok = next_item_one(&it);
+        if (!ok || it.valid < 0) break;
+        const int n0 = it.n01 & 0xffff, n1 = it.n01 >> 16;
+        const int xi0 = box_index(n0 >> 1), xi1 = box_index(n1 >> 1);
+        const CUtensorMap* map0 = &maps.x[xi0];
+        const CUtensorMap* map1 = &maps.x[xi1];
+        const uint32_t tx = 2u * TILE_K * (box_rows_of(xi0) + (n1 ? box_rows_of(xi1) : 0u));
+        const int row0 = it.row0 + (int)rank * (n0 >> 1), row1 = it.row0 + n0 + (int)rank * (n1 >> 1);
+        for (int u = 0; ok && u < it.units; ++u) {
+          for (int kt = 0; kt < kt_count; ++kt) {
+            const int x1 = x + 1 == X_STAGES ? 0 : x + 1;
+            int back = step - ctl->x_user[n1 ? x1 : x];      // the later of the slots' users, in steps back
+            if (back > W_STAGES) back = W_STAGES;
+            if (back <= step) {
+              const int us = s - back;                       // its weight slot, of this revolution or of the one before
+              ok = ptx::mbar_wait(&ctl->empty[us < 0 ? us + W_STAGES : us], us < 0 ? ph ^ 1u : ph, abort_flag);
+              if (!ok) break;
+            }
+            if (rank == 0) ptx::mbar_arrive_expect_tx(&ctl->full[s], tx);
+            ptx::tma_load_2d_pair_hint(x_ring + (size_t)x * X_SLOT, map0, &ctl->full[s], kt * TILE_K, row0, ptx::kL2EvictLast);
+            ctl->x_user[x] = step;
+            x = x1;
+            if (n1) {
+              ptx::tma_load_2d_pair_hint(x_ring + (size_t)x * X_SLOT, map1, &ctl->full[s], kt * TILE_K, row1, ptx::kL2EvictLast);
+              ctl->x_user[x] = step;
+              if (++x == X_STAGES) x = 0;
+            }
+            ++step;
+            if (++s == W_STAGES) { s = 0; ph ^= 1u; }
+          }
+        }
+      }
+      if (!ok) give_up(ERR_PRODUCER);
+    }
+    __syncwarp();
+  } else if (warp == MMA_WARP) {
+    // ------------------------------------------------------------------ scale copies and MMAs (leader, one thread)
+    if (rank == 0 && ptx::elect_one()) {
+      int s = 0, x = 0;
+      uint32_t ph = 0, cnt = 0;
+      const uint32_t smem_base = ptx::smem_u32(smem), x_base = ptx::smem_u32(x_ring);
+      bool ok = true;
+      while (ok) {
+        Item it;
+        ok = next_item_one(&it);
+        if (!ok || it.valid < 0) break;
+        const int n0 = it.n01 & 0xffff, n1 = it.n01 >> 16;
+        const int atoms = (it.valid + 127) >> 7;
+        const uint32_t idesc0 = ptx::make_idesc_mxf8(2 * TILE_N, n0, 0, 0), idesc1 = ptx::make_idesc_mxf8(2 * TILE_N, n1, 0, 0);
+        for (int u = 0; ok && u < it.units; ++u) {
+          const uint32_t a0 = cnt & 1u, a1 = a0 ^ 1u;
+          ok = ptx::mbar_wait(&ctl->acc_empty[a0], ((cnt >> 1) & 1u) ^ 1u, abort_flag);
+          if (!ok) break;
+          // one K step's scale copies and MMAs of sub-tile 0
+          auto first_half = [&](int kt) {
+            if (!ptx::mbar_wait(&ctl->full[s], ph, abort_flag)) return false;
             ptx::tc_fence_after_sync();
-            const uint32_t stage = ptx::smem_u32(smem + (size_t)s * STAGE_BYTES);
-            const uint32_t sfw_t = tmem_base + SF_COL0 + s * SF_SLOT_COLS;
-            // sub-tile 1 starts 192 rows = 6 scale columns into the item's block of token scales
-            const uint32_t sfx_t = sfw_t + 4 + sub * 6;
-            const uint64_t a_desc = ptx::make_desc_k_sw128(stage);
-            const uint64_t b_desc = ptx::make_desc_k_sw128(stage + W_BYTES + sub * X_BYTES);
+            const uint32_t slot = smem_base + s * W_SLOT;
+            const uint32_t sfw_t = tmem_base + SF_COL0 + s * SF_SLOT_COLS, sfx_t = sfw_t + 4;
+            const uint64_t a_desc = ptx::make_desc_k_sw128(slot);
+            const uint64_t sf_desc = ptx::make_desc_sf(slot + W_BYTES);
+            const uint64_t b_desc = ptx::make_desc_k_sw128(x_base + x * X_SLOT);
+            ptx::tc_cp_sf_pair(sfw_t, sf_desc);
+            ptx::tc_cp_sf_pair(sfx_t, sf_desc + (512 >> 4));
+            if (atoms > 1) ptx::tc_cp_sf_pair(sfx_t + 4, sf_desc + (1024 >> 4));
+            if (atoms > 2) ptx::tc_cp_sf_pair(sfx_t + 8, sf_desc + (1536 >> 4));
 #pragma unroll
             for (uint32_t j = 0; j < 4; ++j)
-              ptx::tc_mma_mxf8_pair(d_acc, a_desc + 2 * j, b_desc + 2 * j, ptx::make_idesc_mxf8(2 * TILE_N, n_mma, j, j),
+              ptx::tc_mma_mxf8_pair(tmem_base + a0 * ACC_COLS, a_desc + 2 * j, b_desc + 2 * j, idesc0 | (j << 4) | (j << 29),
                                     sfw_t | (j << 30), sfx_t | (j << 30), (kt | j) != 0 ? 1u : 0u);
+            return true;
+          };
+          // the MMAs of sub-tile 1 of the K step in weight slot sl, token slot xl
+          auto second_half = [&](int kt, int sl, int xl) {
+            const uint32_t sfw_t = tmem_base + SF_COL0 + sl * SF_SLOT_COLS;
+            const uint32_t sfx_t = sfw_t + 4 + (n0 >> 5);      // sub-tile 1 starts n0 rows into the token scales
+            const uint64_t a_desc = ptx::make_desc_k_sw128(smem_base + sl * W_SLOT);
+            const uint64_t b_desc = ptx::make_desc_k_sw128(x_base + xl * X_SLOT);
+#pragma unroll
+            for (uint32_t j = 0; j < 4; ++j)
+              ptx::tc_mma_mxf8_pair(tmem_base + a1 * ACC_COLS, a_desc + 2 * j, b_desc + 2 * j, idesc1 | (j << 4) | (j << 29),
+                                    sfw_t | (j << 30), sfx_t | (j << 30), (kt | j) != 0 ? 1u : 0u);
+            ptx::tc_commit_pair(&ctl->empty[sl], 3);
+          };
+          auto next_x = [&](int i) { return i + 1 == X_STAGES ? 0 : i + 1; };
+          auto next_step = [&]() { if (++s == W_STAGES) { s = 0; ph ^= 1u; } };
+          if (n1 == 0) {
+            for (int kt = 0; ok && kt < kt_count; ++kt) {
+              ok = first_half(kt);
+              if (!ok) break;
+              ptx::tc_commit_pair(&ctl->empty[s], 3);
+              x = next_x(x);
+              next_step();
+            }
+            if (!ok) break;
+            ptx::tc_commit_pair(&ctl->acc_full[a0], 3);
+            cnt += 1;
+          } else {
+            // The first two and the last two K steps go sub-tile by sub-tile: accumulator 0 is then complete 2 x 4 MMAs before
+            // accumulator 1 and wanted back as much earlier, which hides the time that the epilogue takes to empty it.
+            for (int kt = 0; ok && kt < kt_count;) {
+              const bool two = kt + 1 < kt_count && (kt == 0 || kt + 2 == kt_count);
+              const int s0 = s, x0 = next_x(x);
+              ok = first_half(kt);
+              if (!ok) break;
+              x = next_x(x0);
+              next_step();
+              int s1 = s, x1 = 0;
+              if (two) {
+                x1 = next_x(x);
+                ok = first_half(kt + 1);
+                if (!ok) break;
+                x = next_x(x1);
+                next_step();
+              }
+              if (kt + (two ? 2 : 1) == kt_count) ptx::tc_commit_pair(&ctl->acc_full[a0], 3);
+              if (kt == 0) {
+                ok = ptx::mbar_wait(&ctl->acc_empty[a1], (((cnt + 1) >> 1) & 1u) ^ 1u, abort_flag);
+                if (!ok) break;
+                ptx::tc_fence_after_sync();
+              }
+              second_half(kt, s0, x0);
+              if (two) second_half(kt + 1, s1, x1);
+              kt += two ? 2 : 1;
+            }
+            if (!ok) break;
+            ptx::tc_commit_pair(&ctl->acc_full[a1], 3);
+            cnt += 2;
           }
-          ptx::tc_commit_pair(&ctl->empty[s], 3);       // this lane's share: both CTAs may refill once both have
-          if (++s == STAGES) { s = 0; ph ^= 1u; }
-        }
-        if (!ok) {
-          *abort_flag = 1;
-          atomicOr(&g_status, ERR_MMA);
-          break;
-        }
-        if (n_mma > 0) ptx::tc_commit_pair(&ctl->tmem_full[sub], 3);     // this accumulator is complete in both CTAs
-      }
-    }
-  } else if (warp == COPY_WARP) {
-    // ------------------------------------------------------------------ scale copies (leader CTA, one lane)
-    // Token rows 0..383 of the item = scale atoms 0..2: sub-tile 0 reads atoms 0 and 1, sub-tile 1 atoms 1 and 2.
-    if (lane == 0 && rank == 0) {
-      int s = 0, qs = 0;
-      uint32_t ph = 0, qph = 0;
-      bool ok = true;
-      while (ok) {
-        if (!ptx::mbar_wait(&ctl->q_full[qs], qph, abort_flag)) {
-          *abort_flag = 1;
-          atomicOr(&g_status, ERR_SCALE_COPY);
-          break;
-        }
-        const int t = ctl->q_item[qs].x;
-        const int e = ctl->q_item[qs].y;
-        ptx::mbar_arrive(&ctl->q_empty[qs]);
-        if (++qs == QUEUE_DEPTH) { qs = 0; qph ^= 1u; }
-        if (t < 0) break;
-        const TileInfo ti = decode_tile(t, e, tab, n, n_pairs);
-        for (int kt = 0; kt < kt_count; ++kt) {
-          if (!ptx::mbar_wait(&ctl->full[s], ph, abort_flag)) { ok = false; break; }
-          ptx::tc_fence_after_sync();
-          const uint32_t sf_smem = ptx::smem_u32(smem + (size_t)s * STAGE_BYTES) + W_BYTES + 2 * X_BYTES;
-          const uint32_t sfw_t = tmem_base + SF_COL0 + s * SF_SLOT_COLS;
-          ptx::tc_cp_sf_pair(sfw_t, ptx::make_desc_sf(sf_smem));
-          ptx::tc_cp_sf_pair(sfw_t + 4, ptx::make_desc_sf(sf_smem + SFW_BYTES));
-          if (ti.n_atoms > 1) ptx::tc_cp_sf_pair(sfw_t + 8, ptx::make_desc_sf(sf_smem + SFW_BYTES + 512));
-          if (ti.n_atoms > 2) ptx::tc_cp_sf_pair(sfw_t + 12, ptx::make_desc_sf(sf_smem + SFW_BYTES + 1024));
-          ptx::tc_commit_pair(&ctl->sf_ready[s], 1);    // leader's barrier, once the copies have landed in both TMEMs
-          if (++s == STAGES) { s = 0; ph ^= 1u; }
-        }
-        if (!ok) {
-          *abort_flag = 1;
-          atomicOr(&g_status, ERR_SCALE_COPY);
         }
       }
+      if (!ok) give_up(ERR_MMA);
     }
+    __syncwarp();
   } else {
-    // ------------------------------------------------------------------ epilogue (both CTAs), 16 warps: four per
-    // TMEM lane quadrant share the twelve 32-column chunks of an item's two accumulators, three each (two of one
-    // accumulator and one of the other).  A warp reads its chunks of accumulator 0 into registers (converted), hands
-    // accumulator 0 back, does the same for accumulator 1, and stores afterwards: both accumulators of an item
-    // complete together, the MMA lanes get them back after ~two TMEM reads each instead of after the stores (which
-    // take several thousand cycles per item), and the next item's MMAs run during the stores.
-    //   slot 0: accumulator 0, columns 32 idx          slot 1: idx < 2 ? accumulator 0, columns 32 idx + 128
-    //   slot 2: idx < 2 ? accumulator 1, columns 32 (idx + 2)              : accumulator 1, columns 32 (idx - 2)
-    //                   : accumulator 1, columns 32 (idx - 2) + 128
+    // ------------------------------------------------------------------ epilogue (both CTAs), 12 warps: three per TMEM lane
+    // quadrant share the 32-column chunks of the accumulators, at most two per sub-tile.  A warp reads its chunks of a
+    // weight pair's accumulators into registers (converted), hands each accumulator back, and stores afterwards: the next
+    // weight pair's MMAs run during the stores.
     const int q = warp & 3;
-    const int idx = (warp - 2) >> 2;      // 0..3 within the lane quadrant
-    const bool low = idx < 2;
-    const int col0 = idx * 32;
-    const int col1 = low ? idx * 32 + 128 : (idx - 2) * 32;
-    const int col2 = low ? (idx + 2) * 32 : (idx - 2) * 32 + 128;
-    OutT* stage_warp = reinterpret_cast<OutT*>(epi_stage) + (warp - 2) * (EPI_BYTES_PER_WARP / 2);
-    // HOLD = false (chosen by the host for one or two K steps per item): each chunk is stored right after it is read.
-    // Such a call is bound by the output stores themselves (n x k is small against the m x n output) and holding only
-    // adds concurrent load traffic to them (measured at k = 256: 1.03 ms held, 0.71 ms not).
-    uint32_t full_ph = 0, qph = 0;        // both accumulators' barriers advance once per item that uses them
-    uint32_t full1_ph = 0;
-    int qs = 0;
-    while (true) {
-      const bool have = rank == 0 ? ptx::mbar_wait(&ctl->q_full[qs], qph, abort_flag)
-                                  : ptx::mbar_wait_cluster(&ctl->q_full[qs], qph, abort_flag);
-      if (!__all_sync(0xffffffffu, have)) {
-        if (lane == 0) {
-          *abort_flag = 1;
-          atomicOr(&g_status, ERR_EPILOGUE);
-        }
-        break;
-      }
-      const int t = ctl->q_item[qs].x;
-      const int e = ctl->q_item[qs].y;
-      __syncwarp();
-      if (lane == 0) ptx::mbar_arrive_cluster(&ctl->q_empty[qs], 0);   // leader's barrier
-      if (++qs == QUEUE_DEPTH) { qs = 0; qph ^= 1u; }
-      if (t < 0) break;
-      const TileInfo ti = decode_tile(t, e, tab, n, n_pairs);
-      const int nt = ti.np * 2 + (int)rank;
-      const bool store = nt < n_tiles;
-      const bool store_now = !HOLD && store;
-      const uint32_t lane_base = tmem_base + ((uint32_t)(q * 32) << 16);
-      uint32_t held0[16], held1[16], held2[16];
-      // which of this warp's chunks exist in this item (warp-uniform)
-      const bool has0 = col0 < ti.n0;
-      const bool has1 = low ? col1 < ti.n0 : col1 < ti.n1;
-      const bool has2 = col2 < ti.n1;
-      // token row (within the item) of each slot's first column
-      const int tok0 = col0;
-      const int tok1 = low ? col1 : SUB_TILE + col1;
-      const int tok2 = SUB_TILE + col2;
-      const int col_off = nt * TILE_N + q * 32;
-      auto store_slot = [&](const uint32_t (&held)[16], int tok) {
-        if (scatter.meta == nullptr) {
-          uint16_t* out = reinterpret_cast<uint16_t*>(d + (int64_t)(ti.row0 + tok) * n + col_off);
-          store_held_chunk_dense(held, out, n, ti.valid - tok, lane);
-        } else {
-          // lane l fetches the destination of token l of the chunk
-          OutT* dest = scatter_row_ptr<OutT>(scatter, ti.row0 + tok + lane, tok + lane < ti.valid, n, col_off, &g_status);
-          store_held_chunk_scatter<OutT>(held, stage_warp, dest, lane);
-        }
-      };
-      bool got = ptx::mbar_wait(&ctl->tmem_full[0], full_ph, abort_flag);
-      if (!__all_sync(0xffffffffu, got)) {
-        if (lane == 0) {
-          *abort_flag = 1;
-          atomicOr(&g_status, ERR_EPILOGUE);
-        }
-        break;
-      }
-      full_ph ^= 1u;
-      ptx::tc_fence_after_sync();
-      if (has0) {
-        read_held_chunk<OutT>(lane_base + col0, held0);
-        if (store_now) store_slot(held0, tok0);
-      }
-      if (low && has1) {
-        read_held_chunk<OutT>(lane_base + col1, held1);
-        if (store_now) store_slot(held1, tok1);
-      }
-      ptx::tc_fence_before_sync();
-      __syncwarp();
-      if (lane == 0) ptx::mbar_arrive_cluster(&ctl->tmem_empty[0], 0);     // leader's barrier
-      if (ti.n1 > 0) {                                      // an item of <= 192 rows does not use accumulator 1
-        got = ptx::mbar_wait(&ctl->tmem_full[1], full1_ph, abort_flag);
-        if (!__all_sync(0xffffffffu, got)) {
-          if (lane == 0) {
-            *abort_flag = 1;
-            atomicOr(&g_status, ERR_EPILOGUE);
-          }
-          break;
-        }
-        full1_ph ^= 1u;
+    const int idx = (warp - EPI_WARP0) >> 2;      // 0..2 within the lane quadrant
+    const uint32_t stage = ptx::smem_u32(epi_stage) + (warp - EPI_WARP0) * EPI_BYTES_PER_WARP;
+    const uint32_t lane_base = tmem_base + ((uint32_t)(q * 32) << 16);
+    OutT* const d = static_cast<OutT*>(args.d);
+    const bool scattered = scatter.meta != nullptr;
+    uint32_t cnt = 0;
+    int turn = idx;                               // first chunk of this warp; rotates so that small tiles go round
+    bool ok = true;
+    while (ok) {
+      Item it;
+      ok = next_item(&it);
+      if (!ok || it.valid < 0) break;
+      const int n0 = it.n01 & 0xffff, n1 = it.n01 >> 16;
+      for (int u = 0; u < it.units; ++u) {
+        const int nt = (it.np0 + u) * 2 + (int)rank;
+        const int col_off = nt * TILE_N + q * 32;
+        const uint32_t a0 = cnt & 1u, a1 = a0 ^ 1u;
+        const uint32_t p0 = (cnt >> 1) & 1u, p1 = ((cnt + 1) >> 1) & 1u;
+        const int c0 = turn * 32, c1 = c0 + 96;
+        uint32_t held[4][16];
+        ok = __all_sync(0xffffffffu, ptx::mbar_wait(&ctl->acc_full[a0], p0, abort_flag));
+        if (!ok) break;
         ptx::tc_fence_after_sync();
-        if (!low && has1) {
-          read_held_chunk<OutT>(lane_base + ACC_COLS + col1, held1);
-          if (store_now) store_slot(held1, tok1);
-        }
-        if (has2) {
-          read_held_chunk<OutT>(lane_base + ACC_COLS + col2, held2);
-          if (store_now) store_slot(held2, tok2);
-        }
+        const uint32_t t0 = lane_base + a0 * ACC_COLS, t1 = lane_base + a1 * ACC_COLS;
+        if (c1 < n0) read_two_chunks<OutT>(t0 + c0, t0 + c1, held[0], held[1]);
+        else if (c0 < n0) read_chunk<OutT>(t0 + c0, held[0]);
         ptx::tc_fence_before_sync();
         __syncwarp();
-        if (lane == 0) ptx::mbar_arrive_cluster(&ctl->tmem_empty[1], 0);
-      }
-      if (HOLD && store) {
-        if (has0) store_slot(held0, tok0);
-        if (has1) store_slot(held1, tok1);
-        if (has2) store_slot(held2, tok2);
+        if (lane == 0) ptx::mbar_arrive_cluster_relaxed(&ctl->acc_empty[a0], 0);
+        if (n1 != 0) {
+          ok = __all_sync(0xffffffffu, ptx::mbar_wait(&ctl->acc_full[a1], p1, abort_flag));
+          if (!ok) break;
+          ptx::tc_fence_after_sync();
+          if (c0 < n1) read_chunk<OutT>(t1 + c0, held[2]);
+          if (c1 < n1) read_chunk<OutT>(t1 + c1, held[3]);
+          ptx::tc_fence_before_sync();
+          __syncwarp();
+          if (lane == 0) ptx::mbar_arrive_cluster_relaxed(&ctl->acc_empty[a1], 0);
+        }
+        if (nt < n_tiles) {
+          OutT* out = d + (int64_t)it.row0 * n + col_off;
+          auto store = [&](const uint32_t (&h)[16], int tok) {
+            OutT* dest = nullptr;
+            if (scattered)
+              dest = scatter_row_ptr<OutT>(scatter, it.row0 + tok + lane, tok + lane < it.valid, n, col_off, &g_status);
+            store_chunk_16B<OutT>(h, stage, tok, it.valid, out, n, lane, scattered, dest);
+          };
+          if (c0 < n0) store(held[0], c0);
+          if (c1 < n0) store(held[1], c1);
+          if (c0 < n1) store(held[2], n0 + c0);
+          if (c1 < n1) store(held[3], n0 + c1);
+        }
+        cnt += n1 != 0 ? 2 : 1;
+        turn = turn == 0 ? 2 : turn - 1;
       }
     }
+    if (!ok && lane == 0) give_up(ERR_EPILOGUE);
   }
 
+  if (scatter.meta != nullptr) __threadfence_system();
   // neither CTA may leave (or free TMEM) while its partner can still signal it or read its shared memory
   ptx::tc_fence_before_sync();
   __syncthreads();
   ptx::settle_if_aborted(abort_flag);
   ptx::cluster_sync();
-  if (warp == 1) {
+  if (warp == MMA_WARP) {
     __syncwarp();
     ptx::tmem_dealloc_pair(tmem_base, TMEM_COLS);
   }
-  end_of_kernel(counters, wait_at_start != 0, last_of_call != 0, earlier_ctas, scatter.meta != nullptr, &g_status);
+  // the last CTA of the call clears the counters
+  if (threadIdx.x == 0 && args.counters != nullptr && atomicAdd(&args.counters[1], 1u) == gridDim.x - 1) {
+    args.counters[0] = 0;
+    args.counters[1] = 0;
+  }
 }
 
-template <typename OutT, bool HOLD>
-int launch_as(const mm::CallArgs& c, int min_rows, int cluster_cap, bool first_of_call, bool last_of_call,
-              uint32_t* earlier_ctas) {
+template <typename OutT, class S>
+int launch_as(const CallArgs& c) {
   DeviceInfo info;
   int rc = get_device_info(&info);
   if (rc != ES_B200_OK) return rc;
@@ -569,70 +700,65 @@ int launch_as(const mm::CallArgs& c, int min_rows, int cluster_cap, bool first_o
   if (rc != ES_B200_OK) return rc;
   // whole 128-row atoms only; loads past the end read as zero (a map needs at least one row)
   const uint64_t sfx_rows = (uint64_t)(c.sfa_rows / 128);
-  rc = make_tensormap_record_columns(&maps.sfx, c.sfa, sfx_rows ? sfx_rows : 1, (uint64_t)kt_count, 3);
+  rc = make_tensormap_record_columns(&maps.sfx1, c.sfa, sfx_rows ? sfx_rows : 1, (uint64_t)kt_count, 1);
+  if (rc != ES_B200_OK) return rc;
+  rc = make_tensormap_record_columns(&maps.sfx3, c.sfa, sfx_rows ? sfx_rows : 1, (uint64_t)kt_count, ITEM_ATOMS);
   if (rc != ES_B200_OK) return rc;
 
-  auto kernel = mxfp8_grouped_mm_pair_kernel<OutT, HOLD>;
+  auto kernel = mxfp8_grouped_mm_pair_kernel<OutT, S>;
   static bool configured[64] = {false};
+  static int resident_pairs[64] = {0};
   int dev = 0;
   ES_CUDA_TRY(cudaGetDevice(&dev));
   if (!configured[dev & 63]) {
-    ES_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_BYTES));
+    ES_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes<S>()));
     configured[dev & 63] = true;
   }
   cudaLaunchConfig_t cfg = {};
   cfg.blockDim = dim3(THREADS);
-  cfg.dynamicSmemBytes = SMEM_BYTES;
+  cfg.dynamicSmemBytes = smem_bytes<S>();
   cfg.stream = c.stream;
   cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = 2;
   attr[0].val.clusterDim.y = 1;
   attr[0].val.clusterDim.z = 1;
-  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  attr[1] = c.overlap;
   cfg.attrs = attr;
+  cfg.numAttrs = 1;
 
   // how many CTA pairs can be resident at once (SMs pair up inside a GPC, so this can be below sm_count / 2)
-  static int resident_clusters[64] = {0};
-  if (resident_clusters[dev & 63] == 0) {
+  if (resident_pairs[dev & 63] == 0) {
     cfg.gridDim = dim3(info.sm_count & ~1);
-    cfg.numAttrs = 1;
     int nc = 0;
     ES_CUDA_TRY(cudaOccupancyMaxActiveClusters(&nc, kernel, &cfg));
     if (nc < 1) return fail(ES_B200_ERR_CUDA, "no CTA pair of the grouped GEMM kernel fits on this device");
-    resident_clusters[dev & 63] = nc;
+    resident_pairs[dev & 63] = nc;
   }
+  if (attr[1].id == cudaLaunchAttributeProgrammaticStreamSerialization) cfg.numAttrs = 2;
   const int n_pairs = (c.n / TILE_N + 1) / 2;
-  const int64_t max_tiles = ((c.num_rows + TOK_TILE - 1) / TOK_TILE + c.num_experts) * (int64_t)n_pairs;
-  int max_clusters = resident_clusters[dev & 63];
-  if (cluster_cap > 0 && cluster_cap < max_clusters) max_clusters = cluster_cap;
-  const int clusters = (int)(max_tiles < max_clusters ? max_tiles : max_clusters);
-  cfg.gridDim = dim3(2 * clusters);
-  cfg.numAttrs = 2;
-  ES_CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, maps, static_cast<OutT*>(c.d), c.ps, c.eo, c.bo, c.num_experts, c.n, c.k,
-                                 min_rows, first_of_call ? 1 : 0, *c.scatter, c.counters, last_of_call ? 1 : 0,
-                                 *earlier_ctas));
-  *earlier_ctas += 2u * (uint32_t)clusters;
+  const int64_t used = c.num_experts < c.num_rows ? c.num_experts : c.num_rows;
+  const int group_light = weight_tiles_per_item(tunables().mm_item_k_steps, kt_count, used * n_pairs, info.sm_count);
+  const int group_heavy = (group_light + 3) / 4;
+  const int64_t max_items = ((c.num_rows + 128 * ITEM_ATOMS - 1) / (128 * ITEM_ATOMS) + c.num_experts) * (int64_t)n_pairs;
+  int max_pairs = resident_pairs[dev & 63];
+  if (c.max_pairs > 0 && c.max_pairs < max_pairs) max_pairs = c.max_pairs;
+  cfg.gridDim = dim3(2 * (unsigned)(max_items < max_pairs ? max_items : max_pairs));
+  KernelArgs args = {c.d, c.ps, c.eo, c.bo, c.num_experts, c.n, c.k, c.heavy_min, group_heavy, group_light, c.counters};
+  ES_CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, maps, args, *c.scatter));
   return ES_B200_OK;
 }
 
-// items of one or two K steps store each chunk as soon as it is read (see the epilogue)
+// Which division of shared memory, by the mean number of rows per expert (the only thing about them that the host knows):
+// 512 rows on 256 experts, n = 7168, k = 2048 239 us with seven weight slots, 246 with six; 64 experts of 100 rows, n = k =
+// 2048 55.4 and 56.5; 256 rows on each of 128 experts, n = 1536, k = 2048 128.5 and 117.6; 32768 Zipf rows on 256 experts,
+// n = 4096, k = 7168 1604 and 1589; 14600 rows of 1 to 1000 on 256 experts, n = 7168, k = 256 125.0 and 123.1.
 template <typename OutT>
-int launch(const mm::CallArgs& c, int min_rows, int cluster_cap, bool first_of_call, bool last_of_call,
-           uint32_t* earlier_ctas) {
-  return c.k / TILE_K > 2 ? launch_as<OutT, true>(c, min_rows, cluster_cap, first_of_call, last_of_call, earlier_ctas)
-                          : launch_as<OutT, false>(c, min_rows, cluster_cap, first_of_call, last_of_call, earlier_ctas);
+int launch(const CallArgs& c) {
+  return c.num_rows < (int64_t)112 * c.num_experts ? launch_as<OutT, FewRows>(c) : launch_as<OutT, ManyRows>(c);
 }
-
-int launch_bf16(const mm::CallArgs& c, int min_rows, int max_clusters, bool first_of_call, bool last_of_call,
-                uint32_t* earlier_ctas) {
-  return launch<__nv_bfloat16>(c, min_rows, max_clusters, first_of_call, last_of_call, earlier_ctas);
-}
-int launch_fp16(const mm::CallArgs& c, int min_rows, int max_clusters, bool first_of_call, bool last_of_call,
-                uint32_t* earlier_ctas) {
-  return launch<__half>(c, min_rows, max_clusters, first_of_call, last_of_call, earlier_ctas);
-}
+int launch_bf16(const CallArgs& c) { return launch<__nv_bfloat16>(c); }
+int launch_fp16(const CallArgs& c) { return launch<__half>(c); }
 
 int read_and_clear_status(uint32_t* out) {
   uint32_t v = 0;
@@ -645,5 +771,5 @@ int read_and_clear_status(uint32_t* out) {
   return ES_B200_OK;
 }
 
-}  // namespace mm2
+}  // namespace mm
 }  // namespace es_b200

@@ -122,25 +122,8 @@ __device__ __forceinline__ void bulk_load(void* smem_dst, const void* gmem_src, 
                : "memory");
 }
 
-// ---- LSU-side asynchronous copies (cp.async): the second way into shared memory besides TMA --------------------
-// 16 bytes global -> shared, bypassing L1; src_bytes = 0 writes zeros instead of reading (rows past the end of a tensor)
-__device__ __forceinline__ void cp_async_16(uint32_t smem_dst, const void* gmem_src, uint32_t src_bytes) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_dst), "l"(gmem_src), "r"(src_bytes) : "memory");
-}
-// arrive on an mbarrier (without raising its pending count) once all cp.async issued so far by this thread have landed
-__device__ __forceinline__ void cp_async_arrive_noinc(uint64_t* bar) {
-  asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
-// the same with an L2 eviction-priority hint
-__device__ __forceinline__ void cp_async_16_hint(uint32_t smem_dst, const void* gmem_src, uint64_t hint) {
-  asm volatile("cp.async.cg.shared.global.L2::cache_hint [%0], [%1], 16, %2;" ::"r"(smem_dst), "l"(gmem_src), "l"(hint)
-               : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait_group() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
-// orders this thread's completed generic-proxy writes to shared memory (st.shared, cp.async) before later reads of
-// that memory through the async proxy (tcgen05.mma / tcgen05.cp operands) by threads it then synchronises with
+// orders this thread's completed generic-proxy writes to shared memory (st.shared), and its reads, before later
+// accesses to that memory through the async proxy (TMA writes, tcgen05 operands) by threads it then synchronises with
 __device__ __forceinline__ void fence_proxy_async_shared() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
 // ---- tensor memory ----------------------------------------------------------------------------
@@ -214,16 +197,6 @@ __device__ __forceinline__ void tc_mma_f8(uint32_t d_tmem, uint64_t a_desc, uint
       : "memory");
 }
 
-// 32 lanes x 16 consecutive 32-bit columns -> 16 registers per thread (lane i of the warp reads TMEM lane base+i)
-__device__ __forceinline__ void tc_ld_32x32b_x16(uint32_t taddr, uint32_t (&v)[16]) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
-      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
-        "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
-      : "r"(taddr)
-      : "memory");
-}
 __device__ __forceinline__ void tc_ld_32x32b_x32(uint32_t taddr, uint32_t (&v)[32]) {
   asm volatile(
       "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
@@ -235,6 +208,29 @@ __device__ __forceinline__ void tc_ld_32x32b_x32(uint32_t taddr, uint32_t (&v)[3
         "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
       : "r"(taddr)
       : "memory");
+}
+// 16 lanes x 32 consecutive 32-bit columns -> 16 registers per thread, in the order of 8x8 matrix fragments: registers
+// 4g, 4g+1 hold lane base + l/4, columns 8g + 2(l%4) and the next (l: lane of the warp); 4g+2, 4g+3 the lane 8 further
+__device__ __forceinline__ void tc_ld_16x256b_x4(uint32_t taddr, uint32_t (&v)[16]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.16x256b.x4.b32 "
+      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
+        "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
+      : "r"(taddr)
+      : "memory");
+}
+// four 8x8 matrices of 16-bit values, each stored transposed: the 16 bytes at the address of lane 8i + j are column j of
+// matrix i
+__device__ __forceinline__ void stmatrix_x4_trans(uint32_t smem_addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+  asm volatile("stmatrix.sync.aligned.m8n8.x4.trans.shared.b16 [%0], {%1, %2, %3, %4};" ::"r"(smem_addr), "r"(a), "r"(b),
+               "r"(c), "r"(d)
+               : "memory");
+}
+__device__ __forceinline__ uint4 ld_shared_16B(uint32_t smem_addr) {
+  uint4 v;
+  asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(smem_addr) : "memory");
+  return v;
 }
 __device__ __forceinline__ void tc_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
@@ -248,44 +244,40 @@ __device__ __forceinline__ void cluster_sync() {
   asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
   asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
-// arrive on the barrier at the same shared-memory offset in CTA `rank` of the cluster
-__device__ __forceinline__ void mbar_arrive_cluster(uint64_t* bar, uint32_t rank) {
+// the two halves of cluster_sync, for work in between (the arrival releases, the wait acquires)
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+// Arrive on the barrier at the same shared-memory offset in CTA `rank` of the cluster, without release semantics: for
+// arrivals that publish no memory of the caller's — an accumulator handed back
+// after tcgen05.wait::ld + tcgen05.fence::before_thread_sync, a queue entry that has been read.  A releasing arrival at
+// cluster scope first waits for the caller's outstanding global stores (2000 - 3000 cycles in an epilogue that stores).
+__device__ __forceinline__ void mbar_arrive_cluster_relaxed(uint64_t* bar, uint32_t rank) {
   asm volatile(
       "{\n\t"
       ".reg .b32 remAddr32;\n\t"
       "mapa.shared::cluster.u32 remAddr32, %0, %1;\n\t"
-      "mbarrier.arrive.release.cluster.shared::cluster.b64 _, [remAddr32];\n\t"
+      "mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [remAddr32];\n\t"
       "}"
       ::"r"(smem_u32(bar)), "r"(rank)
       : "memory");
 }
-// store one 32-bit word at the same shared-memory offset in CTA `rank` of the cluster (distributed shared memory);
-// ordered before a following mbar_arrive_cluster by that arrive's release
-__device__ __forceinline__ void st_shared_cluster_u32(void* local_addr, uint32_t rank, uint32_t value) {
-  asm volatile(
-      "{\n\t"
-      ".reg .b32 remAddr32;\n\t"
-      "mapa.shared::cluster.u32 remAddr32, %0, %1;\n\t"
-      "st.shared::cluster.u32 [remAddr32], %2;\n\t"
-      "}"
-      ::"r"(smem_u32(local_addr)), "r"(rank), "r"(value)
-      : "memory");
-}
-// Sends 8 bytes to the same shared-memory offset in CTA `rank` of the cluster and counts them on that CTA's mbarrier
-// (same offset as `local_bar`): one arrival that expects 8 bytes, then an asynchronous store that completes them.
-// Nothing here waits for the other CTA — a plain remote store followed by a releasing remote arrive cost the sender
+// Sends 32 bytes (16-byte aligned) to the same shared-memory offset in CTA `rank` of the cluster and counts them on that
+// CTA's mbarrier (same offset as `local_bar`): one arrival that expects 32 bytes, then asynchronous stores that complete
+// them.  Nothing here waits for the other CTA — a plain remote store followed by a releasing remote arrive cost the sender
 // ~2000 cycles per use (measured).  The receiver waits on its own barrier (acquire) and reads its own copy.
-__device__ __forceinline__ void send_u64_to_cluster_cta(void* local_dst, uint64_t* local_bar, uint32_t rank, uint32_t lo,
-                                                        uint32_t hi) {
+__device__ __forceinline__ void send_32B_to_cluster_cta(void* local_dst, uint64_t* local_bar, uint32_t rank, const int4& a,
+                                                        const int4& b) {
   asm volatile(
       "{\n\t"
       ".reg .b32 remDst, remBar;\n\t"
       "mapa.shared::cluster.u32 remDst, %0, %2;\n\t"
       "mapa.shared::cluster.u32 remBar, %1, %2;\n\t"
-      "mbarrier.arrive.expect_tx.relaxed.cluster.shared::cluster.b64 _, [remBar], 8;\n\t"
-      "st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v2.b32 [remDst], {%3, %4}, [remBar];\n\t"
+      "mbarrier.arrive.expect_tx.relaxed.cluster.shared::cluster.b64 _, [remBar], 32;\n\t"
+      "st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [remDst], {%3, %4, %5, %6}, [remBar];\n\t"
+      "st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [remDst + 16], {%7, %8, %9, %10}, [remBar];\n\t"
       "}"
-      ::"r"(smem_u32(local_dst)), "r"(smem_u32(local_bar)), "r"(rank), "r"(lo), "r"(hi)
+      ::"r"(smem_u32(local_dst)), "r"(smem_u32(local_bar)), "r"(rank), "r"(a.x), "r"(a.y), "r"(a.z), "r"(a.w), "r"(b.x),
+        "r"(b.y), "r"(b.z), "r"(b.w)
       : "memory");
 }
 // bounded wait whose acquire covers writes made by the other CTA of the cluster before its arrive
@@ -318,14 +310,8 @@ __device__ __forceinline__ bool mbar_wait_cluster(uint64_t* bar, uint32_t parity
 // the even CTA of the pair (the MMA leader).
 constexpr uint32_t kPeerBitMask = 0xFEFFFFFFu;
 
-// 2-D tiled load whose completion bytes are credited to the LEADER CTA's mbarrier (either CTA of the pair may issue)
-__device__ __forceinline__ void tma_load_2d_pair(void* smem_dst, const CUtensorMap* map, uint64_t* bar, int c0, int c1) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
-      ::"r"(smem_u32(smem_dst)), "l"(reinterpret_cast<uint64_t>(map)), "r"(smem_u32(bar) & kPeerBitMask), "r"(c0), "r"(c1)
-      : "memory");
-}
-// same, with an L2 eviction-priority hint
+// 2-D tiled load whose completion bytes are credited to the LEADER CTA's mbarrier (either CTA of the pair may issue), with an
+// L2 eviction-priority hint
 __device__ __forceinline__ void tma_load_2d_pair_hint(void* smem_dst, const CUtensorMap* map, uint64_t* bar, int c0,
                                                       int c1, uint64_t hint) {
   asm volatile(

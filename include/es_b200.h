@@ -80,16 +80,15 @@ int es_b200_mxfp8_silu_mul_grouped_quant(const void* gate_up, int input_dtype, c
 /*
  * Scratch requirement (bytes of device memory, 16-byte aligned) of the MXFP8 grouped GEMM entry points.  Stands where
  * the reference allocates per-call torch::empty scratch tensors and a CUTLASS workspace
- * (es_sm100_mxfp8_blockscaled_launcher.cuh:163-176,140-142).  The kernels build their work lists in shared memory;
- * the scratch only holds the work counters through which the kernels of one call share out their tiles.  Rules:
+ * (es_sm100_mxfp8_blockscaled_launcher.cuh:163-176,140-142).  The kernel builds its work list in shared memory; the
+ * scratch only holds the counters through which the CTA pairs of a call share out its work items.  Rules:
  *   - zero it once (cudaMemset) before the first call that uses it; every call leaves it zeroed, so the same buffer
  *     serves any number of calls on one stream, graph replays included;
  *   - calls that may overlap on the GPU (different streams) need different scratch buffers;
  *   - after es_b200_check_status has reported a device-side error, zero it again (a kernel that gave up may have
  *     left counters behind); es_b200_error_epoch() counts those reports, so an owner of scratch buffers can compare
  *     it with the value it saw when it last zeroed a buffer.
- * scratch may be NULL: the kernels then deal their tiles round-robin and a large call runs its row-count buckets one
- * after the other instead of side by side (slower, same results).
+ * scratch may be NULL: the items are then dealt round-robin (slower where they differ in size, same results).
  */
 size_t es_b200_grouped_mm_scratch_bytes(int num_experts, int64_t num_rows, int n, int k);
 uint64_t es_b200_error_epoch(void);
@@ -231,16 +230,15 @@ int es_b200_ep_route_count_static(const void* topk_ids, int ids_are_int64, int p
                                   void* stream);
 
 /*
- * Tunables of the tile-shape dispatcher (no counterpart in the reference, whose bucket rules are compile-time
- * functors: es_fp8_blockwise_functor.cuh:122-256).  Process-wide; each also has an environment override read once,
- * ES_B200_<NAME IN CAPITALS>.  Names: "mm_heavy_min_rows" (experts with at least this many rows use CTA-pair tiles;
- * 0 = per-(n, k) table; at most 113), "mm_tiny_max_rows" (0 = table), "mm_pair_first_clusters",
- * "mm_split_min_rows", "mm_stream_max_ctas", "mm_pair_max_clusters" (grid shaping of a split call, 0 = no cap),
- * "mm_dynamic" (0: ignore the work counters), "mm_stream_lsu" (0: the streaming CTAs load by TMA only),
- * "mm_stream_mid_lead_ctas" (CTAs of the 112-token shape that start before the 32-token shape's; negative = built-in
- * default), "mm_item_k_steps" (K steps that a streaming work item should span: it takes that many weight tiles, at
- * most 8; at the default, 16, fewer where a call has too few tiles to occupy half the SMs, any other value is taken as
- * it is).  Unknown name: ES_B200_ERR_INVALID_ARGUMENT.
+ * Tunables (no counterpart in the reference, whose bucket rules are compile-time functors:
+ * es_fp8_blockwise_functor.cuh:122-256).  Process-wide; each also has an environment override read once,
+ * ES_B200_<NAME IN CAPITALS>.  Of the MXFP8 grouped GEMM: "mm_heavy_min_rows" (experts with at least this many rows are
+ * the heavy ones of the work list; 0 = built-in, 113), "mm_pair_max_clusters" (cap of the grid in CTA pairs, 0 = no
+ * cap), "mm_dynamic" (0: ignore the work counters, deal items round-robin), "mm_item_k_steps" (K steps that a work item
+ * should span: it takes that many tiles of 256 weight rows, at most 8; at the default, 16, fewer where a call has too few
+ * tiles to occupy half the SMs).  Accepted without effect, from earlier versions with several
+ * kernels per call: "mm_tiny_max_rows", "mm_pair_first_clusters", "mm_split_min_rows", "mm_stream_max_ctas",
+ * "mm_stream_lsu", "mm_stream_mid_lead_ctas".  Unknown name: ES_B200_ERR_INVALID_ARGUMENT.
  */
 int es_b200_set_tunable(const char* name, int value);
 
