@@ -45,7 +45,7 @@ constexpr int TILE_K = 128;
 constexpr int X_BYTES = TILE_M * TILE_K;
 constexpr int STAGE_BYTES = X_BYTES + TILE_N * TILE_K;
 constexpr int STAGES = 6;
-constexpr int PARTS = 4;             // TMEM partial buffers
+constexpr int PARTS = 4;             // TMEM partial buffers: two pairs, one for every two consecutive K blocks of a tile
 constexpr int GROUP_COLS = TILE_N / 4;   // columns of one epilogue warp
 constexpr int QUEUE_DEPTH = 4;
 constexpr int SCALES_AHEAD = 4;      // K blocks per read of the scales
@@ -68,10 +68,10 @@ struct __align__(16) Tile {
 struct SharedCtl {
   uint64_t full[STAGES];
   uint64_t empty[STAGES];
-  uint64_t part_full[PARTS];
-  uint64_t part_empty[PARTS];   // one arrival per epilogue warp
+  uint64_t pair_full[PARTS / 2];
+  uint64_t pair_empty[PARTS / 2];   // one arrival per epilogue warp
   uint64_t q_full[QUEUE_DEPTH];     // 1 arrival: the work-list lane has written the entry
-  uint64_t q_empty[QUEUE_DEPTH];    // producer, two MMA lanes, 16 epilogue warps have read it
+  uint64_t q_empty[QUEUE_DEPTH];    // producer, MMA thread, 16 epilogue warps have read it
   Tile tile[QUEUE_DEPTH];
   uint32_t tmem_base;
   int abort_flag;
@@ -80,9 +80,6 @@ struct SharedCtl {
 };
 
 constexpr size_t SMEM_BYTES = 1024 + (size_t)STAGES * STAGE_BYTES + sizeof(SharedCtl);
-// A waiter may be at most one phase ahead of its mbarrier.  K blocks alternate between two MMA lanes, so each ring
-// barrier has one waiting lane per revolution only if the rings are even.
-static_assert(STAGES % 2 == 0 && PARTS % 2 == 0, "alternating owners need even rings");
 static_assert(SMEM_BYTES <= 232448, "shared memory of one CTA per SM");
 
 __device__ uint32_t g_status = 0;
@@ -121,6 +118,13 @@ __device__ __forceinline__ void read_scales(const float* p, int left, bool vec4,
   }
 }
 
+// sixteen columns of a partial, times the scale, onto the accumulators from acc[first] on
+__device__ __forceinline__ void promote(const uint32_t (&v)[16], float2 scale, float2 (&acc)[GROUP_COLS / 2], int first) {
+#pragma unroll
+  for (int j = 0; j < 8; ++j)
+    acc[first + j] = fma2(make_float2(__uint_as_float(v[2 * j]), __uint_as_float(v[2 * j + 1])), scale, acc[first + j]);
+}
+
 template <typename OutT>
 __global__ void __launch_bounds__(THREADS, 1)
 fp8_blockwise_many_rows_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x16,
@@ -144,13 +148,13 @@ fp8_blockwise_many_rows_kernel(const __grid_constant__ CUtensorMap map_w, const 
       ptx::mbar_init(&ctl->full[s], 1);
       ptx::mbar_init(&ctl->empty[s], 1);
     }
-    for (int p = 0; p < PARTS; ++p) {
-      ptx::mbar_init(&ctl->part_full[p], 1);
-      ptx::mbar_init(&ctl->part_empty[p], EPI_WARPS);
+    for (int p = 0; p < PARTS / 2; ++p) {
+      ptx::mbar_init(&ctl->pair_full[p], 1);
+      ptx::mbar_init(&ctl->pair_empty[p], EPI_WARPS);
     }
     for (int q = 0; q < QUEUE_DEPTH; ++q) {
       ptx::mbar_init(&ctl->q_full[q], 1);
-      ptx::mbar_init(&ctl->q_empty[q], 3 + EPI_WARPS);
+      ptx::mbar_init(&ctl->q_empty[q], 2 + EPI_WARPS);
     }
     ctl->abort_flag = 0;
     ptx::fence_mbar_init();
@@ -223,7 +227,7 @@ fp8_blockwise_many_rows_kernel(const __grid_constant__ CUtensorMap map_w, const 
         if (!ok && lane == 0) give_up(abort_flag, ERR_WORK_LIST);
         if (__any_sync(0xffffffffu, t >= total)) break;      // the batch held the end mark
       }
-    } else if (lane == 0) {
+    } else if (warp <= 1 && ptx::elect_one()) {
       if (warp == 0) {
         // ---------------------------------------------------------------- producer
         QueueReader queue;
@@ -249,15 +253,12 @@ fp8_blockwise_many_rows_kernel(const __grid_constant__ CUtensorMap map_w, const 
         }
         if (!ok) give_up(abort_flag, ERR_PRODUCER);
       } else {
-        // ---------------------------------------------------------------- MMA issue: K blocks alternate between the
-        // two lanes, counted over all tiles of this CTA.  Token rows past the tile's valid ones multiply whatever the
-        // stage held before: their lanes of the accumulator are never read.
-        // A lane's own K blocks are every second one, whatever the tile: its stage and partial advance by two.
+        // ---------------------------------------------------------------- MMA issue.  Token rows past the tile's valid
+        // ones multiply whatever the stage held before: their lanes of the accumulator are never read.
         const uint32_t idesc = ptx::make_idesc_f8(TILE_M, TILE_N);
         const uint64_t desc0 = ptx::make_desc_k_sw128(ptx::smem_u32(smem));
         QueueReader queue;
-        int first = warp - 1;                       // index in the tile of this lane's first K block
-        int s = warp - 1, p = warp - 1;
+        int s = 0, p = 0;                    // stage of the next K block, pair of partials of the next two
         uint32_t ph = 0, p_ph = 0;
         bool ok = true;
         while (ok) {
@@ -265,25 +266,24 @@ fp8_blockwise_many_rows_kernel(const __grid_constant__ CUtensorMap map_w, const 
           const int valid = queue.entry(ctl).valid;
           queue.release(ctl);
           if (valid == 0) break;
-          int kt = first;
-          for (; kt < kt_count; kt += 2) {
-            if (!ptx::mbar_wait(&ctl->part_empty[p], p_ph ^ 1u, abort_flag) ||
-                !ptx::mbar_wait(&ctl->full[s], ph, abort_flag)) {
-              ok = false;
-              break;
-            }
-            ptx::tc_fence_after_sync();
-            const uint64_t x_desc = desc0 + (uint32_t)(s * (STAGE_BYTES / 16));
-            const uint64_t w_desc = x_desc + X_BYTES / 16;
-            const uint32_t part = tmem_base + p * TILE_N;
+          for (int kt = 0; ok && kt < kt_count; kt += 2) {
+            ok = ptx::mbar_wait(&ctl->pair_empty[p], p_ph ^ 1u, abort_flag);
+            for (int h = 0; ok && h < 2 && kt + h < kt_count; ++h) {
+              ok = ptx::mbar_wait(&ctl->full[s], ph, abort_flag);
+              if (!ok) break;
+              ptx::tc_fence_after_sync();
+              const uint64_t x_desc = desc0 + (uint32_t)(s * (STAGE_BYTES / 16));
+              const uint64_t w_desc = x_desc + X_BYTES / 16;
+              const uint32_t part = tmem_base + (2 * p + h) * TILE_N;
 #pragma unroll
-            for (uint32_t j = 0; j < 4; ++j) ptx::tc_mma_f8(part, x_desc + 2 * j, w_desc + 2 * j, idesc, j != 0 ? 1u : 0u);
-            ptx::tc_commit(&ctl->empty[s]);
-            ptx::tc_commit(&ctl->part_full[p]);
-            if ((s += 2) >= STAGES) { s -= STAGES; ph ^= 1u; }
-            if ((p += 2) >= PARTS) { p -= PARTS; p_ph ^= 1u; }
+              for (uint32_t j = 0; j < 4; ++j) ptx::tc_mma_f8(part, x_desc + 2 * j, w_desc + 2 * j, idesc, j != 0 ? 1u : 0u);
+              ptx::tc_commit(&ctl->empty[s]);
+              if (++s == STAGES) { s = 0; ph ^= 1u; }
+            }
+            if (!ok) break;
+            ptx::tc_commit(&ctl->pair_full[p]);
+            if (++p == PARTS / 2) { p = 0; p_ph ^= 1u; }
           }
-          first = kt - kt_count;
         }
         if (!ok) give_up(abort_flag, ERR_MMA);
       }
@@ -340,26 +340,37 @@ fp8_blockwise_many_rows_kernel(const __grid_constant__ CUtensorMap map_w, const 
           read_scales(sb + kt0 + SCALES_AHEAD, kt_count - kt0 - SCALES_AHEAD, vec4, sb_next);
         }
 #pragma unroll
-        for (int i = 0; i < SCALES_AHEAD; ++i) {
+        for (int i = 0; i < SCALES_AHEAD; i += 2) {
           if (kt0 + i >= kt_count) break;
-          ok = __all_sync(0xffffffffu, ptx::mbar_wait(&ctl->part_full[p], p_ph, abort_flag));
+          ok = __all_sync(0xffffffffu, ptx::mbar_wait(&ctl->pair_full[p], p_ph, abort_flag));
           if (!ok) break;
           if (active) {
+            // Sixteen columns at a time, so that the reads of the next ones are on their way during the multiplications.
             ptx::tc_fence_after_sync();
-            const float2 s2 = make_float2(s[i], s[i]);
-            uint32_t v[32];
-            ptx::tc_ld_32x32b_x32(taddr0 + p * TILE_N, v);
+            const uint32_t taddr = taddr0 + p * 2 * TILE_N;
+            const bool two = kt0 + i + 1 < kt_count;
+            const float2 s0 = make_float2(s[i], s[i]), s1 = make_float2(s[i + 1], s[i + 1]);
+            uint32_t va[16], vb[16];
+            ptx::tc_ld_32x32b_x16(taddr, va);
+            ptx::tc_ld_32x32b_x16(taddr + 16, vb);
             ptx::tc_wait_ld();
+            promote(va, s0, acc, 0);
+            if (two) ptx::tc_ld_32x32b_x16(taddr + TILE_N, va);
+            promote(vb, s0, acc, 8);
+            if (two) {
+              ptx::tc_wait_ld();
+              ptx::tc_ld_32x32b_x16(taddr + TILE_N + 16, vb);
+              promote(va, s1, acc, 0);
+              ptx::tc_wait_ld();
+            }
             ptx::tc_fence_before_sync();
             __syncwarp();
-            if (lane == 0) ptx::mbar_arrive(&ctl->part_empty[p]);   // the tensor core may overwrite this partial
-#pragma unroll
-            for (int j = 0; j < 16; ++j)
-              acc[j] = fma2(make_float2(__uint_as_float(v[2 * j]), __uint_as_float(v[2 * j + 1])), s2, acc[j]);
+            if (lane == 0) ptx::mbar_arrive(&ctl->pair_empty[p]);   // the tensor core may overwrite these partials
+            if (two) promote(vb, s1, acc, 8);
           } else if (lane == 0) {
-            ptx::mbar_arrive(&ctl->part_empty[p]);
+            ptx::mbar_arrive(&ctl->pair_empty[p]);
           }
-          if (++p == PARTS) { p = 0; p_ph ^= 1u; }
+          if (++p == PARTS / 2) { p = 0; p_ph ^= 1u; }
         }
       }
       if (!ok) break;
