@@ -738,7 +738,9 @@ int launch_as(const CallArgs& c) {
   if (attr[1].id == cudaLaunchAttributeProgrammaticStreamSerialization) cfg.numAttrs = 2;
   const int n_pairs = (c.n / TILE_N + 1) / 2;
   const int64_t used = c.num_experts < c.num_rows ? c.num_experts : c.num_rows;
-  const int group_light = weight_tiles_per_item(tunables().mm_item_k_steps, kt_count, used * n_pairs, info.sm_count);
+  const int most_light = weight_tiles_per_item(tunables().mm_item_k_steps, kt_count, used * n_pairs, info.sm_count);
+  const int light_items = (n_pairs + most_light - 1) / most_light;
+  const int group_light = (n_pairs + light_items - 1) / light_items;     // all of about the same length
   const int group_heavy = (group_light + 3) / 4;
   const int64_t max_items = ((c.num_rows + 128 * ITEM_ATOMS - 1) / (128 * ITEM_ATOMS) + c.num_experts) * (int64_t)n_pairs;
   int max_pairs = resident_pairs[dev & 63];
