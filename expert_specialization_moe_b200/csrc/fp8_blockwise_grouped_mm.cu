@@ -18,9 +18,8 @@
 //
 // This file: the few-rows kernel and the entry point.
 //   warp 0     producer: TMA loads of the weight tile and the token tile per K block
-//   warps 1, 2 MMA issue, one lane each: warp 1 (which also owns the TMEM allocation) takes the even K blocks, warp 2
-//              the odd ones — consecutive K blocks go to different partial buffers, and a tcgen05.mma costs its
-//              issuing thread ~90 cycles against 64 cycles of tensor time for a 128 x 128 x 32 MMA
+//   warps 1, 2 MMA issue, one thread each: warp 1 (which also owns the TMEM allocation) takes the even K blocks, warp 2
+//              the odd ones (consecutive K blocks go to different partial buffers); with short K warp 1 alone
 //   warps 3, 4 scale loaders, alternating chunks: sa[token, kb] * sb[tile, kb] for 8 K blocks at a time, transposed to
 //              [kb][token] in a ring of chunks, so that the epilogue reads one broadcast float4 per 4 tokens and never
 //              waits on global memory, whatever K is
@@ -47,6 +46,7 @@ constexpr int STAGE_BYTES = W_BYTES + TOK * TILE_K;
 constexpr int STAGES = 10;
 constexpr int NPART = 4;             // TMEM partial buffers
 constexpr uint32_t TMEM_COLS = NPART * TOK;
+constexpr int SHORT_K_BLOCKS = 4;    // fewer K blocks than this: short K
 constexpr int CH_KT = 8;             // K blocks per scale chunk
 constexpr int NCH = 4;               // scale chunks in the ring
 constexpr int CHUNK_FLOATS = CH_KT * TOK;
@@ -118,7 +118,12 @@ struct TileWalk {
 };
 
 // One CTA per SM; serves the experts with 1 .. FEW_ROWS rows.  First kernel of its call.
-template <typename OutT>
+// SHORT_K (fewer than four K blocks): ONE thread issues all MMAs, elected (a thread found by lane == 0 needs 550 cycles for
+// the four MMAs, waits and commits of a K block, an elected one 350, and K blocks then need no second thread).  Per call,
+// two threads and one: 4096 rows on 256 experts, n = 7168, k = 256 91.8 and 87.3 us; 1500 Zipf rows on 128, n = 4096, k = 384
+// 45.2 and 43.3; but 2000 rows on 256, n = 4096, k = 512 92.2 and 94.3; E = 256, n = 512, k = 7168 149.8 and 153.3: bound by
+// HBM, which a quicker turn-round of the stages does not suit.
+template <typename OutT, bool SHORT_K>
 __global__ void __launch_bounds__(THREADS, 1)
 fp8_blockwise_grouped_mm_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x16,
                                 const __grid_constant__ CUtensorMap map_x32, const float* scales_a,
@@ -215,10 +220,9 @@ fp8_blockwise_grouped_mm_kernel(const __grid_constant__ CUtensorMap map_w, const
       }
     }
   } else if (warp == 1 || warp == 2) {
-    // ------------------------------------------------------------------ MMA issue: K blocks alternate between the
-    // two lanes; g counts K blocks over all tiles of this CTA (stage = g mod STAGES, partial = g mod 4)
-    if (lane == 0) {
-      const int mine = warp - 1;
+    // ------------------------------------------------------------------ MMA issue; g counts K blocks over all tiles of this
+    // CTA (stage = g mod STAGES, partial = g mod 4).  With long K the K blocks alternate between the two threads.
+    auto issue = [&](int mine) {
       int g = 0;
       bool ok = true;
       TileWalk walk(block, blocks);
@@ -226,7 +230,7 @@ fp8_blockwise_grouped_mm_kernel(const __grid_constant__ CUtensorMap map_w, const
         const TileInfo& ti = walk.ti;
         const uint32_t idesc = ptx::make_idesc_f8(TILE_N, ti.n_mma);
         for (int kt = 0; kt < kt_count; ++kt, ++g) {
-          if ((g & 1) != mine) continue;
+          if (!SHORT_K && (g & 1) != mine) continue;
           const int s = g % STAGES;
           const uint32_t ph = (uint32_t)(g / STAGES) & 1u;
           const int p = g & (NPART - 1);
@@ -249,6 +253,11 @@ fp8_blockwise_grouped_mm_kernel(const __grid_constant__ CUtensorMap map_w, const
           atomicOr(&g_status, ERR_MMA);
         }
       }
+    };
+    if constexpr (SHORT_K) {
+      if (warp == 1 && ptx::elect_one()) issue(0);
+    } else {
+      if (lane == 0) issue(warp - 1);
     }
   } else if (warp < EPI_WARP0) {
     // ------------------------------------------------------------------ scale loaders: chunks alternate between the
@@ -405,8 +414,8 @@ static int tiles_per_item(int k) {
   return group < 1 ? 1 : group;
 }
 
-template <typename OutT>
-int launch_few_rows(const CallArgs& c) {
+template <typename OutT, bool SHORT_K>
+int launch_few_rows_as(const CallArgs& c) {
   DeviceInfo info;
   int rc = get_device_info(&info);
   if (rc != ES_B200_OK) return rc;
@@ -415,7 +424,7 @@ int launch_few_rows(const CallArgs& c) {
   if (rc == ES_B200_OK) rc = make_tensormap_u8_sw128(&map_x16, c.a, (uint64_t)c.num_rows, (uint64_t)c.k, 16);
   if (rc == ES_B200_OK) rc = make_tensormap_u8_sw128(&map_x32, c.a, (uint64_t)c.num_rows, (uint64_t)c.k, 32);
   if (rc != ES_B200_OK) return rc;
-  auto kernel = fp8_blockwise_grouped_mm_kernel<OutT>;
+  auto kernel = fp8_blockwise_grouped_mm_kernel<OutT, SHORT_K>;
   static bool configured[64] = {false};
   int dev = 0;
   ES_CUDA_TRY(cudaGetDevice(&dev));
@@ -440,6 +449,11 @@ int launch_few_rows(const CallArgs& c) {
   ES_CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, map_w, map_x16, map_x32, c.sa, c.sb, static_cast<OutT*>(c.d), c.ps, c.eo,
                                  c.num_experts, c.n, c.k, group));
   return ES_B200_OK;
+}
+
+template <typename OutT>
+int launch_few_rows(const CallArgs& c) {
+  return c.k / TILE_K < SHORT_K_BLOCKS ? launch_few_rows_as<OutT, true>(c) : launch_few_rows_as<OutT, false>(c);
 }
 
 int read_and_clear_status(uint32_t* out) {

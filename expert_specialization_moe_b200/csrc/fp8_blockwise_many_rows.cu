@@ -10,14 +10,14 @@
 // (a quarter less traffic) hold 64 accumulators a thread, spill, and were 14 % slower; two K blocks per stage and
 // hand-over 13 % slower; the kernel serving the experts of <= 32 rows too (128 MMA rows for a few tokens) 4-8 % slower
 // there than the few-rows kernel.
-// At that size the whole call takes 151 us back to back; with the tokens on N (this kernel's predecessor) 212.  Experts of
+// Two K blocks share a barrier round trip between the MMA thread and the promotion, whose TMEM reads overlap its
+// multiplications: with one K block per round trip and no overlap the promotion set the pace (780 cycles per K block; 585
+// now, of which 512 are the shared-memory pipe's), 165 us against 155.  The whole call took 212 with the tokens on N.  Experts of
 // 33 to 64 rows, whose MMAs are half empty, gain as well, at long K too (bound by HBM): E = 256, 48 rows, n = 512, k = 7168
 // 175 and 213 us; E = 32, 48 rows, n = 4096, k = 7168 167 and 242; E = 128, 33 rows, n = 4096, k = 2048 197 and 286.
 //
 //   warp 0     producer: TMA loads of the token tile and the weight tile per K block
-//   warps 1, 2 MMA issue, one lane each: warp 1 (which also owns the TMEM allocation) takes the even K blocks, warp 2
-//              the odd ones — consecutive K blocks go to different partial buffers, and a tcgen05.mma costs its
-//              issuing thread ~90 cycles
+//   warp 1     TMEM allocation; one elected thread issues the MMAs (warp 2 has no role)
 //   warp 3     work list: decodes this CTA's tiles one after the other and hands them to the other roles through a
 //              queue in shared memory (with every role decoding for itself a tile of two K blocks spent most of its
 //              time there)

@@ -14,7 +14,7 @@ constexpr int kHeavyMinRows = 113;       // tunable mm_heavy_min_rows
 // half the SMs, one per CTA pair, while there are the tiles for it (`tiles`: weight tiles of the call, an upper bound known
 // on the host): a call of few tiles is a matter of latency.  Measured without the rule -> with it: 3 rows on 8
 // experts, n = k = 1024: 8.7 -> 7.3 us; 8, 400 rows, n = 2048, k = 1024: 9.9 -> 8.6; 64, 300 rows, n = 896, k = 512: 11.1 ->
-// 12.5 (it cannot see which experts have rows).  Heavy experts get a quarter of it (their K steps take longer,
+// 12.5 (it cannot see which experts have rows; 11.1 since an expert's tiles are divided evenly).  Heavy experts get a quarter of it (their K steps take longer,
 // and an item must not be long at the end of a call).
 inline int weight_tiles_per_item(int item_k_steps, int k_steps_per_tile, int64_t tiles, int sm_count) {
   const int steps = item_k_steps < 1 ? 1 : item_k_steps;
