@@ -421,9 +421,9 @@ def bench_ep_layer(args, device, rank, world, dist):
                                        else "NCCL all-to-all dispatch/combine"),
                            "experts_per_gpu": e_local},
                 "clocks": clocks, "device_status": status,
-                # ours per step: route count + tables, dispatch-quant-push, unpack, 2 barriers, 1 + 1 GEMM launches,
-                # silu-quant, weighted sum (fused) / 2 quant kernels + 2 GEMMs (all-to-all path)
-                "gpu_launches": args.steps * ((20 if args.workload == "qwen3_ep_pipelined" else 10) if fused else 4)}
+                # ours per step: route count + tables, dispatch-quant-push, unpack, 2 barriers, 2 GEMMs (the first one with
+                # silu-quant in its epilogue), weighted sum (fused) / 2 quant kernels + 2 GEMMs (all-to-all path)
+                "gpu_launches": args.steps * ((18 if args.workload == "qwen3_ep_pipelined" else 9) if fused else 4)}
     del shard, x
     torch.cuda.empty_cache()
     return line

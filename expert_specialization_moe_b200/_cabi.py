@@ -35,6 +35,9 @@ def _declare(lib):
     lib.es_b200_mxfp8_grouped_mm.argtypes = [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p,
                                              c_void_p, c_void_p, c_int, c_int64, c_int, c_int, c_int64, c_void_p,
                                              c_size_t, c_void_p]
+    lib.es_b200_mxfp8_grouped_mm_silu_mul_quant.restype = c_int
+    lib.es_b200_mxfp8_grouped_mm_silu_mul_quant.argtypes = [c_void_p] * 9 + [c_int, c_int64, c_int, c_int, c_int64, c_void_p,
+                                                                             c_size_t, c_void_p]
     lib.es_b200_mxfp8_grouped_mm_scatter.restype = c_int
     lib.es_b200_mxfp8_grouped_mm_scatter.argtypes = [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p,
                                                      c_void_p, c_int, c_int64, c_int, c_int, c_int64, c_void_p,

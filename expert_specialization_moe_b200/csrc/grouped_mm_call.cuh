@@ -13,7 +13,8 @@ struct CallArgs {
   const void* b;
   const uint8_t* sfa;
   const uint8_t* sfb;
-  void* d;
+  void* d;                 // silu_mul_quant: the codes
+  uint8_t* scales;         // silu_mul_quant: their scale bytes
   const int32_t* ps;
   const int32_t* eo;
   const int32_t* bo;
@@ -31,6 +32,7 @@ struct CallArgs {
 
 int launch_bf16(const CallArgs& c);
 int launch_fp16(const CallArgs& c);
+int launch_silu_mul_quant(const CallArgs& c);   // n: gate rows per expert
 int read_and_clear_status(uint32_t* out);
 
 }  // namespace mm

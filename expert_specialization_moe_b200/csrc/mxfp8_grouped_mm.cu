@@ -28,15 +28,16 @@ namespace es_b200 {
 static int grouped_mm_impl(const void* a, const void* b, const uint8_t* sfa, const uint8_t* sfb, void* d, int out_dtype,
                            const int32_t* problem_sizes, const int32_t* expert_offsets,
                            const int32_t* blockscale_offsets, int num_experts, int64_t num_rows, int n, int k,
-                           int64_t sfa_rows, const RowScatter& scatter, void* scratch, size_t scratch_bytes,
-                           void* stream) {
+                           int64_t sfa_rows, const RowScatter& scatter, uint8_t* scales_out, void* scratch,
+                           size_t scratch_bytes, void* stream) {
+  // scales_out: silu(gate) * up requantised into d (codes) and scales_out; n is then the number of gate rows
   ES_REQUIRE(out_dtype == ES_B200_BF16 || out_dtype == ES_B200_FP16, "dtype must be kFloat16 or kBFloat16");
   ES_REQUIRE(k > 0 && k % 128 == 0, "k should align 128");
   ES_REQUIRE(n > 0 && n % 128 == 0, "n should align 128");
   ES_REQUIRE(num_experts >= 0 && num_experts <= ES_B200_MAX_EXPERTS, "Number of experts cannot exceed %d",
              ES_B200_MAX_EXPERTS);
   ES_REQUIRE(num_rows >= 0 && num_rows < (int64_t)1 << 31, "num_rows out of range");
-  ES_REQUIRE((int64_t)num_experts * n < (int64_t)1 << 31, "num_experts * n out of range");
+  ES_REQUIRE((int64_t)num_experts * n * (scales_out ? 2 : 1) < (int64_t)1 << 31, "num_experts * n out of range");
   if (num_experts == 0 || num_rows == 0) return ES_B200_OK;
   ES_REQUIRE(a && b && sfa && sfb && (d || scatter.meta) && problem_sizes && expert_offsets && blockscale_offsets,
              "null pointer argument");
@@ -57,6 +58,7 @@ static int grouped_mm_impl(const void* a, const void* b, const uint8_t* sfa, con
   c.sfa = sfa;
   c.sfb = sfb;
   c.d = d;
+  c.scales = scales_out;
   c.ps = problem_sizes;
   c.eo = expert_offsets;
   c.bo = blockscale_offsets;
@@ -73,6 +75,7 @@ static int grouped_mm_impl(const void* a, const void* b, const uint8_t* sfa, con
   c.overlap.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   c.overlap.val.programmaticStreamSerializationAllowed = 1;
   c.stream = static_cast<cudaStream_t>(stream);
+  if (scales_out != nullptr) return mm::launch_silu_mul_quant(c);
   return out_dtype == ES_B200_BF16 ? mm::launch_bf16(c) : mm::launch_fp16(c);
 }
 }  // namespace es_b200
@@ -84,7 +87,21 @@ extern "C" int es_b200_mxfp8_grouped_mm(const void* a, const void* b, const uint
   es_b200::NvtxRange nvtx_range("es_b200_mxfp8_grouped_mm");
   es_b200::RowScatter dense = {};
   return es_b200::grouped_mm_impl(a, b, sfa, sfb, d, out_dtype, problem_sizes, expert_offsets, blockscale_offsets,
-                                  num_experts, num_rows, n, k, sfa_rows, dense, scratch, scratch_bytes, stream);
+                                  num_experts, num_rows, n, k, sfa_rows, dense, nullptr, scratch, scratch_bytes, stream);
+}
+
+extern "C" int es_b200_mxfp8_grouped_mm_silu_mul_quant(const void* a, const void* b, const uint8_t* sfa, const uint8_t* sfb,
+                                                       void* quant_output, uint8_t* scale_factor,
+                                                       const int32_t* problem_sizes, const int32_t* expert_offsets,
+                                                       const int32_t* blockscale_offsets, int num_experts,
+                                                       int64_t num_rows, int inter, int k, int64_t sfa_rows, void* scratch,
+                                                       size_t scratch_bytes, void* stream) {
+  es_b200::NvtxRange nvtx_range("es_b200_mxfp8_grouped_mm_silu_mul_quant");
+  using namespace es_b200;
+  RowScatter dense = {};
+  ES_REQUIRE(num_experts == 0 || num_rows == 0 || scale_factor != nullptr, "null pointer argument");
+  return grouped_mm_impl(a, b, sfa, sfb, quant_output, ES_B200_BF16, problem_sizes, expert_offsets, blockscale_offsets,
+                         num_experts, num_rows, inter, k, sfa_rows, dense, scale_factor, scratch, scratch_bytes, stream);
 }
 
 extern "C" int es_b200_mxfp8_grouped_mm_scatter(const void* a, const void* b, const uint8_t* sfa, const uint8_t* sfb,
@@ -109,7 +126,7 @@ extern "C" int es_b200_mxfp8_grouped_mm_scatter(const void* a, const void* b, co
     sc.base[i] = const_cast<void*>(peer_out[i]);
   }
   return grouped_mm_impl(a, b, sfa, sfb, nullptr, out_dtype, problem_sizes, expert_offsets, blockscale_offsets,
-                         num_experts, num_rows, n, k, sfa_rows, sc, scratch, scratch_bytes, stream);
+                         num_experts, num_rows, n, k, sfa_rows, sc, nullptr, scratch, scratch_bytes, stream);
 }
 
 extern "C" int es_b200_check_status(void* stream, uint32_t* raw_status) {

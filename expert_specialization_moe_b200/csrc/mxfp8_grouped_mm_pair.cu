@@ -24,6 +24,12 @@
 //     itself: 2000 cycles per item);
 //   * the output leaves as 16-byte stores: matrix fragments from TMEM (16x256b), transposed by stmatrix.
 //
+// GATED (es_b200_mxfp8_grouped_mm_silu_mul_quant): silu(gate) * up and the requantisation in the epilogue.  A work item is 256
+// gate rows, the 256 up rows of the same outputs, and up to 192 token rows; a K step has two weight slots and one token slot,
+// gate goes to the first accumulator, up to the second, so that a thread finds both of an output in the same lane and column,
+// a warp its 32 outputs of a scale block.  The gate_up product is neither rounded to 16 bits nor written: 128 x 1024 rows,
+// inter = 768, k = 2048: 336 us (each kernel timed by a profiler) where the GEMM took 281 and the SiLU kernel 126.
+//
 //   warp 0      producer of weights and scales (both CTAs): per K step one thread loads its 128 weight rows, their scale atom
 //               and the item's token scale atoms; all bytes are credited to the leader CTA's barrier
 //   warp 1      TMEM allocation; in the leader CTA one thread issues the K step's scale copies (tcgen05.cp) and MMAs
@@ -36,6 +42,7 @@
 #include "common.cuh"
 #include "epilogue.cuh"
 #include "grouped_mm_call.cuh"
+#include "mxfp8_quant_math.cuh"
 #include "sm100_ptx.cuh"
 #include "tensormap.cuh"
 #include "work_items.cuh"
@@ -56,15 +63,18 @@ constexpr int X_SLOT = (SUB_TILE / 2) * TILE_K;        // 12288: this CTA's half
 static_assert(W_SLOT % 1024 == 0 && X_SLOT % 1024 == 0, "128-byte swizzle atoms are 1024 bytes");
 // The two rings share what shared memory there is: W weight slots (one per K step), X token slots (one per sub-tile of a K
 // step).  Few rows per expert: seven K steps in flight.  Many: eight token slots are four K steps of two sub-tiles.
-struct FewRows { static constexpr int W = 7, X = 7; };
-struct ManyRows { static constexpr int W = 6, X = 8; };
+// Gated: eight weight and five token slots are four K steps of gate and up.
+struct FewRows { static constexpr int W = 7, X = 7; static constexpr bool GATED = false; };
+struct ManyRows { static constexpr int W = 6, X = 8; static constexpr bool GATED = false; };
+struct Gated { static constexpr int W = 8, X = 5; static constexpr bool GATED = true; };
 constexpr uint32_t TMEM_COLS = 512;
 constexpr uint32_t ACC_COLS = 192;        // accumulators at columns [0,192) and [192,384)
 constexpr uint32_t SF_COL0 = 384;         // per weight slot 16 columns: 4 (weight scales) + 12 (token scales)
 constexpr uint32_t SF_SLOT_COLS = 16;
-static_assert(SF_COL0 + FewRows::W * SF_SLOT_COLS <= TMEM_COLS && ManyRows::W <= FewRows::W, "TMEM budget");
+static_assert(SF_COL0 + Gated::W * SF_SLOT_COLS <= TMEM_COLS && FewRows::W <= Gated::W && ManyRows::W <= Gated::W, "TMEM budget");
+static_assert(Gated::W % 2 == 0, "gate in the even slots, up in the odd ones");
 
-constexpr int MAX_W = 7, MAX_X = 8;
+constexpr int MAX_W = 8, MAX_X = 8;
 constexpr uint32_t ERR_PRODUCER = 0x10u, ERR_MMA = 0x20u, ERR_EPILOGUE = 0x40u, ERR_SCHEDULER = 0x100u;
 constexpr int W_WARP = 0, MMA_WARP = 1, SCHED_WARP = 2, X_WARP = 3, EPI_WARP0 = 4;
 constexpr int EPI_WARPS = 12;                              // 4 TMEM lane quadrants x 3 warps
@@ -76,7 +86,8 @@ constexpr int Q_CONSUMERS = 2 * (2 + EPI_WARPS) + 1;
 struct Item {      // one work item as the scheduler hands it out
   int valid;       // token rows of the item (<= 384); -1: no more work
   int row0;        // first token row in a / d
-  int n01;         // MMA N of the two sub-tiles, n0 | n1 << 16 (multiples of 16; n1 == 0: one sub-tile)
+  int n01;         // MMA N of the two sub-tiles, n0 | n1 << 16 (multiples of 16; n1 == 0: one sub-tile); gated: N | first
+                   // column of the token scales in their atom << 16
   int np0;         // first weight pair
   int units;       // weight pairs of the item
   int e;           // expert
@@ -105,7 +116,7 @@ template <class S>
 constexpr size_t smem_bytes() {
   return 1024 + (size_t)S::W * W_SLOT + (size_t)S::X * X_SLOT + EPI_WARPS * EPI_BYTES_PER_WARP + sizeof(SharedCtl);
 }
-static_assert(smem_bytes<FewRows>() <= 232448 && smem_bytes<ManyRows>() <= 232448, "shared memory of one CTA per SM");
+static_assert(smem_bytes<FewRows>() <= 232448 && smem_bytes<ManyRows>() <= 232448 && smem_bytes<Gated>() <= 232448, "shared memory of one CTA per SM");
 
 __device__ uint32_t g_status = 0;
 
@@ -118,11 +129,12 @@ struct Maps {
 };
 
 struct KernelArgs {
-  void* d;
+  void* d;                   // gated: the e4m3 codes
+  uint8_t* scales;           // gated: their scale bytes
   const int* problem_sizes;
   const int* expert_offsets;
   const int* blockscale_offsets;
-  int num_experts, n, k;
+  int num_experts, n, k;     // n: weight rows per expert (gated: gate rows, as many up rows follow them)
   int heavy_min;             // experts with at least this many rows come first in the work list
   int group_heavy, group_light;   // weight pairs per work item
   uint32_t* counters;
@@ -183,6 +195,32 @@ __device__ __forceinline__ void pack_chunk(const uint32_t (&lo)[16], const uint3
     held[4 * g + 3] = pack_pair_from_f32<OutT>(__uint_as_float(hi[4 * g + 2]), __uint_as_float(hi[4 * g + 3]));
   }
 }
+// silu(g) * u in fp32 (hardware exponential and quotient: a few units in the last place, against 2^-4 of an e4m3 code)
+__device__ __forceinline__ float silu_mul(float g, float u) { return __fdividef(g, 1.0f + __expf(-g)) * u; }
+
+// gated: a chunk's fp32 fragments, and silu of them times the up accumulator's
+__device__ __forceinline__ void read_fragments(uint32_t taddr, float (&v)[32]) {
+  uint32_t lo[16], hi[16];
+  ptx::tc_ld_16x256b_x4(taddr, lo);
+  ptx::tc_ld_16x256b_x4(taddr + (16u << 16), hi);
+  ptx::tc_wait_ld();
+#pragma unroll
+  for (int i = 0; i < 16; ++i) {
+    v[i] = __uint_as_float(lo[i]);
+    v[16 + i] = __uint_as_float(hi[i]);
+  }
+}
+__device__ __forceinline__ void times_up(uint32_t taddr, float (&v)[32]) {
+  uint32_t lo[16], hi[16];
+  ptx::tc_ld_16x256b_x4(taddr, lo);
+  ptx::tc_ld_16x256b_x4(taddr + (16u << 16), hi);
+  ptx::tc_wait_ld();
+#pragma unroll
+  for (int i = 0; i < 16; ++i) {
+    v[i] = silu_mul(v[i], __uint_as_float(lo[i]));
+    v[16 + i] = silu_mul(v[16 + i], __uint_as_float(hi[i]));
+  }
+}
 template <typename OutT>
 __device__ __forceinline__ void read_chunk(uint32_t taddr, uint32_t (&held)[16]) {
   uint32_t lo[16], hi[16];
@@ -203,11 +241,56 @@ __device__ __forceinline__ void read_two_chunks(uint32_t taddr0, uint32_t taddr1
   pack_chunk<OutT>(lo1, hi1, held1);
 }
 
+// Quantises a 32-token chunk of 32 outputs (one scale block per token) and stores codes and scale bytes.  v: fp32 fragments,
+// v[4 g + 2 h + j] the value of output lane / 4 + 8 h, token 8 g + 2 (lane % 4) + j (h = 0, 1), v[16 + ...] the outputs 16
+// further.  `codes`: first token, first output of the chunk; `scales`: the byte of token 0 of the item's atom rows and this
+// block.  Arithmetic as in mxfp8_quant_math.cuh, from fp32 values.
+__device__ __forceinline__ void store_chunk_quantised(const float (&v)[32], uint32_t stage, int tok, int valid, int sf_row,
+                                                      uint8_t* codes, int64_t ld, uint8_t* scales, int kt_out, int lane) {
+#pragma unroll
+  for (int p = 0; p < 2; ++p) {
+    if (tok + p * 16 >= valid) break;       // warp-uniform
+#pragma unroll
+    for (int gl = 0; gl < 2; ++gl) {
+      const int g = p * 2 + gl;
+      float inv[2];
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        float m = fmaxf(fmaxf(fabsf(v[4 * g + j]), fabsf(v[4 * g + 2 + j])),
+                        fmaxf(fabsf(v[16 + 4 * g + j]), fabsf(v[16 + 4 * g + 2 + j])));
+        m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 4));
+        m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 8));
+        m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 16));
+        const uint32_t sf = __nv_cvt_float_to_e8m0(m * rcp_approx_ftz(448.0f), __NV_SATFINITE, cudaRoundPosInf);
+        const uint32_t inv_bits = sf == 0 ? 0x7f800000u : sf == 255u ? 0x7fffffffu : (254u - sf) << 23;
+        inv[j] = m != 0.f ? __uint_as_float(inv_bits) : 0.0f;
+        const int t = tok + 8 * g + 2 * (lane & 3) + j;
+        if ((lane >> 2) == g && t < valid) scales[scale_word_offset(sf_row + t, kt_out)] = (uint8_t)sf;
+      }
+      const uint32_t row = stage + (gl * 8 + 2 * (lane & 3)) * 32 + (lane >> 2);
+#pragma unroll
+      for (int h = 0; h < 4; ++h) {         // outputs lane / 4 + 8 h
+        const int i = (h >> 1) * 16 + 4 * g + (h & 1) * 2;
+        const uint32_t c = e4m3x4(make_float2(v[i] * inv[0], v[i + 1] * inv[1]), make_float2(0.f, 0.f));
+        ptx::st_shared_u8(row + 8 * h, c);
+        ptx::st_shared_u8(row + 32 + 8 * h, c >> 8);
+      }
+    }
+    __syncwarp();
+    const uint4 val = ptx::ld_shared_16B(stage + lane * 16);
+    const int t = tok + p * 16 + (lane >> 1);
+    if (t < valid) *reinterpret_cast<uint4*>(codes + (int64_t)(t - tok) * ld + (lane & 1) * 16) = val;
+    __syncwarp();
+  }
+}
+
 template <typename OutT, class S>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
 mxfp8_grouped_mm_pair_kernel(const __grid_constant__ Maps maps, const __grid_constant__ KernelArgs args,
                              const __grid_constant__ RowScatter scatter) {
   constexpr int W_STAGES = S::W, X_STAGES = S::X;
+  constexpr bool GATED = S::GATED;
+  constexpr int TILE_ROWS = GATED ? SUB_TILE : 128 * ITEM_ATOMS;     // token rows of a work item at most
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = ptx::align1024(smem_raw);
   uint8_t* x_ring = smem + (size_t)W_STAGES * W_SLOT;
@@ -222,7 +305,7 @@ mxfp8_grouped_mm_pair_kernel(const __grid_constant__ Maps maps, const __grid_con
 
   if (threadIdx.x == SCHED_WARP * 32) {
     for (int s = 0; s < W_STAGES; ++s) {
-      ptx::mbar_init(&ctl->full[s], 2);
+      ptx::mbar_init(&ctl->full[s], GATED && (s & 1) ? 1 : 2);
       ptx::mbar_init(&ctl->empty[s], 1);
     }
     for (int a = 0; a < 2; ++a) {
@@ -272,8 +355,8 @@ mxfp8_grouped_mm_pair_kernel(const __grid_constant__ Maps maps, const __grid_con
         facts[2 * ES_B200_MAX_EXPERTS + e] = bs;
         if (m > 0) {
           if ((bs & 127) != 0) atomicOr(&g_status, ERR_SCALE_OFFSET_BIT);
-          else if (m >= args.heavy_min) h[i] = (int)(((int64_t)m + 128 * ITEM_ATOMS - 1) / (128 * ITEM_ATOMS)) * heavy_groups;
-          else l[i] = (int)(((int64_t)m + 128 * ITEM_ATOMS - 1) / (128 * ITEM_ATOMS)) * light_groups;
+          else if (m >= args.heavy_min) h[i] = (int)(((int64_t)m + TILE_ROWS - 1) / TILE_ROWS) * heavy_groups;
+          else l[i] = (int)(((int64_t)m + TILE_ROWS - 1) / TILE_ROWS) * light_groups;
         }
       }
     }
@@ -375,26 +458,34 @@ mxfp8_grouped_mm_pair_kernel(const __grid_constant__ Maps maps, const __grid_con
           const int sf_first = (t == pair ? facts[2 * ES_B200_MAX_EXPERTS + e] : args.blockscale_offsets[e]) >> 7;
           const int groups = (n_pairs + group - 1) / group;
           const int atoms = (m + 127) >> 7;
-          const int tiles = (atoms + ITEM_ATOMS - 1) / ITEM_ATOMS;
+          const int tiles = (m + TILE_ROWS - 1) / TILE_ROWS;
           // Consecutive items run at the same time on different CTA pairs and share one operand in L2 while they sweep
           // the other: the swept operand should be the SMALLER one.
           int tt, g;
           if (tiles == 1) { tt = 0; g = i; }
           else if (m <= n) { g = i / tiles; tt = i - g * tiles; }
           else { tt = i / groups; g = i - tt * groups; }
-          const int base = atoms / tiles, rem = atoms - base * tiles;      // the atoms in tiles of base or base + 1
-          const int atom0 = tt * base + (tt < rem ? tt : rem);
-          const int rows = (base + (tt < rem ? 1 : 0)) * 128;
-          const int left = m - atom0 * 128;
+          int first, rows, hi;
+          if (GATED) {             // tiles of as many 64 rows as divide them evenly, 192 at most
+            rows = (((m + tiles - 1) / tiles) + 63) & ~63;
+            first = tt * rows;
+            hi = (first >> 5) & 3;
+          } else {                 // the atoms in tiles of base or base + 1
+            const int base = atoms / tiles, rem = atoms - base * tiles;
+            first = (tt * base + (tt < rem ? tt : rem)) * 128;
+            rows = (base + (tt < rem ? 1 : 0)) * 128;
+            hi = 0;
+          }
+          const int left = m - first;
           it.valid = left < rows ? left : rows;
-          it.row0 = row_first + atom0 * 128;
+          it.row0 = row_first + first;
           const int n0 = it.valid <= SUB_TILE ? (it.valid + 15) & ~15 : it.valid <= 256 ? 128 : SUB_TILE;
-          const int n1 = it.valid > n0 ? (it.valid - n0 + 15) & ~15 : 0;
-          it.n01 = n0 | (n1 << 16);
+          if (!GATED) hi = it.valid > n0 ? (it.valid - n0 + 15) & ~15 : 0;
+          it.n01 = n0 | (hi << 16);
           it.np0 = g * group;
           it.units = n_pairs - it.np0 < group ? n_pairs - it.np0 : group;
           it.e = e;
-          it.sfx_row = sf_first + atom0;
+          it.sfx_row = sf_first + (first >> 7);
           it.one_tile = tiles == 1;
         }
         if (!__all_sync(0xffffffffu, ptx::mbar_wait(&ctl->q_empty[qs], qph ^ 1u, abort_flag))) {
@@ -425,21 +516,22 @@ mxfp8_grouped_mm_pair_kernel(const __grid_constant__ Maps maps, const __grid_con
         Item it;
         ok = next_item_one(&it);
         if (!ok || it.valid < 0) break;
-        const bool three = it.valid > 128;
+        const bool three = GATED || it.valid > 128;
         const uint32_t mine = W_BYTES + SF_BYTES + (three ? SFX_BYTES : SF_BYTES);
         const uint64_t hint = it.one_tile ? ptx::kL2EvictFirst : ptx::kL2EvictLast;
         const CUtensorMap* sfx_map = three ? &maps.sfx3 : &maps.sfx1;
+        const int e_tile = it.e * n_tiles * (GATED ? 2 : 1);
         for (int u = 0; ok && u < it.units; ++u) {
           const int nt = (it.np0 + u) * 2 + (int)rank;
           const bool have = nt < n_tiles;          // n / 128 odd: the last pair's second half does not exist
-          const uint32_t tx = mine * ((it.np0 + u) * 2 + 1 < n_tiles ? 2u : 1u);
-          const int w_row = it.e * n + nt * TILE_N;
-          const int sfw_atom = (it.e * n_tiles + nt) * kt_count;
+          const uint32_t halves = (it.np0 + u) * 2 + 1 < n_tiles ? 2u : 1u;
+          const int w_row = (e_tile + nt) * TILE_N;
+          const int sfw_atom = (e_tile + nt) * kt_count;
           for (int kt = 0; kt < kt_count; ++kt) {
             ok = ptx::mbar_wait(&ctl->empty[s], ph ^ 1u, abort_flag);
             if (!ok) break;
             uint8_t* slot = smem + (size_t)s * W_SLOT;
-            if (rank == 0) ptx::mbar_arrive_expect_tx(&ctl->full[s], tx);
+            if (rank == 0) ptx::mbar_arrive_expect_tx(&ctl->full[s], mine * halves);
             if (have) {
               ptx::tma_load_2d_pair_hint(slot, &maps.w, &ctl->full[s], kt * TILE_K, w_row, hint);
               ptx::tma_load_2d_pair_hint(slot + W_BYTES, &maps.sfw, &ctl->full[s], 0, sfw_atom + kt, ptx::kL2EvictNormal);
@@ -447,6 +539,18 @@ mxfp8_grouped_mm_pair_kernel(const __grid_constant__ Maps maps, const __grid_con
                                          ptx::kL2EvictNormal);
             }
             if (++s == W_STAGES) { s = 0; ph ^= 1u; }
+            if constexpr (GATED) {                 // the up rows' slot (both slots of a step are freed together)
+              ok = ptx::mbar_wait(&ctl->empty[s], ph ^ 1u, abort_flag);
+              if (!ok) break;
+              slot = smem + (size_t)s * W_SLOT;
+              if (rank == 0) ptx::mbar_arrive_expect_tx(&ctl->full[s], (W_BYTES + SF_BYTES) * halves);
+              if (have) {
+                ptx::tma_load_2d_pair_hint(slot, &maps.w, &ctl->full[s], kt * TILE_K, w_row + n, hint);
+                ptx::tma_load_2d_pair_hint(slot + W_BYTES, &maps.sfw, &ctl->full[s], 0, sfw_atom + n_tiles * kt_count + kt,
+                                           ptx::kL2EvictNormal);
+              }
+              if (++s == W_STAGES) { s = 0; ph ^= 1u; }
+            }
           }
         }
       }
@@ -459,15 +563,16 @@ mxfp8_grouped_mm_pair_kernel(const __grid_constant__ Maps maps, const __grid_con
     // weight slot.  A step further back than W_STAGES is not waited for but the one W_STAGES back is, whose weight slot this
     // step takes anyway: a parity wait cannot tell a phase from the one two further.
     if (ptx::elect_one()) {
-      int s = 0, x = 0, step = 0;
+      constexpr int PER_STEP = GATED ? 2 : 1, STEPS = W_STAGES / PER_STEP;     // weight slots per K step; K steps in the ring
+      int s = 0, x = 0, step = 0;                     // s: weight slots of the step in K steps
       uint32_t ph = 0;
-      for (int i = 0; i < X_STAGES; ++i) ctl->x_user[i] = -W_STAGES;
+      for (int i = 0; i < X_STAGES; ++i) ctl->x_user[i] = -STEPS;
       bool ok = true;
       while (ok) {
         Item it;
         ok = next_item_one(&it);
         if (!ok || it.valid < 0) break;
-        const int n0 = it.n01 & 0xffff, n1 = it.n01 >> 16;
+        const int n0 = it.n01 & 0xffff, n1 = GATED ? 0 : it.n01 >> 16;
         const int xi0 = box_index(n0 >> 1), xi1 = box_index(n1 >> 1);
         const CUtensorMap* map0 = &maps.x[xi0];
         const CUtensorMap* map1 = &maps.x[xi1];
@@ -477,23 +582,23 @@ mxfp8_grouped_mm_pair_kernel(const __grid_constant__ Maps maps, const __grid_con
           for (int kt = 0; kt < kt_count; ++kt) {
             const int x1 = x + 1 == X_STAGES ? 0 : x + 1;
             int back = step - ctl->x_user[n1 ? x1 : x];      // the later of the slots' users, in steps back
-            if (back > W_STAGES) back = W_STAGES;
+            if (back > STEPS) back = STEPS;
             if (back <= step) {
               const int us = s - back;                       // its weight slot, of this revolution or of the one before
-              ok = ptx::mbar_wait(&ctl->empty[us < 0 ? us + W_STAGES : us], us < 0 ? ph ^ 1u : ph, abort_flag);
+              ok = ptx::mbar_wait(&ctl->empty[(us < 0 ? us + STEPS : us) * PER_STEP + PER_STEP - 1], us < 0 ? ph ^ 1u : ph, abort_flag);
               if (!ok) break;
             }
-            if (rank == 0) ptx::mbar_arrive_expect_tx(&ctl->full[s], tx);
-            ptx::tma_load_2d_pair_hint(x_ring + (size_t)x * X_SLOT, map0, &ctl->full[s], kt * TILE_K, row0, ptx::kL2EvictLast);
+            if (rank == 0) ptx::mbar_arrive_expect_tx(&ctl->full[s * PER_STEP], tx);
+            ptx::tma_load_2d_pair_hint(x_ring + (size_t)x * X_SLOT, map0, &ctl->full[s * PER_STEP], kt * TILE_K, row0, ptx::kL2EvictLast);
             ctl->x_user[x] = step;
             x = x1;
             if (n1) {
-              ptx::tma_load_2d_pair_hint(x_ring + (size_t)x * X_SLOT, map1, &ctl->full[s], kt * TILE_K, row1, ptx::kL2EvictLast);
+              ptx::tma_load_2d_pair_hint(x_ring + (size_t)x * X_SLOT, map1, &ctl->full[s * PER_STEP], kt * TILE_K, row1, ptx::kL2EvictLast);
               ctl->x_user[x] = step;
               if (++x == X_STAGES) x = 0;
             }
             ++step;
-            if (++s == W_STAGES) { s = 0; ph ^= 1u; }
+            if (++s == STEPS) { s = 0; ph ^= 1u; }
           }
         }
       }
@@ -511,8 +616,10 @@ mxfp8_grouped_mm_pair_kernel(const __grid_constant__ Maps maps, const __grid_con
         Item it;
         ok = next_item_one(&it);
         if (!ok || it.valid < 0) break;
-        const int n0 = it.n01 & 0xffff, n1 = it.n01 >> 16;
-        const int atoms = (it.valid + 127) >> 7;
+        // gated: both accumulators have the same token rows, the second one the up rows
+        const int n0 = it.n01 & 0xffff, n1 = GATED ? n0 : it.n01 >> 16;
+        const int sf_col = GATED ? it.n01 >> 16 : 0;      // first column of the token scales
+        const int atoms = (it.valid + sf_col * 32 + 127) >> 7;
         const uint32_t idesc0 = ptx::make_idesc_mxf8(2 * TILE_N, n0, 0, 0), idesc1 = ptx::make_idesc_mxf8(2 * TILE_N, n1, 0, 0);
         for (int u = 0; ok && u < it.units; ++u) {
           const uint32_t a0 = cnt & 1u, a1 = a0 ^ 1u;
@@ -534,23 +641,32 @@ mxfp8_grouped_mm_pair_kernel(const __grid_constant__ Maps maps, const __grid_con
 #pragma unroll
             for (uint32_t j = 0; j < 4; ++j)
               ptx::tc_mma_mxf8_pair(tmem_base + a0 * ACC_COLS, a_desc + 2 * j, b_desc + 2 * j, idesc0 | (j << 4) | (j << 29),
-                                    sfw_t | (j << 30), sfx_t | (j << 30), (kt | j) != 0 ? 1u : 0u);
+                                    sfw_t | (j << 30), (sfx_t + sf_col) | (j << 30), (kt | j) != 0 ? 1u : 0u);
             return true;
           };
-          // the MMAs of sub-tile 1 of the K step in weight slot sl, token slot xl
-          auto second_half = [&](int kt, int sl, int xl) {
-            const uint32_t sfw_t = tmem_base + SF_COL0 + sl * SF_SLOT_COLS;
-            const uint32_t sfx_t = sfw_t + 4 + (n0 >> 5);      // sub-tile 1 starts n0 rows into the token scales
-            const uint64_t a_desc = ptx::make_desc_k_sw128(smem_base + sl * W_SLOT);
+          // the MMAs of sub-tile 1 of the K step in weight slot sl, token slot xl (gated: of the up rows, in the slot behind)
+          auto second_half = [&](int kt, int sl, int xl, uint32_t phl) {
+            const int wl = GATED ? sl + 1 : sl;
+            if (GATED) {
+              if (!ptx::mbar_wait(&ctl->full[wl], phl, abort_flag)) return false;
+              ptx::tc_fence_after_sync();
+              ptx::tc_cp_sf_pair(tmem_base + SF_COL0 + wl * SF_SLOT_COLS, ptx::make_desc_sf(smem_base + wl * W_SLOT + W_BYTES));
+            }
+            const uint32_t sfw_t = tmem_base + SF_COL0 + wl * SF_SLOT_COLS;
+            // sub-tile 1 starts n0 rows into the token scales
+            const uint32_t sfx_t = tmem_base + SF_COL0 + sl * SF_SLOT_COLS + 4 + (GATED ? sf_col : n0 >> 5);
+            const uint64_t a_desc = ptx::make_desc_k_sw128(smem_base + wl * W_SLOT);
             const uint64_t b_desc = ptx::make_desc_k_sw128(x_base + xl * X_SLOT);
 #pragma unroll
             for (uint32_t j = 0; j < 4; ++j)
               ptx::tc_mma_mxf8_pair(tmem_base + a1 * ACC_COLS, a_desc + 2 * j, b_desc + 2 * j, idesc1 | (j << 4) | (j << 29),
                                     sfw_t | (j << 30), sfx_t | (j << 30), (kt | j) != 0 ? 1u : 0u);
             ptx::tc_commit_pair(&ctl->empty[sl], 3);
+            if (GATED) ptx::tc_commit_pair(&ctl->empty[wl], 3);
+            return true;
           };
           auto next_x = [&](int i) { return i + 1 == X_STAGES ? 0 : i + 1; };
-          auto next_step = [&]() { if (++s == W_STAGES) { s = 0; ph ^= 1u; } };
+          auto next_step = [&]() { if ((s += GATED ? 2 : 1) == W_STAGES) { s = 0; ph ^= 1u; } };
           if (n1 == 0) {
             for (int kt = 0; ok && kt < kt_count; ++kt) {
               ok = first_half(kt);
@@ -567,14 +683,18 @@ mxfp8_grouped_mm_pair_kernel(const __grid_constant__ Maps maps, const __grid_con
             // accumulator 1 and wanted back as much earlier, which hides the time that the epilogue takes to empty it.
             for (int kt = 0; ok && kt < kt_count;) {
               const bool two = kt + 1 < kt_count && (kt == 0 || kt + 2 == kt_count);
-              const int s0 = s, x0 = next_x(x);
+              // (gated: gate and up multiply the same token slot)
+              const int s0 = s, x0 = GATED ? x : next_x(x);
+              const uint32_t ph0 = ph;
               ok = first_half(kt);
               if (!ok) break;
               x = next_x(x0);
               next_step();
-              int s1 = s, x1 = 0;
+              const int s1 = s;
+              const uint32_t ph1 = ph;
+              int x1 = 0;
               if (two) {
-                x1 = next_x(x);
+                x1 = GATED ? x : next_x(x);
                 ok = first_half(kt + 1);
                 if (!ok) break;
                 x = next_x(x1);
@@ -586,8 +706,8 @@ mxfp8_grouped_mm_pair_kernel(const __grid_constant__ Maps maps, const __grid_con
                 if (!ok) break;
                 ptx::tc_fence_after_sync();
               }
-              second_half(kt, s0, x0);
-              if (two) second_half(kt + 1, s1, x1);
+              ok = second_half(kt, s0, x0, ph0) && (!two || second_half(kt + 1, s1, x1, ph1));
+              if (!ok) break;
               kt += two ? 2 : 1;
             }
             if (!ok) break;
@@ -617,13 +737,45 @@ mxfp8_grouped_mm_pair_kernel(const __grid_constant__ Maps maps, const __grid_con
       Item it;
       ok = next_item(&it);
       if (!ok || it.valid < 0) break;
-      const int n0 = it.n01 & 0xffff, n1 = it.n01 >> 16;
+      const int n0 = it.n01 & 0xffff, n1 = GATED ? n0 : it.n01 >> 16;
       for (int u = 0; u < it.units; ++u) {
         const int nt = (it.np0 + u) * 2 + (int)rank;
         const int col_off = nt * TILE_N + q * 32;
         const uint32_t a0 = cnt & 1u, a1 = a0 ^ 1u;
         const uint32_t p0 = (cnt >> 1) & 1u, p1 = ((cnt + 1) >> 1) & 1u;
         const int c0 = turn * 32, c1 = c0 + 96;
+        if constexpr (GATED) {
+          // this warp's chunks of the gate accumulator, then each one's up values: silu(gate) * up in their place
+          float act0[32], act1[32];
+          ok = __all_sync(0xffffffffu, ptx::mbar_wait(&ctl->acc_full[a0], p0, abort_flag));
+          if (!ok) break;
+          ptx::tc_fence_after_sync();
+          const uint32_t t0 = lane_base + a0 * ACC_COLS, t1 = lane_base + a1 * ACC_COLS;
+          if (c0 < n0) read_fragments(t0 + c0, act0);
+          if (c1 < n0) read_fragments(t0 + c1, act1);
+          ptx::tc_fence_before_sync();
+          __syncwarp();
+          if (lane == 0) ptx::mbar_arrive_cluster_relaxed(&ctl->acc_empty[a0], 0);
+          ok = __all_sync(0xffffffffu, ptx::mbar_wait(&ctl->acc_full[a1], p1, abort_flag));
+          if (!ok) break;
+          ptx::tc_fence_after_sync();
+          if (c0 < n0) times_up(t1 + c0, act0);
+          if (c1 < n0) times_up(t1 + c1, act1);
+          ptx::tc_fence_before_sync();
+          __syncwarp();
+          if (lane == 0) ptx::mbar_arrive_cluster_relaxed(&ctl->acc_empty[a1], 0);
+          if (nt < n_tiles) {
+            // scale block of these 32 outputs: K block col_off / 32 of the next GEMM's operand
+            uint8_t* codes = static_cast<uint8_t*>(args.d) + (int64_t)it.row0 * n + col_off;
+            uint8_t* scales = args.scales + ((int64_t)it.sfx_row * n_tiles + nt) * 512 + q;
+            const int sf_row = (it.n01 >> 16) * 32;
+            if (c0 < n0) store_chunk_quantised(act0, stage, c0, it.valid, sf_row, codes + (int64_t)c0 * n, n, scales, n_tiles, lane);
+            if (c1 < n0) store_chunk_quantised(act1, stage, c1, it.valid, sf_row, codes + (int64_t)c1 * n, n, scales, n_tiles, lane);
+          }
+          cnt += 2;
+          turn = turn == 0 ? 2 : turn - 1;
+          continue;
+        }
         uint32_t held[4][16];
         ok = __all_sync(0xffffffffu, ptx::mbar_wait(&ctl->acc_full[a0], p0, abort_flag));
         if (!ok) break;
@@ -689,14 +841,15 @@ int launch_as(const CallArgs& c) {
   const int kt_count = c.k / TILE_K;
 
   Maps maps;
-  rc = make_tensormap_u8_sw128(&maps.w, c.b, (uint64_t)c.num_experts * c.n, (uint64_t)c.k, TILE_N);
+  const uint64_t w_rows = (uint64_t)c.num_experts * c.n * (S::GATED ? 2 : 1);
+  rc = make_tensormap_u8_sw128(&maps.w, c.b, w_rows, (uint64_t)c.k, TILE_N);
   if (rc != ES_B200_OK) return rc;
   const uint32_t boxes[5] = {8, 16, 32, 64, 96};
   for (int i = 0; i < 5; ++i) {
     rc = make_tensormap_u8_sw128(&maps.x[i], c.a, (uint64_t)c.num_rows, (uint64_t)c.k, boxes[i]);
     if (rc != ES_B200_OK) return rc;
   }
-  rc = make_tensormap_records512(&maps.sfw, c.sfb, (uint64_t)c.num_experts * (c.n / TILE_N) * kt_count);
+  rc = make_tensormap_records512(&maps.sfw, c.sfb, w_rows / TILE_N * kt_count);
   if (rc != ES_B200_OK) return rc;
   // whole 128-row atoms only; loads past the end read as zero (a map needs at least one row)
   const uint64_t sfx_rows = (uint64_t)(c.sfa_rows / 128);
@@ -738,15 +891,17 @@ int launch_as(const CallArgs& c) {
   if (attr[1].id == cudaLaunchAttributeProgrammaticStreamSerialization) cfg.numAttrs = 2;
   const int n_pairs = (c.n / TILE_N + 1) / 2;
   const int64_t used = c.num_experts < c.num_rows ? c.num_experts : c.num_rows;
-  const int most_light = weight_tiles_per_item(tunables().mm_item_k_steps, kt_count, used * n_pairs, info.sm_count);
+  const int most_light = weight_tiles_per_item(tunables().mm_item_k_steps, kt_count * (S::GATED ? 2 : 1),
+                                               used * n_pairs, info.sm_count);
   const int light_items = (n_pairs + most_light - 1) / most_light;
   const int group_light = (n_pairs + light_items - 1) / light_items;     // all of about the same length
   const int group_heavy = (group_light + 3) / 4;
-  const int64_t max_items = ((c.num_rows + 128 * ITEM_ATOMS - 1) / (128 * ITEM_ATOMS) + c.num_experts) * (int64_t)n_pairs;
+  const int tile_rows = S::GATED ? SUB_TILE : 128 * ITEM_ATOMS;
+  const int64_t max_items = ((c.num_rows + tile_rows - 1) / tile_rows + c.num_experts) * (int64_t)n_pairs;
   int max_pairs = resident_pairs[dev & 63];
   if (c.max_pairs > 0 && c.max_pairs < max_pairs) max_pairs = c.max_pairs;
   cfg.gridDim = dim3(2 * (unsigned)(max_items < max_pairs ? max_items : max_pairs));
-  KernelArgs args = {c.d, c.ps, c.eo, c.bo, c.num_experts, c.n, c.k, c.heavy_min, group_heavy, group_light, c.counters};
+  KernelArgs args = {c.d, c.scales, c.ps, c.eo, c.bo, c.num_experts, c.n, c.k, c.heavy_min, group_heavy, group_light, c.counters};
   ES_CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, maps, args, *c.scatter));
   return ES_B200_OK;
 }
@@ -761,6 +916,7 @@ int launch(const CallArgs& c) {
 }
 int launch_bf16(const CallArgs& c) { return launch<__nv_bfloat16>(c); }
 int launch_fp16(const CallArgs& c) { return launch<__half>(c); }
+int launch_silu_mul_quant(const CallArgs& c) { return launch_as<__nv_bfloat16, Gated>(c); }
 
 int read_and_clear_status(uint32_t* out) {
   uint32_t v = 0;

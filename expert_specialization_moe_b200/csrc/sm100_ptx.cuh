@@ -237,6 +237,9 @@ __device__ __forceinline__ void stmatrix_x4_trans(uint32_t smem_addr, uint32_t a
                "r"(c), "r"(d)
                : "memory");
 }
+__device__ __forceinline__ void st_shared_u8(uint32_t smem_addr, uint32_t v) {
+  asm volatile("st.shared.u8 [%0], %1;" ::"r"(smem_addr), "r"(v) : "memory");
+}
 __device__ __forceinline__ uint4 ld_shared_16B(uint32_t smem_addr) {
   uint4 v;
   asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(smem_addr) : "memory");

@@ -196,32 +196,31 @@ class ExpertShard:
         capacity-sized intermediates.  Returns [capacity, H] (rows past the valid ones are undefined) — or, with
         `scatter` = (row_meta, peer table, world, slots), nothing: the down GEMM then stores every output row
         straight into its (GPU, slot) destination (es_b200_mxfp8_grouped_mm_scatter)."""
+        from . import _cabi
         from .ops import es_sm100_mxfp8_blockscaled_grouped_mm as mm
-        from .ops import es_sm100_mxfp8_silu_mul_grouped_quant as silu_mul_quant
         cap, dev = a.shape[0], a.device
         if work.get("cap") != cap:
             work.clear()
-            ps = lambda n, k: torch.tensor([[0, n, k]] * self.e_local, dtype=torch.int32, device=dev)
             work.update(cap=cap,
-                        h1=torch.empty((cap, self.n1), dtype=torch.bfloat16, device=dev),
                         a2=torch.empty((cap, self.i), dtype=torch.uint8, device=dev).view(torch.float8_e4m3fn),
                         sfa2=torch.zeros((sfa.shape[0], self.i // 32), dtype=torch.uint8, device=dev),
-                        ps1=ps(self.n1, self.h), ps2=ps(self.h, self.i))
-        # problem lists live in the work set: only the row counts change from step to step (no allocation per step)
-        ps1, ps2 = work["ps1"], work["ps2"]
-        ps1[:, 0].copy_(rows)
+                        ps=torch.tensor([[0, self.h, self.i]] * self.e_local, dtype=torch.int32, device=dev))
+        # the problem list lives in the work set: only the row counts change from step to step (no allocation per step)
+        ps2 = work["ps"]
         ps2[:, 0].copy_(rows)
-        mm(work["h1"], a, self.w1.transpose(1, 2), sfa, self.sf1, ps1, eo, bo)
-        silu_mul_quant(work["h1"], ps2, eo, bo, work["a2"], work["sfa2"])
+        stream = torch.cuda.current_stream(dev).cuda_stream
+        scratch = _cabi.grouped_mm_scratch(dev, stream)
+        # gate_up GEMM, SiLU * mul and requantisation in one kernel (of the problem list it reads the row counts only)
+        _cabi.check(_cabi.load().es_b200_mxfp8_grouped_mm_silu_mul_quant(
+            a.data_ptr(), self.w1.data_ptr(), sfa.data_ptr(), self.sf1.data_ptr(), work["a2"].data_ptr(),
+            work["sfa2"].data_ptr(), ps2.data_ptr(), eo.data_ptr(), bo.data_ptr(), self.e_local, cap, self.i, self.h,
+            sfa.numel() // (self.h // 32), scratch.data_ptr(), scratch.numel(), stream))
         if scatter is None:
             if "out" not in work:
                 work["out"] = torch.empty((cap, self.h), dtype=torch.bfloat16, device=dev)
             mm(work["out"], work["a2"], self.w2.transpose(1, 2), work["sfa2"], self.sf2, ps2, eo, bo)
             return work["out"]
-        from . import _cabi
         meta, table, world, slots = scatter
-        stream = torch.cuda.current_stream(dev).cuda_stream
-        scratch = _cabi.grouped_mm_scratch(dev, stream)
         _cabi.check(_cabi.load().es_b200_mxfp8_grouped_mm_scatter(
             work["a2"].data_ptr(), self.w2.data_ptr(), work["sfa2"].data_ptr(), self.sf2.data_ptr(), _cabi.BF16,
             ps2.data_ptr(), eo.data_ptr(), bo.data_ptr(), self.e_local, cap, self.h, self.i,

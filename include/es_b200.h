@@ -143,6 +143,20 @@ int es_b200_mxfp8_grouped_mm_scatter(const void* a, const void* b, const uint8_t
                                      void* stream);
 
 /*
+ * The gate_up GEMM of a gated MLP with silu(gate) * up and the MXFP8 requantisation in its epilogue: what
+ * es_b200_mxfp8_grouped_mm (n = 2 * inter) followed by es_b200_mxfp8_silu_mul_grouped_quant computes, from the fp32
+ * products (nothing is rounded to 16 bits in between).  b [num_experts, 2 * inter, k]: an expert's gate rows, then its up
+ * rows; sfb as there.  quant_output [num_rows, inter] e4m3, scale_factor swizzled UE8M0 with expert e at
+ * blockscale_offsets[e] * inter / 32; scale bytes of padding rows are not written.  inter % 128 == 0; quant_output 16-byte
+ * aligned; a row count in problem_sizes[e][0], the other two are not read.  No counterpart in the reference.
+ */
+int es_b200_mxfp8_grouped_mm_silu_mul_quant(const void* a, const void* b, const uint8_t* sfa, const uint8_t* sfb,
+                                            void* quant_output, uint8_t* scale_factor, const int32_t* problem_sizes,
+                                            const int32_t* expert_offsets, const int32_t* blockscale_offsets,
+                                            int num_experts, int64_t num_rows, int inter, int k, int64_t sfa_rows,
+                                            void* scratch, size_t scratch_bytes, void* stream);
+
+/*
  * Expert-parallel exchange over peer memory (one process per GPU; the experts of a layer are spread over the GPUs of a
  * node).  No counterpart in the reference, which has no distributed code: these three calls replace what a caller
  * would otherwise build from an all-to-all, a permutation and es_sm100_mxfp8_blockscaled_grouped_quant
