@@ -45,10 +45,11 @@ constexpr int TILE_K = 128;
 constexpr int X_BYTES = TILE_M * TILE_K;
 constexpr int STAGE_BYTES = X_BYTES + TILE_N * TILE_K;
 constexpr int STAGES = 6;
-constexpr int PARTS = 4;             // TMEM partial buffers: two pairs, one for every two consecutive K blocks of a tile
+constexpr int PARTS = 4;             // TMEM partial buffers
 constexpr int GROUP_COLS = TILE_N / 4;   // columns of one epilogue warp
 constexpr int QUEUE_DEPTH = 4;
 constexpr int SCALES_AHEAD = 4;      // K blocks per read of the scales
+constexpr int ODD_K_BLOCKS = 10;     // odd numbers of K blocks below this: one K block per hand-over
 constexpr uint32_t TMEM_COLS = 512;
 // Registers: the kernel is launched with 96 per thread (20 warps); the epilogue warps (32 accumulators, 32 values on their
 // way from TMEM, scales of eight K blocks) take over what the other four do not need: 16 x 112 + 4 x 32 = 20 x 96.
@@ -68,8 +69,8 @@ struct __align__(16) Tile {
 struct SharedCtl {
   uint64_t full[STAGES];
   uint64_t empty[STAGES];
-  uint64_t pair_full[PARTS / 2];
-  uint64_t pair_empty[PARTS / 2];   // one arrival per epilogue warp
+  uint64_t part_full[PARTS];      // one for the partials of a hand-over
+  uint64_t part_empty[PARTS];     // one arrival per epilogue warp
   uint64_t q_full[QUEUE_DEPTH];     // 1 arrival: the work-list lane has written the entry
   uint64_t q_empty[QUEUE_DEPTH];    // producer, MMA thread, 16 epilogue warps have read it
   Tile tile[QUEUE_DEPTH];
@@ -125,7 +126,11 @@ __device__ __forceinline__ void promote(const uint32_t (&v)[16], float2 scale, f
     acc[first + j] = fma2(make_float2(__uint_as_float(v[2 * j]), __uint_as_float(v[2 * j + 1])), scale, acc[first + j]);
 }
 
-template <typename OutT>
+// HAND: K blocks per hand-over from the MMA thread to the promotion: two, but one where a tile has an odd number of K blocks
+// below ten, of which the last would take a round trip for itself.  us per call with two and with one: k = 128 (16000 rows,
+// 64 experts, n = 4096) 49.1 and 45.8; 384 (21460 Zipf rows, 18, 2816) 61.3 and 57.1; 640 (8000, 64, 2048) 38.8 and 37.1; 896
+// 44.4 and 43.3; 1152 52.2 and 51.8; 1664 62.0 both.
+template <typename OutT, int HAND>
 __global__ void __launch_bounds__(THREADS, 1)
 fp8_blockwise_many_rows_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x16,
                                const __grid_constant__ CUtensorMap map_x32, const __grid_constant__ CUtensorMap map_x64,
@@ -148,9 +153,9 @@ fp8_blockwise_many_rows_kernel(const __grid_constant__ CUtensorMap map_w, const 
       ptx::mbar_init(&ctl->full[s], 1);
       ptx::mbar_init(&ctl->empty[s], 1);
     }
-    for (int p = 0; p < PARTS / 2; ++p) {
-      ptx::mbar_init(&ctl->pair_full[p], 1);
-      ptx::mbar_init(&ctl->pair_empty[p], EPI_WARPS);
+    for (int p = 0; p < PARTS / HAND; ++p) {
+      ptx::mbar_init(&ctl->part_full[p], 1);
+      ptx::mbar_init(&ctl->part_empty[p], EPI_WARPS);
     }
     for (int q = 0; q < QUEUE_DEPTH; ++q) {
       ptx::mbar_init(&ctl->q_full[q], 1);
@@ -258,7 +263,7 @@ fp8_blockwise_many_rows_kernel(const __grid_constant__ CUtensorMap map_w, const 
         const uint32_t idesc = ptx::make_idesc_f8(TILE_M, TILE_N);
         const uint64_t desc0 = ptx::make_desc_k_sw128(ptx::smem_u32(smem));
         QueueReader queue;
-        int s = 0, p = 0;                    // stage of the next K block, pair of partials of the next two
+        int s = 0, p = 0;                    // stage of the next K block, partials of the next hand-over
         uint32_t ph = 0, p_ph = 0;
         bool ok = true;
         while (ok) {
@@ -266,23 +271,23 @@ fp8_blockwise_many_rows_kernel(const __grid_constant__ CUtensorMap map_w, const 
           const int valid = queue.entry(ctl).valid;
           queue.release(ctl);
           if (valid == 0) break;
-          for (int kt = 0; ok && kt < kt_count; kt += 2) {
-            ok = ptx::mbar_wait(&ctl->pair_empty[p], p_ph ^ 1u, abort_flag);
-            for (int h = 0; ok && h < 2 && kt + h < kt_count; ++h) {
+          for (int kt = 0; ok && kt < kt_count; kt += HAND) {
+            ok = ptx::mbar_wait(&ctl->part_empty[p], p_ph ^ 1u, abort_flag);
+            for (int h = 0; ok && h < HAND && kt + h < kt_count; ++h) {
               ok = ptx::mbar_wait(&ctl->full[s], ph, abort_flag);
               if (!ok) break;
               ptx::tc_fence_after_sync();
               const uint64_t x_desc = desc0 + (uint32_t)(s * (STAGE_BYTES / 16));
               const uint64_t w_desc = x_desc + X_BYTES / 16;
-              const uint32_t part = tmem_base + (2 * p + h) * TILE_N;
+              const uint32_t part = tmem_base + (HAND * p + h) * TILE_N;
 #pragma unroll
               for (uint32_t j = 0; j < 4; ++j) ptx::tc_mma_f8(part, x_desc + 2 * j, w_desc + 2 * j, idesc, j != 0 ? 1u : 0u);
               ptx::tc_commit(&ctl->empty[s]);
               if (++s == STAGES) { s = 0; ph ^= 1u; }
             }
             if (!ok) break;
-            ptx::tc_commit(&ctl->pair_full[p]);
-            if (++p == PARTS / 2) { p = 0; p_ph ^= 1u; }
+            ptx::tc_commit(&ctl->part_full[p]);
+            if (++p == PARTS / HAND) { p = 0; p_ph ^= 1u; }
           }
         }
         if (!ok) give_up(abort_flag, ERR_MMA);
@@ -340,23 +345,23 @@ fp8_blockwise_many_rows_kernel(const __grid_constant__ CUtensorMap map_w, const 
           read_scales(sb + kt0 + SCALES_AHEAD, kt_count - kt0 - SCALES_AHEAD, vec4, sb_next);
         }
 #pragma unroll
-        for (int i = 0; i < SCALES_AHEAD; i += 2) {
+        for (int i = 0; i < SCALES_AHEAD; i += HAND) {
           if (kt0 + i >= kt_count) break;
-          ok = __all_sync(0xffffffffu, ptx::mbar_wait(&ctl->pair_full[p], p_ph, abort_flag));
+          ok = __all_sync(0xffffffffu, ptx::mbar_wait(&ctl->part_full[p], p_ph, abort_flag));
           if (!ok) break;
           if (active) {
             // Sixteen columns at a time, so that the reads of the next ones are on their way during the multiplications.
             ptx::tc_fence_after_sync();
-            const uint32_t taddr = taddr0 + p * 2 * TILE_N;
-            const bool two = kt0 + i + 1 < kt_count;
-            const float2 s0 = make_float2(s[i], s[i]), s1 = make_float2(s[i + 1], s[i + 1]);
+            const uint32_t taddr = taddr0 + p * HAND * TILE_N;
+            const bool two = HAND == 2 && kt0 + i + 1 < kt_count;
+            const float2 s0 = make_float2(s[i], s[i]), s1 = make_float2(s[i + HAND - 1], s[i + HAND - 1]);
             uint32_t va[16], vb[16];
             ptx::tc_ld_32x32b_x16(taddr, va);
             ptx::tc_ld_32x32b_x16(taddr + 16, vb);
             ptx::tc_wait_ld();
             promote(va, s0, acc, 0);
             if (two) ptx::tc_ld_32x32b_x16(taddr + TILE_N, va);
-            promote(vb, s0, acc, 8);
+            if (HAND == 2) promote(vb, s0, acc, 8);
             if (two) {
               ptx::tc_wait_ld();
               ptx::tc_ld_32x32b_x16(taddr + TILE_N + 16, vb);
@@ -365,12 +370,12 @@ fp8_blockwise_many_rows_kernel(const __grid_constant__ CUtensorMap map_w, const 
             }
             ptx::tc_fence_before_sync();
             __syncwarp();
-            if (lane == 0) ptx::mbar_arrive(&ctl->pair_empty[p]);   // the tensor core may overwrite these partials
-            if (two) promote(vb, s1, acc, 8);
+            if (lane == 0) ptx::mbar_arrive(&ctl->part_empty[p]);   // the tensor core may overwrite these partials
+            if (two || HAND == 1) promote(vb, s1, acc, 8);
           } else if (lane == 0) {
-            ptx::mbar_arrive(&ctl->pair_empty[p]);
+            ptx::mbar_arrive(&ctl->part_empty[p]);
           }
-          if (++p == PARTS / 2) { p = 0; p_ph ^= 1u; }
+          if (++p == PARTS / HAND) { p = 0; p_ph ^= 1u; }
         }
       }
       if (!ok) break;
@@ -402,8 +407,8 @@ fp8_blockwise_many_rows_kernel(const __grid_constant__ CUtensorMap map_w, const 
   pdl_wait_prior_grid();   // do not complete before the few-rows kernel of this call has
 }
 
-template <typename OutT>
-int launch(const CallArgs& c) {
+template <typename OutT, int HAND>
+int launch_as(const CallArgs& c) {
   DeviceInfo info;
   int rc = get_device_info(&info);
   if (rc != ES_B200_OK) return rc;
@@ -415,7 +420,7 @@ int launch(const CallArgs& c) {
     rc = make_tensormap_u8_sw128(&map_x[i], c.a, (uint64_t)c.num_rows, (uint64_t)c.k, boxes[i]);
     if (rc != ES_B200_OK) return rc;
   }
-  auto kernel = fp8_blockwise_many_rows_kernel<OutT>;
+  auto kernel = fp8_blockwise_many_rows_kernel<OutT, HAND>;
   static bool configured[64] = {false};
   int dev = 0;
   ES_CUDA_TRY(cudaGetDevice(&dev));
@@ -450,6 +455,12 @@ int launch(const CallArgs& c) {
                                  static_cast<OutT*>(c.d), c.ps, c.eo, c.num_experts, c.n, c.k,
                                  (reinterpret_cast<uintptr_t>(c.d) & 31u) == 0 ? 1 : 0, vec4 ? 1 : 0));
   return ES_B200_OK;
+}
+
+template <typename OutT>
+int launch(const CallArgs& c) {
+  const int kt_count = c.k / TILE_K;
+  return (kt_count & 1) != 0 && kt_count < ODD_K_BLOCKS ? launch_as<OutT, 1>(c) : launch_as<OutT, 2>(c);
 }
 
 }  // namespace many
